@@ -7,6 +7,7 @@
 #include <cstdint>
 
 #include "acg_common.h"
+#include "acg_fx.cuh"
 
 #define ACG_CUDA_TRY(expr)                                                    \
   do {                                                                        \
@@ -54,26 +55,23 @@ struct OnlineLse;
 
 template <>
 struct OnlineLse<double> {
-  double m, s;
-  __device__ __forceinline__ void init() {
-    m = -CUDART_INF;
-    s = 0.0;
-  }
-  __device__ __forceinline__ void add(double x) {
-    if (!(x > -CUDART_INF)) return;
-    if (x > m) {
-      s = s * exp(m - x) + 1.0;
-      m = x;
-    } else {
-      s += exp(x - m);
-    }
-  }
+  FxLse a;  // integer arithmetic (acg_fx.cuh)
+  __device__ __forceinline__ void init() { fx_init(a); }
+  __device__ __forceinline__ void add(double x) { fx_add(a, x); }
   // add x = hi + lo (lo tiny next to hi)
   __device__ __forceinline__ void add2(double hi, double lo) { add(hi + lo); }
   __device__ __forceinline__ void add2_fast(double hi, double lo) { add(hi + lo); }
   __device__ __forceinline__ void add_fast(double x) { add(x); }
-  __device__ __forceinline__ double mval() const { return m; }
-  __device__ __forceinline__ double sval() const { return s; }
+  __device__ __forceinline__ double mval() const {
+    double m, s;
+    fx_pair(a, m, s);
+    return m;
+  }
+  __device__ __forceinline__ double sval() const {
+    double m, s;
+    fx_pair(a, m, s);
+    return s;
+  }
 };
 
 template <>

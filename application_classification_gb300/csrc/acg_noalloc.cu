@@ -105,8 +105,8 @@ prior_stats_kernel(const double* __restrict__ x, long long n, int K, const doubl
   if (rl < R)
     for (long long r = (long long)blockIdx.x * R + rl; r < n; r += (long long)gridDim.x * R)
       l.add(-dist_row(x + (size_t)r * K, s_y + p * K, K));
-  s_m[threadIdx.x] = l.m;
-  s_s[threadIdx.x] = l.s;
+  s_m[threadIdx.x] = l.mval();
+  s_s[threadIdx.x] = l.sval();
   __syncthreads();
   for (int c = threadIdx.x; c < P; c += kNaThreads) {
     double m = -CUDART_INF, s = 0.0;

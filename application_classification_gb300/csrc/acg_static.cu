@@ -177,7 +177,11 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
   // per element.  A column whose nearest edge is so far (mn above
   // exp_ref_limit) that the terms leave the normal range is summed again
   // relative to its minimum, which is rare and uniform across the warp.
-  T mn[NQ], qx[NQ], sm[NQ], sc[NQ];
+  // FP64 instead keeps each column's sum in integer arithmetic relative to its
+  // own largest term (acg_fx.cuh): no FP64 exponential and no range to leave.
+  constexpr bool kFx = sizeof(T) == 8;
+  T mn[NQ], qx[NQ], sm[kFx ? 1 : NQ], sc[kFx ? 1 : NQ];
+  FxLse fl[kFx ? NQ : 1];
   // quirk coverage of column q: original edge id < lim - q * De (no edge for
   // the columns q >= qcov, whose quirk value is never read)
   long long qlim[NQ];
@@ -185,8 +189,12 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
   for (int k = 0; k < NQ; ++k) {
     mn[k] = pos_inf<T>();
     qx[k] = neg_inf<T>();
-    sm[k] = T(0);
-    sc[k] = T(0);
+    if constexpr (kFx) {
+      fx_init(fl[k]);
+    } else {
+      sm[k] = T(0);
+      sc[k] = T(0);
+    }
     const int q = (qc + NPOW * (k / W)) * W + k % W;
     qlim[k] = q < qcov ? __ldg(a.qlim_col + q) : 0;
   }
@@ -254,28 +262,48 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
           const T d = sg<T>(x[u][k], w);
           const int j = k * W + w;
           mn[j] = fmin(mn[j], d);
-          kahan_add(sm[j], sc[j], exp_fast(-d));
+          if constexpr (kFx) fx_add(fl[j], -d);
+          else kahan_add(sm[j], sc[j], exp_fast(-d));
           qx[j] = fmax(qx[j], (long long)ecur[u] < qlim[j] ? -d : T(0));
         }
     if (item_done) {
       T lm[NQ], lsum[NQ];  // the column's (reference, sum of exp(-dE - reference))
+      if constexpr (!kFx) {
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) lsum[k] = sm[k] - sc[k];
+        for (int k = 0; k < NQ; ++k) lsum[k] = sm[k] - sc[k];
+      }
 #pragma unroll
       for (int o = NPOW; o < 32; o <<= 1)
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
           mn[k] = fmin(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
           qx[k] = fmax(qx[k], __shfl_xor_sync(0xffffffffu, qx[k], o));
-          lsum[k] += __shfl_xor_sync(0xffffffffu, lsum[k], o);
+          if constexpr (kFx) {
+            FxLse b;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) b.w[i] = __shfl_xor_sync(0xffffffffu, fl[k].w[i], o);
+            fx_merge(fl[k], b);
+          } else {
+            lsum[k] += __shfl_xor_sync(0xffffffffu, lsum[k], o);
+          }
         }
       bool far = false;
+      if constexpr (kFx) {
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) {
-        lm[k] = T(0);
-        far |= mn[k] > exp_ref_limit<T>() && mn[k] < pos_inf<T>();
+        for (int k = 0; k < NQ; ++k) {
+          double m = 0, sv = 0;
+          if (slot == 0) fx_pair(fl[k], m, sv);
+          lm[k] = m;
+          lsum[k] = sv;
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) {
+          lm[k] = T(0);
+          far |= mn[k] > exp_ref_limit<T>() && mn[k] < pos_inf<T>();
+        }
       }
-      if (__any_sync(0xffffffffu, far)) {
+      if (!kFx && __any_sync(0xffffffffu, far)) if constexpr (!kFx) {
         // sum exp(mn - dE) again over this item's edges, for every column
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
@@ -331,8 +359,12 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
       for (int k = 0; k < NQ; ++k) {
         mn[k] = pos_inf<T>();
         qx[k] = neg_inf<T>();
-        sm[k] = T(0);
-        sc[k] = T(0);
+        if constexpr (kFx) {
+          fx_init(fl[k]);
+        } else {
+          sm[k] = T(0);
+          sc[k] = T(0);
+        }
       }
       if (!more) break;
       ++it;
