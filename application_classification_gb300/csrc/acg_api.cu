@@ -393,7 +393,9 @@ vertex_phase:
     va.rec_mh = (T*)P->rec->mh[t];
     va.rec_ml = (T*)P->rec->ml[t];
   }
-  ACG_TRY(launch_vertex_update<T>(va, P->vert_blocks, s));
+  va.lse_pos = P->gv + Pn;
+  if constexpr (std::is_same_v<T, double>) ACG_TRY(launch_vertex_fx(va, P->vert_blocks, s));
+  else ACG_TRY(launch_vertex_update<T>(va, P->vert_blocks, s));
   ACG_TRY(launch_finalize(P->bpart, P->vert_blocks,
                           StatSpec{2 * Pe, 2 * Pe + Pn, P->prec != ACG_PREC_FP64}, P->gi[t & 1], s));
   ACG_TRY(launch_capture_s(P->gi[t & 1] + 4 * Pe, P->iters_p, t, P->S_final, Pn, s));
@@ -808,14 +810,15 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
     for (int p = 0; p < Pn; ++p) md = std::max(md, io[p + 1] - io[p] + oo[p + 1] - oo[p]);
     P->maxdeg = md;
     std::vector<uint32_t> vs;
-    P->vterms = vertex_warp_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, &vs);
+    P->vterms = eb == 8 ? vertex_fx_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, &vs)
+                        : vertex_warp_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, &vs);
     if (P->vterms > 0) {
       st = dev_alloc(&P->owned, sizeof(uint32_t) * vs.size(), (void**)&P->vsched, s);
       if (st != ACG_OK) return fail(st);
       ACG_CUDA_TRY(cudaMemcpyAsync(P->vsched, vs.data(), sizeof(uint32_t) * vs.size(),
                                    cudaMemcpyHostToDevice, s));
     }
-    P->vert_blocks = eb == 8 ? vertex_update_blocks<double>(Pn, Pe, Pp, P->Pnp, P->vterms, nsm, Dn)
+    P->vert_blocks = eb == 8 ? vertex_fx_blocks(Pn, Pe, Pp, P->Pnp, P->vterms, nsm)
                              : vertex_update_blocks<float>(Pn, Pe, Pp, P->Pnp, P->vterms, nsm, Dn);
     if (o.vertex_blocks_per_sm > 0)
       P->vert_blocks = std::min(P->vert_blocks, nsm * o.vertex_blocks_per_sm);

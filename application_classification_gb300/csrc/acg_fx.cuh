@@ -95,28 +95,9 @@ ACG_FX_HD int32_t fx_mulhi(int32_t a, int32_t b) {
 // |x| below this (2^14) takes the integer path; the high word's bits
 constexpr uint32_t kFxLimit = 0x40d00000u;
 
-// exp(x) = 2^k f / 2^61 for |x| < 2^14; f in (0.99, 2.02) 2^61.
-ACG_FX_HD uint64_t fx_exp(uint64_t bits, int& k) {
-  const uint32_t hi = (uint32_t)(bits >> 32), lo = (uint32_t)bits;
-  const uint32_t t = hi & 0x7fffffffu;
-  // x as a float, truncated (exponent rebased from 1023 to 127; 0 below 2^-15,
-  // where n is 0 whatever the value)
-  uint32_t fb = ((hi << 3) | (lo >> 29)) - 0xc0000000u;
-  fb = t < 0x3f000000u ? 0u : (fb | (hi & 0x80000000u));
-  float xf;
-  int n;
-#ifdef __CUDA_ARCH__
-  xf = __uint_as_float(fb);
-  n = __float_as_int(__fmaf_rn(xf, 92.33248262f, 12582912.f)) - 0x4b400000;
-#else
-  std::memcpy(&xf, &fb, 4);
-  n = (int)std::lrintf(xf * 92.33248262f);
-#endif
-  // x with 60 fraction bits, modulo 2^64
-  const uint64_t m = ((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
-  const int c = (int)(t >> 20) - 1015;
-  uint64_t X = c >= 0 ? m << c : (c > -53 ? m >> -c : 0ull);
-  if ((int32_t)hi < 0) X = 0ull - X;
+// exp(x) = 2^k f / 2^61 from x with 60 fraction bits modulo 2^64 (X) and
+// n = 64 x / ln 2 rounded; f in (0.99, 2.02) 2^61.
+ACG_FX_HD uint64_t fx_exp_core(uint64_t X, int n, int& k) {
   // r = x - n ln2 / 64: 92 fraction bits of ln2 / 64
   const int64_t r = (int64_t)(X - (uint64_t)((int64_t)n * (int64_t)0x2c5c85fdf473dell)) -
                     (((int64_t)n * (int64_t)0x6af278edll) >> 32);
@@ -141,6 +122,65 @@ ACG_FX_HD uint64_t fx_exp(uint64_t bits, int& k) {
   const int64_t a = (int64_t)(int32_t)Th * ph;
   const int64_t b = (int64_t)((uint64_t)Th * pl) + (int64_t)Tl * ph;
   return T + (uint64_t)(a << 4) + (uint64_t)(b >> 28);
+}
+
+// exp(x) for a double, |x| < 2^14.
+ACG_FX_HD uint64_t fx_exp(uint64_t bits, int& k) {
+  const uint32_t hi = (uint32_t)(bits >> 32), lo = (uint32_t)bits;
+  const uint32_t t = hi & 0x7fffffffu;
+  // x as a float, truncated (exponent rebased from 1023 to 127; 0 below 2^-15,
+  // where n is 0 whatever the value)
+  uint32_t fb = ((hi << 3) | (lo >> 29)) - 0xc0000000u;
+  fb = t < 0x3f000000u ? 0u : (fb | (hi & 0x80000000u));
+  float xf;
+  int n;
+#ifdef __CUDA_ARCH__
+  xf = __uint_as_float(fb);
+  n = __float_as_int(__fmaf_rn(xf, 92.33248262f, 12582912.f)) - 0x4b400000;
+#else
+  std::memcpy(&xf, &fb, 4);
+  n = (int)std::lrintf(xf * 92.33248262f);
+#endif
+  // x with 60 fraction bits, modulo 2^64
+  const uint64_t m = ((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+  const int c = (int)(t >> 20) - 1015;
+  uint64_t X = c >= 0 ? m << c : (c > -53 ? m >> -c : 0ull);
+  if ((int32_t)hi < 0) X = 0ull - X;
+  return fx_exp_core(X, n, k);
+}
+
+// exp(x) for x = X / 2^Q, 47 <= Q <= 54 and |x| < 2^15.
+ACG_FX_HD uint64_t fx_exp_scaled(int64_t X, int Q, int& k) {
+  const int32_t xi = (int32_t)(X >> (Q - 16));  // 16 fraction bits
+  // 64 / ln2 / 2^16 with 32 fraction bits, rounded at the end
+  const int n = (int)(((int64_t)xi * 6051102 + 0x80000000ll) >> 32);
+  return fx_exp_core((uint64_t)X << (60 - Q), n, k);
+}
+
+// x with Q fraction bits, truncated toward zero, for |x| < 2^(60 - Q); +-2^60
+// beyond that.
+ACG_FX_HD int64_t fx_from_double(double x, int Q) {
+  const uint64_t b = fx_bits(x);
+  const uint32_t hi = (uint32_t)(b >> 32);
+  const int sh = 1083 - Q - (int)((hi >> 20) & 0x7ffu);
+  uint64_t v = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 8;
+  v = sh < 0 ? 1ull << 60 : v >> (sh < 63 ? sh : 63);
+  return (int32_t)hi < 0 ? -(int64_t)v : (int64_t)v;
+}
+// v / 2^Q rounded to a double.
+ACG_FX_HD double fx_to_double(int64_t v, int Q) {
+  const uint64_t sign = (uint64_t)v & 0x8000000000000000ull;
+  uint64_t a = (uint64_t)(v < 0 ? -v : v);
+  if (a == 0) return 0.0;
+#ifdef __CUDA_ARCH__
+  const int lz = __clzll((long long)a);
+#else
+  const int lz = __builtin_clzll(a);
+#endif
+  a <<= lz;
+  // 53 bits, rounded half up; the leading one adds to the exponent field
+  const uint64_t m = (a >> 11) + ((a >> 10) & 1u);
+  return fx_double(sign | (((uint64_t)(1085 - lz - Q) << 52) + m));
 }
 
 // A log-sum-exp state in four words.  Integer form (bit 31 of w[3] clear):

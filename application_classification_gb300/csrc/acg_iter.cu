@@ -1281,15 +1281,12 @@ template acg_status launch_heavy_combine_arg<double>(const double*, const int*, 
 template acg_status launch_heavy_combine_arg<float>(const float*, const int*, const int*, const int*, const int*, int, int, float*, int*, cudaStream_t);
 template acg_status launch_heavy_combine<double>(const double*, const int*, const int*, const int*, int, int, double*, cudaStream_t);
 template acg_status launch_heavy_combine<float>(const float*, const int*, const int*, const int*, int, int, float*, cudaStream_t);
-template acg_status launch_vertex_update<double>(const VertexUpdArgs<double>&, int, cudaStream_t);
 template acg_status launch_vertex_update<float>(const VertexUpdArgs<float>&, int, cudaStream_t);
 template int edge_max_blocks_per_sm<double>(WarpShape);
 template int edge_max_blocks_per_sm<float>(WarpShape);
-template int vertex_update_blocks<double>(int, int, int, int, int, int, int);
 template int vertex_update_blocks<float>(int, int, int, int, int, int, int);
 template acg_status launch_fill<double>(double*, size_t, double, cudaStream_t);
 template acg_status launch_fill<float>(float*, size_t, float, cudaStream_t);
-template int vertex_update_blocks_per_sm<double>(int, int, int);
 template int vertex_update_blocks_per_sm<float>(int, int, int);
 
 }  // namespace acg

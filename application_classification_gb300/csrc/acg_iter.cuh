@@ -85,12 +85,19 @@ struct VertexUpdArgs {
   // MU_raw sums of one stage, [vterms][32] (vertex_warp_schedule)
   const uint32_t* vsched = nullptr;
   int vterms = 0;
+  const double* lse_pos = nullptr;  // [Pn] LSE_v(dV), which bounds |CV| (FP64 only)
 };
 // The warp form's schedule for a pattern (pat: the incidence arrays of
 // build_incidence): per lane, the terms of its (staged vertex, pattern vertex)
 // sums in order.  Returns the terms per lane, 0 when the pattern takes the
 // tile form.
 int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
+// The vertex phase of FP64 plans (acg_vertex_fx.cu), every pattern size: its
+// schedule (nonzero for every pattern), launch and grid.
+int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
+int vertex_fx_warps(int pn, int pp);  // warps that share a stage
+acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s);
+int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms);
 // S_final[p] = S[p] of this iteration where it is p's last (S = the column
 // log-sum-exp of MU_raw in the statistics just finalised).
 acg_status launch_capture_s(const double* S, const int* iters_p, int t, double* S_final, int Pn,

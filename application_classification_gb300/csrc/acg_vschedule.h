@@ -25,7 +25,7 @@ namespace acg {
 
 // schedule word: element offset of the term in the stage (bits 0-11), first
 // term of its job (bit 12), last term (bit 13), the job's slot
-// jv * (32 PPL + 1) + p in the per-warp MU_raw rows (bits 16-24); stored
+// jv * row + p (row: Pn rounded up to 32, plus 1) in the per-warp MU_raw rows (bits 16-24); stored
 // [t / 4][lane][t % 4] so that a lane's four next words are one 16-byte load
 constexpr uint32_t kSchedStart = 1u << 12, kSchedEnd = 1u << 13;
 
@@ -47,17 +47,18 @@ struct VwStage {
 // The schedule for a pattern whose incidence arrays (build_incidence's layout:
 // psrc[pe], pdst[pe], in_off[pn + 1], in_q[pe], out_off[pn + 1], out_q[pe])
 // are at pat, for stages of vps vertices.  Returns the terms per lane (a
-// multiple of 4) and fills out[terms * 32]; 0 when the pattern takes the tile
-// form (more than 64 pattern vertices or padded edge columns) or the stage is
-// too large for the word's fields.
+// multiple of 4) and fills out[terms * nlanes] for nlanes lanes (32, or the
+// lanes of a group of warps); 0 when the pattern has more than two vertices or
+// two padded edge columns per lane, or the stage is too large for the word's
+// fields.
 inline int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, int vps,
-                                std::vector<uint32_t>* out) {
+                                std::vector<uint32_t>* out, int nlanes = 32) {
   out->clear();
-  if (pn <= 0 || pn > 64 || pp > 64 || vps <= 0) return 0;
-  const int ppl = pn <= 32 ? 1 : 2;
+  if (pn <= 0 || pn > 2 * nlanes || pp > 2 * nlanes || vps <= 0) return 0;
+  const int row = (pn + 31) / 32 * 32 + 1;  // a vertex's MU_raw row
   const VwStage G(pp, pnp, false, vps);  // offsets of M, Y, CV (the same for FP32 and FP64)
   // every offset and slot must fit its field of the word
-  if (G.oC + vps * pnp > 0x1000 || vps * (32 * ppl + 1) > 0x200) return 0;
+  if (G.oC + vps * pnp > 0x1000 || vps * row > 0x200) return 0;
   const int* inoff = pat + 2 * pe;
   const int* inq = inoff + pn + 1;
   const int* outoff = inq + pe;
@@ -72,13 +73,13 @@ inline int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp,
     for (int p = 0; p < pn; ++p)
       jobs.push_back({jv, p, 1 + inoff[p + 1] - inoff[p] + outoff[p + 1] - outoff[p]});
   std::stable_sort(jobs.begin(), jobs.end(), [](const Job& x, const Job& y) { return x.len > y.len; });
-  std::vector<std::vector<uint32_t>> lanes(32);
+  std::vector<std::vector<uint32_t>> lanes(nlanes);
   for (const Job& j : jobs) {
     int best = 0;
-    for (int l = 1; l < 32; ++l)
+    for (int l = 1; l < nlanes; ++l)
       if (lanes[l].size() < lanes[best].size()) best = l;
     std::vector<uint32_t>& L = lanes[best];
-    const uint32_t slot = (uint32_t)(j.jv * (32 * ppl + 1) + j.p) << 16;
+    const uint32_t slot = (uint32_t)(j.jv * row + j.p) << 16;
     std::vector<uint32_t> terms;
     terms.push_back((uint32_t)(G.oC + j.jv * pnp + j.p));  // -CV
     for (int i = inoff[j.p]; i < inoff[j.p + 1]; ++i)        // F[q], dst_q = p
@@ -93,9 +94,10 @@ inline int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp,
   for (const auto& L : lanes) nt = std::max(nt, L.size());
   nt = (nt + 3) / 4 * 4;
   // padding terms (word 0) come after a lane's last job and change nothing it stores
-  out->assign(nt * 32, 0u);
-  for (int l = 0; l < 32; ++l)
-    for (size_t t = 0; t < lanes[l].size(); ++t) (*out)[(t / 4) * 128 + l * 4 + t % 4] = lanes[l][t];
+  out->assign(nt * nlanes, 0u);
+  for (int l = 0; l < nlanes; ++l)
+    for (size_t t = 0; t < lanes[l].size(); ++t)
+      (*out)[(t / 4) * 4 * nlanes + l * 4 + t % 4] = lanes[l][t];
   return (int)nt;
 }
 

@@ -1,0 +1,58 @@
+"""FP64 plans whose work runs on the integer pipes, against the FP64 numpy model
+of the algorithm (kernel_algebra, itself pinned to the reference's golden
+outputs): sizes at the edges of the kernels' shapes, and inputs that leave the
+integer form's range in whole or in part, where FP64 takes over.
+
+Tolerance: the FP64 path's, 1e-10 relative to max|mu| (test_gpu_parity.py)."""
+import numpy as np
+import pytest
+
+import kernel_algebra
+from application_classification_gb300 import matcher
+from application_classification_gb300.graph import Graph
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-10
+
+
+def _graphs(dn, de, pn, pe, seed, kv=5, ke=6, vscale=1.0, escale=1.0):
+    rng = np.random.default_rng(seed)
+    ends = lambda n, m: rng.integers(0, n, size=m).astype(np.uint64)  # noqa: E731
+    d = Graph(vscale * rng.normal(size=(dn, kv)), escale * rng.normal(size=(de, ke)), ends(dn, de), ends(dn, de))
+    p = Graph(vscale * rng.normal(size=(pn, kv)), escale * rng.normal(size=(pe, ke)), ends(pn, pe), ends(pn, pe))
+    return d, p
+
+
+def _check(d, p, iters, **kw):
+    ref = kernel_algebra.match(d, p, iters, **kw)
+    mu = matcher.match(d, p, "fp64", num_iters=iters, **kw)
+    assert np.isfinite(mu).all()
+    assert np.abs(mu - ref).max() <= REL * max(1.0, np.abs(ref).max())
+
+
+# lanes, warps of a group, columns and pattern vertices of a lane; ragged last
+# stages (two vertices each), more groups than vertices
+@pytest.mark.parametrize("pn,pe", [(1, 1), (31, 32), (33, 31), (32, 33), (64, 64), (65, 20), (20, 65),
+                                   (128, 128), (64, 129), (128, 255), (5, 256)])
+@pytest.mark.parametrize("dn", [1, 5001])
+def test_vertex_shapes(cuda, dn, pn, pe):
+    d, p = _graphs(dn, 3 * dn + 2, pn, pe, seed=pn * 1000 + pe)
+    _check(d, p, 3)
+
+
+# constants beyond 2^13: the whole launch in FP64 (distances of thousands); and
+# below it with some vertices and edges far outside: their stages in FP64
+@pytest.mark.parametrize("vscale,escale", [(4e3, 1.0), (1.0, 4e3), (3e4, 3e4), (1e-9, 1e-9), (1e9, 1e9)])
+def test_scales(cuda, vscale, escale):
+    d, p = _graphs(700, 2500, 7, 12, seed=4, vscale=vscale, escale=escale)
+    _check(d, p, 3)
+
+
+@pytest.mark.parametrize("far", [2e3, 1e5, 1e12])
+@pytest.mark.parametrize("pn,pe", [(7, 12), (40, 100)])
+def test_outliers(cuda, far, pn, pe):
+    d, p = _graphs(3000, 9000, pn, pe, seed=9)
+    d.edge_feats[::500] *= far
+    d.node_feats[::333] *= 3.0
+    _check(d, p, 3)
