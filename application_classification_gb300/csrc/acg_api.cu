@@ -348,6 +348,7 @@ acg_status iterate(acg_plan* P, int t, double* mu_out, cudaStream_t s) {
     EdgeMaxArgs<T> ea{P->ew.items, P->ew.nitems, P->ew.wsplit, D->dcsr.other,
                       (const T*)P->dE, (const T*)P->vr[(t - 1) & 1], (T*)P->M,
                       (T*)P->part_iter, Pp};
+    ea.Pe = Pe;
     ea.nranges = P->ew.nparts;
     ea.ctr = P->range_ctr;
     ea.pheavy = P->ew.pheavy;

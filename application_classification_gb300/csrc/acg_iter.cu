@@ -104,6 +104,101 @@ __device__ __forceinline__ void heavy_finish(const T* partial, T* M, size_t b0, 
   }
 }
 
+// FP64 maxima without FP64 arithmetic per element.  A difference and a maximum
+// in FP64 occupy an SM for 32 cycles per warp (2 lanes per clock), which bounds
+// the FP64 edge phase at twice the time of its bytes.  Instead each element
+// x - y gets an interval [l, u] from the high words of x and y read as floats,
+// and a column keeps the pair (x, y) of its largest element so far with that
+// pair's interval.  Per step, the elements (and the pair kept) whose interval
+// reaches the largest lower bound are candidates; a single one is the new pair,
+// and only where there are more (two elements within 2^-18 of the operands) are
+// the differences formed in FP64 and compared.  The difference of the pair that
+// remains is formed once per item.  FP64 rounding is monotone, so the result
+// has the bits of the element-wise FP64 maximum.
+// R-MAT 20, pattern 32/64: 4.31 -> 1.99 ms an iteration (9.1 GB: 1.4 ms at the
+// copy bandwidth).
+struct LazyMax {
+  double x, y;  // the largest element so far is x - y
+  float l, u;   // bounds of it; none yet: x = l = u = -inf
+  __device__ __forceinline__ void init() {
+    x = -CUDART_INF;
+    y = 0.0;
+    l = u = -CUDART_INF_F;
+  }
+  __device__ __forceinline__ double value() const { return x - y; }
+  __device__ __forceinline__ void set(bool r, double nx, double ny, float nl, float nu) {
+    x = r ? nx : x;
+    y = r ? ny : y;
+    l = r ? nl : l;
+    u = r ? nu : u;
+  }
+};
+// The float of a high word without sign: truncated toward zero to 20 mantissa
+// bits, 0 below 2^-126 and an infinity from 2^128 on (NaN included).
+__device__ __forceinline__ float trunc_magnitude(uint32_t hi) {
+  const uint32_t t = min(max(hi, 0x38000000u), 0x47f00000u);
+  return __uint_as_float(t * 8u - 0xc0000000u);
+}
+// [l, u] of x - y for y >= 0; where a float cannot hold it, or y is a NaN, a
+// NaN in u (every comparison of a candidate then fails the other way, and FP64
+// decides).  Truncation is below 2^-20 of each operand (2^-126 absolute below
+// the float range), the roundings here below 2^-22.
+__device__ __forceinline__ void diff_bounds(double x, double y, float& l, float& u) {
+  const uint32_t hx = (uint32_t)__double2hiint(x), hy = (uint32_t)__double2hiint(y);
+  const float ax = trunc_magnitude(hx & 0x7fffffffu), fy = trunc_magnitude(hy);
+  const float fx = __uint_as_float(__float_as_uint(ax) | (hx & 0x80000000u));
+  const float d = fx - fy, w = fmaf(ax + fy, 0x1p-19f, 0x1p-124f);
+  l = d - w;
+  u = d + w;
+}
+// One step of a column: N elements x - y, ok where there is one, at positions
+// e, e + stride, ...; the whole warp calls it.  col: a pattern edge's column,
+// not one of the row's padding, whose zeros would tie with each other.  ARG:
+// pos, the first maximal position (-1: none yet).
+template <int N, bool ARG>
+__device__ __forceinline__ void lazy_step(LazyMax& b, int& pos, const double (&x)[N],
+                                          const double (&y)[N], const bool (&ok)[N], bool col, int e,
+                                          int stride) {
+  float l[N], u[N], top = b.l;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    diff_bounds(x[i], y[i], l[i], u[i]);
+    top = fmaxf(top, l[i]);  // (no element: l = -inf)
+  }
+  bool c[N];
+  int n = !(b.u < top);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    c[i] = ok[i] && !(u[i] < top);
+    n += c[i];
+  }
+  if (__any_sync(0xffffffffu, n > 1 && col)) {
+    // in FP64, in order (volatile: not computed ahead of the vote)
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      double v, m;
+      asm volatile("sub.f64 %0, %1, %2;" : "=d"(v) : "d"(x[i]), "d"(y[i]));
+      asm volatile("sub.f64 %0, %1, %2;" : "=d"(m) : "d"(b.x), "d"(b.y));
+      const bool r = ok[i] && (v > m || (ARG && pos < 0));
+      b.set(r, x[i], y[i], l[i], u[i]);
+      if constexpr (ARG) pos = r ? e + i * stride : pos;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      b.set(c[i], x[i], y[i], l[i], u[i]);
+      if constexpr (ARG) pos = c[i] ? e + i * stride : pos;
+    }
+  }
+}
+// max of two doubles that are not NaN, as integers
+__device__ __forceinline__ double max_bits(double a, double b) {
+  const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+  const long long ka = ia ^ ((ia >> 63) & 0x7fffffffffffffffll);
+  const long long kb = ib ^ ((ib >> 63) & 0x7fffffffffffffffll);
+  return ka >= kb ? a : b;
+}
+
 // One range of a warp's items, [it, it_end).
 template <typename T, int NPOW, int NQV, bool ARG>
 __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, const int it_end,
@@ -128,13 +223,17 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
     const int e = base + slot + S * u;
     sidx[u] = e < item.z ? __ldg(a.src_of + e) : 0;
   }
+  constexpr bool kLazy = sizeof(T) == 8;
   T acc[NQ];
+  LazyMax best[kLazy ? NQ : 1];
   int pos[ARG ? NQ : 1];
+  bool col[NQ];
 #pragma unroll
-  for (int k = 0; k < NQ; ++k) acc[k] = neg_inf<T>();
-  if constexpr (ARG) {
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) pos[k] = -1;
+  for (int k = 0; k < NQ; ++k) {
+    acc[k] = neg_inf<T>();
+    col[k] = (qc + NPOW * (k / W)) * W + k % W < a.Pe;
+    if constexpr (kLazy) best[k].init();
+    if constexpr (ARG) pos[k] = -1;
   }
   for (;;) {
     // rows of this step
@@ -169,6 +268,24 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
       const int e = nbase + slot + S * u;
       sidx[u] = (more && e < nend) ? __ldg(a.src_of + e) : 0;
     }
+    if constexpr (kLazy) {
+      bool ok[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) ok[u] = base + slot + S * u < item.z;
+#pragma unroll
+      for (int k = 0; k < NQV; ++k)
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+          const int j = k * W + w;
+          double xs[kU], ys[kU];
+#pragma unroll
+          for (int u = 0; u < kU; ++u) {
+            xs[u] = vg<T>(x[u][k], w);
+            ys[u] = vg<T>(y[u][k], w);
+          }
+          lazy_step<kU, ARG>(best[j], pos[ARG ? j : 0], xs, ys, ok, col[j], base + slot, S);
+        }
+    } else {
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
       if constexpr (ARG) {
@@ -193,7 +310,12 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
             acc[k * W + w] = fmax(acc[k * W + w], vg<T>(x[u][k], w) - vg<T>(y[u][k], w));
       }
     }
+    }
     if (item_done) {
+      if constexpr (kLazy) {
+#pragma unroll
+        for (int k = 0; k < NQ; ++k) acc[k] = best[k].value();
+      }
       if constexpr (ARG) {
 #pragma unroll
         for (int o = NPOW; o < 32; o <<= 1)
@@ -210,7 +332,11 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
 #pragma unroll
         for (int o = NPOW; o < 32; o <<= 1)
 #pragma unroll
-          for (int k = 0; k < NQ; ++k) acc[k] = fmax(acc[k], __shfl_xor_sync(0xffffffffu, acc[k], o));
+          for (int k = 0; k < NQ; ++k) {
+            const T ob = __shfl_xor_sync(0xffffffffu, acc[k], o);
+            if constexpr (kLazy) acc[k] = max_bits(acc[k], ob);
+            else acc[k] = fmax(acc[k], ob);
+          }
       }
       if (slot == 0) {
         T* row = item.w >= 0 ? a.partial + (size_t)item.w * Pp : a.M + (size_t)item.x * Pp;
@@ -249,10 +375,10 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
         }
       }
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) acc[k] = neg_inf<T>();
-      if constexpr (ARG) {
-#pragma unroll
-        for (int k = 0; k < NQ; ++k) pos[k] = -1;
+      for (int k = 0; k < NQ; ++k) {
+        acc[k] = neg_inf<T>();
+        if constexpr (kLazy) best[k].init();
+        if constexpr (ARG) pos[k] = -1;
       }
       if (!more) break;
       ++it;
@@ -263,8 +389,14 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
   }
 }
 
+// (FP64: three blocks per SM hide the longer chains, RMAT-20 78 -> 64 ms of edge
+// phases; the wide shapes keep what their registers allow.)
+template <typename T, int NQV>
+constexpr int edge_min_blocks() {
+  return sizeof(T) == 4 ? ACG_EDGE_MINB : NQV == 1 ? 3 : NQV == 2 ? 2 : 1;
+}
 template <typename T, int NPOW, int NQV, bool ARG>
-__global__ void __launch_bounds__(kAT, ACG_EDGE_MINB)
+__global__ void __launch_bounds__(kAT, (edge_min_blocks<T, NQV>()))
 edge_max_kernel(const EdgeMaxArgs<T> a) {
   const int lane = threadIdx.x & 31;
   const int slot = lane / NPOW, qc = lane % NPOW;
@@ -289,27 +421,42 @@ edge_max_kernel(const EdgeMaxArgs<T> a) {
   }
 }
 
-// Max over each heavy vertex's partial rows: one warp per heavy vertex.
+template <typename T>
+__device__ __forceinline__ T max_of(T a, T b) {
+  if constexpr (sizeof(T) == 8) return max_bits(a, b);
+  else return fmaxf(a, b);
+}
+
+// Max over each heavy vertex's partial rows: one block per heavy vertex, its
+// warps over the rows (a hub has hundreds; one warp over all of them took 64 us
+// at R-MAT 20), lanes over the columns.
+constexpr int kHeavyCols = 256;  // columns of a row at most
 template <typename T>
 __global__ void __launch_bounds__(256)
 heavy_combine_kernel(const T* __restrict__ partial, const int* __restrict__ hbase,
-                     const int* __restrict__ hcount, const int* __restrict__ hvert, int nheavy,
-                     int Pp, T* __restrict__ M) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= nheavy) return;
-  const T* p0 = partial + (size_t)hbase[warp] * Pp;
-  const int cnt = hcount[warp];
-  T* row = M + (size_t)hvert[warp] * Pp;
+                     const int* __restrict__ hcount, const int* __restrict__ hvert, int Pp,
+                     T* __restrict__ M) {
+  __shared__ T part[8][kHeavyCols];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const T* p0 = partial + (size_t)hbase[blockIdx.x] * Pp;
+  const int cnt = hcount[blockIdx.x];
   for (int q = lane; q < Pp; q += 32) {
     T m = neg_inf<T>();
-    int r = 0;
-    for (; r + 4 <= cnt; r += 4) {
-      const T a0 = p0[(size_t)r * Pp + q], a1 = p0[(size_t)(r + 1) * Pp + q];
-      const T a2 = p0[(size_t)(r + 2) * Pp + q], a3 = p0[(size_t)(r + 3) * Pp + q];
-      m = fmax(m, fmax(fmax(a0, a1), fmax(a2, a3)));
+    int r = w;
+    for (; r + 24 < cnt; r += 32) {
+      const T a0 = p0[(size_t)r * Pp + q], a1 = p0[(size_t)(r + 8) * Pp + q];
+      const T a2 = p0[(size_t)(r + 16) * Pp + q], a3 = p0[(size_t)(r + 24) * Pp + q];
+      m = max_of(m, max_of(max_of(a0, a1), max_of(a2, a3)));
     }
-    for (; r < cnt; ++r) m = fmax(m, p0[(size_t)r * Pp + q]);
+    for (; r < cnt; r += 8) m = max_of(m, p0[(size_t)r * Pp + q]);
+    part[w][q] = m;
+  }
+  __syncthreads();
+  T* row = M + (size_t)hvert[blockIdx.x] * Pp;
+  for (int q = threadIdx.x; q < Pp; q += 256) {
+    T m = part[0][q];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) m = max_of(m, part[k][q]);
     row[q] = m;
   }
 }
@@ -1169,8 +1316,8 @@ template <typename T>
 acg_status launch_heavy_combine(const T* partial, const int* hbase, const int* hcount,
                                 const int* hvert, int nheavy, int Pp, T* M, cudaStream_t s) {
   if (nheavy == 0) return ACG_OK;
-  heavy_combine_kernel<T><<<ceil_div(nheavy, 8), 256, 0, s>>>(partial, hbase, hcount, hvert,
-                                                               nheavy, Pp, M);
+  if (Pp > kHeavyCols) return set_error(ACG_ERR_UNSUPPORTED, "heavy vertices: %d columns", Pp);
+  heavy_combine_kernel<T><<<nheavy, 256, 0, s>>>(partial, hbase, hcount, hvert, Pp, M);
   ACG_LAUNCH_CHECK();
   return ACG_OK;
 }

@@ -42,6 +42,7 @@ struct EdgeMaxArgs {
   const int* hcount = nullptr;
   const int* hvert = nullptr;
   int* hcnt = nullptr;
+  int Pe = 0;          // columns of Pp that are pattern edges
 };
 
 // Column statistics of one iteration (FP64), double-buffered across iterations:

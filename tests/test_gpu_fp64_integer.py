@@ -56,3 +56,25 @@ def test_outliers(cuda, far, pn, pe):
     d.edge_feats[::500] *= far
     d.node_feats[::333] *= 3.0
     _check(d, p, 3)
+
+
+# edges whose costs agree to eps (0: exactly) around each vertex, so that the
+# edge maxima's intervals overlap and FP64 decides
+@pytest.mark.parametrize("eps", [0.0, 1e-15, 1e-9, 1e-5])
+@pytest.mark.parametrize("pn,pe", [(4, 5), (9, 33), (20, 70)])
+def test_near_ties(cuda, eps, pn, pe):
+    d, p = _graphs(300, 6000, pn, pe, seed=2)
+    rng = np.random.default_rng(3)
+    d.edge_feats[:] = d.edge_feats[rng.integers(0, 3, size=6000)] + eps * rng.normal(size=(6000, 6))
+    d.node_feats[:] = d.node_feats[rng.integers(0, 2, size=300)]
+    _check(d, p, 4)
+
+
+# hubs: in- and out-edges in many chunks, whose partial rows a block combines
+@pytest.mark.parametrize("de", [3000, 60001])
+@pytest.mark.parametrize("pn,pe", [(5, 9), (30, 64), (10, 130)])
+def test_hub_chunks(cuda, de, pn, pe):
+    d, p = _graphs(50, de, pn, pe, seed=7)
+    d.dsts[: de // 2] = 3
+    d.srcs[de // 3:] = 11
+    _check(d, p, 3)
