@@ -404,28 +404,53 @@ src_stats_kernel(const SrcStatsArgs<T> a) {
   }
 }
 
-// One warp per heavy vertex: its chunk rows merged in chunk order (FP64).
+// One block per heavy vertex: its chunk rows merged in FP64, warps over the
+// rows (in order within a warp, warps in order), lanes over the columns.  Sums
+// relative to the same reference (FP32 plans: 0 unless an edge is far) are
+// added without an exponential.  One warp over all rows took 846 us per pattern
+// in the many-pattern workload on R-MAT 17.
+__device__ __forceinline__ void ref_merge(double& m, double& s, double m2, double s2) {
+  if (m2 == m && lse_nonempty(m2, s2)) s += s2;
+  else lse_merge(m, s, m2, s2);
+}
+constexpr int kCombCols = 256;  // columns of a row at most
 template <typename T>
 __global__ void __launch_bounds__(256)
 src_stats_combine_kernel(const SrcStatsArgs<T> a, const int* __restrict__ hbase,
-                         const int* __restrict__ hcount, const int* __restrict__ hvert,
-                         int nheavy) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= nheavy) return;
+                         const int* __restrict__ hcount, const int* __restrict__ hvert) {
+  extern __shared__ __align__(16) unsigned char comb_sm[];
   const int Pp = a.Pp, Pqc = a.Pqc;
+  double* s_m = reinterpret_cast<double*>(comb_sm);  // [8][Pp]
+  double* s_s = s_m + 8 * Pp;
+  T* s_n = reinterpret_cast<T*>(s_s + 8 * Pp);
+  T* s_q = s_n + 8 * Pp;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const size_t rs = (size_t)3 * Pp + Pqc;
-  const T* p0 = a.partial + (size_t)hbase[warp] * rs;
-  const int cnt = hcount[warp];
-  const size_t v = (size_t)hvert[warp];
+  const T* p0 = a.partial + (size_t)hbase[blockIdx.x] * rs;
+  const int cnt = hcount[blockIdx.x];
+  const size_t v = (size_t)hvert[blockIdx.x];
   for (int q = lane; q < Pp; q += 32) {
     T mn = pos_inf<T>(), qx = neg_inf<T>();
     double m = -CUDART_INF, s = 0.0;
-    for (int r = 0; r < cnt; ++r) {
+    for (int r = w; r < cnt; r += 8) {
       const T* pr = p0 + (size_t)r * rs;
       mn = fmin(mn, pr[q]);
-      lse_merge(m, s, (double)pr[Pp + q], (double)pr[2 * Pp + q]);
+      ref_merge(m, s, (double)pr[Pp + q], (double)pr[2 * Pp + q]);
       if (q < Pqc) qx = fmax(qx, pr[3 * Pp + q]);
+    }
+    s_m[w * Pp + q] = m;
+    s_s[w * Pp + q] = s;
+    s_n[w * Pp + q] = mn;
+    s_q[w * Pp + q] = qx;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < Pp; q += 256) {
+    T mn = s_n[q], qx = s_q[q];
+    double m = s_m[q], s = s_s[q];
+    for (int k = 1; k < 8; ++k) {
+      mn = fmin(mn, s_n[k * Pp + q]);
+      qx = fmax(qx, s_q[k * Pp + q]);
+      ref_merge(m, s, s_m[k * Pp + q], s_s[k * Pp + q]);
     }
     a.dEmin[v * Pp + q] = mn;
     a.B[v * Pp + q] = (m > -CUDART_INF && s > 0.0) ? (T)(m + log(s)) : neg_inf<T>();
@@ -794,8 +819,12 @@ acg_status launch_src_stats(const SrcStatsArgs<T>& a, WarpShape ws, int blocks, 
 template <typename T>
 acg_status launch_src_stats_combine(const SrcStatsArgs<T>& a, const WarpWork& w, cudaStream_t s) {
   if (w.nheavy == 0) return ACG_OK;
-  src_stats_combine_kernel<T><<<ceil_div(w.nheavy, 8), 256, 0, s>>>(a, w.hbase, w.hcount, w.hvert,
-                                                                    w.nheavy);
+  if (a.Pp > kCombCols) return set_error(ACG_ERR_UNSUPPORTED, "heavy vertices: %d columns", a.Pp);
+  const size_t sm = (size_t)8 * a.Pp * (2 * sizeof(double) + 2 * sizeof(T));  // at most 64 KB
+  if (sm > 48 * 1024)
+    ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_combine_kernel<T>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  src_stats_combine_kernel<T><<<w.nheavy, 256, sm, s>>>(a, w.hbase, w.hcount, w.hvert);
   ACG_LAUNCH_CHECK();
   return ACG_OK;
 }
