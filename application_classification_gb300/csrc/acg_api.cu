@@ -550,6 +550,14 @@ acg_status run_cdist(acg_plan* P, acg_data* D, long long lim, const F* nf, int n
       vdone = true;
     }
   }
+  if constexpr (std::is_same_v<T, double>) {
+    if (cdist_fx_eligible(D->Kv)) {
+      CdistRbArgs<double, double> av{nf, nullptr, nullptr, P->pv, (double*)P->CV, P->bpart, D->Dn, D->De, lim,
+                                     D->Kv, nfs, P->Pn, P->Pnp, P->Pnp};
+      ACG_TRY(launch_cdist_vertex_fx(av, P->cv_blocks, s));
+      vdone = true;
+    }
+  }
   if (!vdone) {
     CdistRbArgs<T, F> av{nf, nullptr, nullptr, P->pv, (T*)P->CV, P->bpart, D->Dn, D->De, lim,
                          D->Kv, nfs, P->Pn, P->Pnp, P->Pnp};

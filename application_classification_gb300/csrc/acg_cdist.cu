@@ -203,7 +203,7 @@ cdist_rb_kernel(const CdistRbArgs<T, F> a) {
 }
 
 
-// One thread per data row, for the edge cost matrix with K <= 32: the row's
+// One thread per data row, for the FP32 edge cost matrix with K <= 32: the row's
 // features in registers (KM = K rounded up to 4, zero padded: (0 - 0)^2 adds
 // nothing), the pattern features in shared memory read as broadcast 16-byte
 // loads, the distances of one row written by its thread as 16-byte stores (L2
@@ -312,8 +312,10 @@ acg_status launch_cdist_rb(const CdistRbArgs<T, F>& a, int mode, int blocks, cud
 template <typename T, typename F>
 acg_status launch_cdist_edges(const CdistRbArgs<T, F>& a, int blocks, cudaStream_t s) {
   if (a.P == 0 || a.nrows == 0) return ACG_OK;
-  const int km = (a.K + 3) / 4 * 4;
-  if (km >= 4) {
+  if constexpr (std::is_same_v<T, double>) {
+    if (cdist_fx_eligible(a.K)) return launch_cdist_fx(a, blocks, s);
+  } else if (a.K > 0) {
+    const int km = (a.K + 3) / 4 * 4;
     ACG_ROWS_CASE(4) ACG_ROWS_CASE(8) ACG_ROWS_CASE(12) ACG_ROWS_CASE(16)
     ACG_ROWS_CASE(20) ACG_ROWS_CASE(24) ACG_ROWS_CASE(28) ACG_ROWS_CASE(32)
   }

@@ -51,4 +51,11 @@ acg_status launch_cdist_vertex_tc(const float* x, int kstride, int K, const doub
                                   float* out, double* bpart, long long nrows, int max_grid, int* grid_used,
                                   int* err, int num_sms, cudaStream_t s);
 
+// The FP64 cost matrices in fixed point (acg_cdist_fx.cu), 1 <= K <= 32: out
+// only, and the vertex matrix with its statistics (kCdistVertex, one partial
+// column per block).
+bool cdist_fx_eligible(int K);
+acg_status launch_cdist_fx(const CdistRbArgs<double, double>& a, int blocks, cudaStream_t s);
+acg_status launch_cdist_vertex_fx(const CdistRbArgs<double, double>& a, int blocks, cudaStream_t s);
+
 }  // namespace acg

@@ -323,4 +323,87 @@ ACG_FX_HD void fx_merge(FxLse& a, FxLse b) {
   a.w[2] = (uint32_t)(t >> 32);
 }
 
+// ---- distances: sqrt(sum_k (x_k - y_k)^2) exactly from fixed point
+// A feature in units of 2^(a - 57), |x| < 2^a, as h 2^29 + l: h signed 29 bits,
+// l 29 bits.  Differences of the parts need no carry, and over at most 32
+// features sum dh^2, sum dh dl and sum dl^2 fit 64 bits each.
+struct FxPart {
+  int32_t h, l;
+};
+// x rounded to a multiple of 2^(a - 57); *big is set where |x| >= 2^a or x is
+// not finite.
+ACG_FX_HD FxPart fx_part(double x, int a, bool* big) {
+  const uint64_t b = fx_bits(x);
+  const uint32_t hi = (uint32_t)(b >> 32);
+  const int e = (int)((hi >> 20) & 0x7ffu);
+  if (e >= a + 1023) *big = true;  // |x| >= 2^a, infinities, NaN
+  // 53-bit mantissa in units of 2^(e - 1075), wanted 2^(a - 57): e - 1018 - a <= 4
+  const uint64_t m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 4;
+  const int sh = a + 1022 - e;
+  uint64_t v = sh < 0 ? 0ull : sh > 62 ? 0ull : sh == 0 ? m : (m + (1ull << (sh - 1))) >> sh;
+  if (e == 0) v = 0;  // zero (a subnormal is far below any unit used)
+  const int64_t s = (int32_t)hi < 0 ? -(int64_t)v : (int64_t)v;
+  FxPart p;
+  p.h = (int32_t)(s >> 29);
+  p.l = (int32_t)((uint32_t)s & 0x1fffffffu);
+  return p;
+}
+
+ACG_FX_HD float fx_rsqrt(float x) {
+#ifdef __CUDA_ARCH__
+  return rsqrtf(x);
+#else
+  return (float)(1.0 / std::sqrt((double)x));
+#endif
+}
+ACG_FX_HD int32_t fx_f2i(float x) {
+#ifdef __CUDA_ARCH__
+  return __float2int_rn(x);
+#else
+  return (int32_t)std::lrintf(x);
+#endif
+}
+ACG_FX_HD uint32_t fx_f2u(float x) {  // saturating
+#ifdef __CUDA_ARCH__
+  return __float2uint_rz(x);
+#else
+  return x >= 4294967296.f ? 0xffffffffu : (uint32_t)x;
+#endif
+}
+
+// sqrt(sh 2^58 + sc 2^30 + sl) 2^(a - 57) rounded to a double, for a radicand of
+// at least 2^102 (fx_small tells; below it the parts' own rounding would show).
+// Two Newton steps from a single-precision reciprocal root: R0 (31 bits), then
+// the residuals of 64 and of the next bits, each multiplied by the same
+// reciprocal; the root carries 58 bits before its rounding.
+ACG_FX_HD bool fx_small(uint64_t sh) { return (sh >> 44) == 0; }
+ACG_FX_HD double fx_root(uint64_t sh, int64_t sc, uint64_t sl, int a) {
+  // the radicand as hi 2^64 + lo
+  const uint64_t c = (uint64_t)sc << 30;
+  uint64_t lo = (sh << 58) + c;
+  uint64_t hi = (sh >> 6) + (uint64_t)(sc >> 34) + (lo < c ? 1u : 0u);
+  lo += sl;
+  hi += lo < sl ? 1u : 0u;
+#ifdef __CUDA_ARCH__
+  const int z = __clzll((long long)hi) & ~1;
+#else
+  const int z = __builtin_clzll(hi) & ~1;
+#endif
+  // (2 <= z <= 28) 2^z radicand in [2^126, 2^128): its upper 64 bits
+  const uint64_t n = (hi << z) | (lo >> (64 - z));
+  const float nf = (float)(uint32_t)(n >> 32);
+  const float y = fx_rsqrt(nf);  // 2^-15 .. 2^-16
+  const uint32_t r0 = fx_f2u(nf * y * 65536.f);
+  const int64_t e0 = (int64_t)(n - (uint64_t)r0 * r0);
+  const int32_t d0 = fx_f2i((float)(int32_t)(e0 >> 14) * y * 32768.f);
+  const uint64_t r1 = ((uint64_t)r0 << 32) + (uint64_t)((int64_t)d0 << 14);
+  const uint32_t h1 = (uint32_t)(r1 >> 32), l1 = (uint32_t)r1;
+  const int32_t e1 = (int32_t)(n - (uint64_t)h1 * h1 - (((uint64_t)h1 * l1) >> 31));
+  const uint64_t r = r1 + (uint64_t)(int64_t)fx_f2i((float)e1 * y * 32768.f);
+  // r 2^(-z / 2) 2^(a - 57), r in [2^63, 2^64]; a carry out of r's 64 bits
+  // cannot occur below the rounding (r <= 2^64 - 2^10 there)
+  const uint64_t m = (r >> 11) + ((r >> 10) & 1u);
+  return fx_double(((uint64_t)(1022 + 63 - (z >> 1) + a - 57) << 52) + m);
+}
+
 }  // namespace acg

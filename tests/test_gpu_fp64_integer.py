@@ -78,3 +78,31 @@ def test_hub_chunks(cuda, de, pn, pe):
     d.dsts[: de // 2] = 3
     d.srcs[de // 3:] = 11
     _check(d, p, 3)
+
+
+# zero BP iterations: mu is the normalised vertex cost matrix itself; with one,
+# the edge matrix too.  Feature counts at and past the kernels' widths, odd
+# columns, rows shared by data and pattern (distance 0), near pairs.
+@pytest.mark.parametrize("kv,ke", [(1, 2), (2, 1), (3, 32), (13, 17), (32, 31), (33, 40)])
+@pytest.mark.parametrize("pn,pe", [(1, 2), (7, 13), (65, 66)])
+def test_cost_matrices(cuda, kv, ke, pn, pe):
+    if kv > 32 and pn == 1:
+        pytest.skip("one pattern vertex with more than 32 features has never been taken")
+    d, p = _graphs(700, 1100, pn, pe, seed=kv * 100 + ke, kv=kv, ke=ke)
+    d.node_feats[5] = p.node_feats[0]
+    d.edge_feats[9] = p.edge_feats[0]
+    d.edge_feats[11] = p.edge_feats[0] + 1e-9
+    _check(d, p, 0)
+    _check(d, p, 1)
+
+
+# rows and patterns outside the fixed-point range of the block's first rows
+@pytest.mark.parametrize("far", [50.0, 1e6, 1e200])
+def test_cost_matrix_outliers(cuda, far):
+    d, p = _graphs(2000, 5000, 6, 11, seed=8)
+    d.edge_feats[777] *= far
+    d.node_feats[1500] *= min(far, 1e6)
+    _check(d, p, 1)
+    if far < 1e100:
+        p.edge_feats[3] *= far
+        _check(d, p, 1)
