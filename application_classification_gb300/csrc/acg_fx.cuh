@@ -16,7 +16,8 @@
 // at 2^-61 of the largest term, and rescaling is a shift.  A sum of 100,000
 // values near 8 comes out within 4e-15 (an FP64 running sum: 1e-13).
 // FP64 kernels before and after: vertex phase of R-MAT 18 with a 16/32 pattern
-// 1,318 -> 357 us an iteration, source-side static pass 7,070 -> 2,093 us.
+// 1,318 -> 357 us an iteration (then acg_vertex_fx.cu), source-side static pass
+// 7,070 -> 1,392 us.
 //
 // The header compiles for the host as well (the tests run it there).
 #pragma once
@@ -53,11 +54,19 @@ namespace acg {
     0x383337bb0aa53844ull, 0x38cfe25cafa29694ull, 0x396e41b9df20d22aull, 0x3a0e5a940f12f71aull, \
     0x3ab031b9f7490e4cull, 0x3b53cc07b6650ae1ull, 0x3bf92e66f736bd73ull, 0x3ca05dcf167fec4eull, \
     0x3d495f454921b30bull, 0x3df437dcc2b44eeeull, 0x3ea0ecb6dc8a80cfull, 0x3f4f83033d21b05dull}
+// round(2^(j / 1024) 2^61), j < 16
+#define ACG_FX_EXP16_TABLE { \
+    0x2000000000000000ull, 0x20058c0bc5d19d8aull, 0x200b190db43813d4ull, 0x2010a705f5df063bull, \
+    0x201635f4b5797dacull, 0x201bc5da1dc1e9ecull, 0x202156b6597a22e1ull, 0x2026e889936b69dbull, \
+    0x202c7b53f6666adbull, 0x20320f15ad433de0ull, 0x2037a3cee2e1682cull, 0x203d397fc227dd90ull, \
+    0x2042d028760501b5ull, 0x204867c9296ea967ull, 0x204e006207621bdfull, 0x205399f33ae4140bull}
 
 #ifdef __CUDACC__
 static __device__ const uint64_t kFxExpDev[64] = ACG_FX_EXP_TABLE;
+static __device__ const uint64_t kFxExp16Dev[16] = ACG_FX_EXP16_TABLE;
 #endif
 static const uint64_t kFxExpHost[64] = ACG_FX_EXP_TABLE;
+static const uint64_t kFxExp16Host[16] = ACG_FX_EXP16_TABLE;
 
 ACG_FX_HD uint64_t fx_exp_entry(int j) {
 #ifdef __CUDA_ARCH__
@@ -149,12 +158,47 @@ ACG_FX_HD uint64_t fx_exp(uint64_t bits, int& k) {
   return fx_exp_core(X, n, k);
 }
 
-// exp(x) for x = X / 2^Q, 47 <= Q <= 54 and |x| < 2^15.
-ACG_FX_HD uint64_t fx_exp_scaled(int64_t X, int Q, int& k) {
-  const int32_t xi = (int32_t)(X >> (Q - 16));  // 16 fraction bits
-  // 64 / ln2 / 2^16 with 32 fraction bits, rounded at the end
-  const int n = (int)(((int64_t)xi * 6051102 + 0x80000000ll) >> 32);
-  return fx_exp_core((uint64_t)X << (60 - Q), n, k);
+// The same from a table of 2^(j / 1024), which leaves a shorter series
+// (|r| < 4e-4: r + r^2 (1/2 + r/6 + r^2/24)) and half the instructions; kernels
+// build it in shared memory (8 KB) with fx_table_entry.
+constexpr int kFxTable = 1024;
+ACG_FX_HD uint64_t fx_table_entry(int j) {
+#ifdef __CUDA_ARCH__
+  const uint64_t a = kFxExpDev[j >> 4], b = kFxExp16Dev[j & 15];
+  const uint64_t hi = __umul64hi(a, b), lo = a * b;
+#else
+  const uint64_t a = kFxExpHost[j >> 4], b = kFxExp16Host[j & 15];
+  const unsigned __int128 p = (unsigned __int128)a * b;
+  const uint64_t hi = (uint64_t)(p >> 64), lo = (uint64_t)p;
+#endif
+  return (hi << 3) | (lo >> 61);
+}
+// n = 1024 x / ln 2 rounded
+ACG_FX_HD uint64_t fx_exp_tab(uint64_t X, int n, const uint64_t* tab, int& k) {
+  const int64_t r = (int64_t)(X - (uint64_t)((int64_t)n * (int64_t)0x2c5c85fdf473dll)) -
+                    (((int64_t)n * (int64_t)0x735793c7ll) >> 31);
+  const uint64_t T = tab[n & (kFxTable - 1)];
+  k = n >> 10;
+  const int32_t rh = (int32_t)(r >> 18);                          // 42 fraction bits
+  const int32_t r2 = (int32_t)(((int64_t)rh * rh) >> 31);         // 53
+  const int32_t c = 0x40000000 + fx_mulhi(rh, 349525) + fx_mulhi(r2, 43);  // 31
+  const int64_t p = r + (((int64_t)r2 * c) >> 24);
+  const int32_t ph = (int32_t)(p >> 32);
+  const uint32_t pl = (uint32_t)p;
+  const uint32_t Th = (uint32_t)(T >> 32), Tl = (uint32_t)T;
+  const int64_t a = (int64_t)(int32_t)Th * ph;
+  const int64_t b = (int64_t)((uint64_t)Th * pl) + (int64_t)Tl * ph;
+  return T + (uint64_t)(a << 4) + (uint64_t)(b >> 28);
+}
+
+// exp(x) for x = X / 2^Q, 47 <= Q <= 54 and |x| < 2^14.
+// c: 1024 / ln 2 with 64 - Q fraction bits (fx_scaled_factor).
+ACG_FX_HD int32_t fx_scaled_factor(int Q) {
+  return (int32_t)((6345039891169ull + (1ull << (Q - 33))) >> (Q - 32));  // 2^32 1024 / ln 2
+}
+ACG_FX_HD uint64_t fx_exp_scaled(int64_t X, int Q, int32_t c, const uint64_t* tab, int& k) {
+  const int n = (int)(((int64_t)(int32_t)(X >> 32) * c + 0x80000000ll) >> 32);
+  return fx_exp_tab((uint64_t)X << (60 - Q), n, tab, k);
 }
 
 // x with Q fraction bits, truncated toward zero, for |x| < 2^(60 - Q); +-2^60
@@ -191,7 +235,7 @@ struct FxLse {
   uint32_t w[4];
 };
 ACG_FX_HD void fx_init(FxLse& a) {
-  a.w[0] = 0x80000000u;  // K = -2^31, below every k
+  a.w[0] = 0xc0000000u;  // K = -2^30, below every k
   a.w[1] = a.w[2] = a.w[3] = 0u;
 }
 ACG_FX_HD bool fx_wide(const FxLse& a) { return (int32_t)a.w[3] < 0; }
@@ -255,21 +299,36 @@ ACG_FX_HD void fx_shift(FxLse& a, uint32_t sh) {
   a.w[3] = (uint32_t)hi;
 }
 
-// add 2^k f / 2^61
+// add 2^k f / 2^61.  A larger term shifts the sum without a branch (some lane of
+// a warp has a new largest term at almost every addition), by up to 31 bits;
+// the first term and larger jumps take the branch.
 ACG_FX_HD void fx_add_term(FxLse& a, int k, uint64_t f) {
-  const int K = (int)a.w[0];
-  if (k > K) {
-    fx_shift(a, (uint32_t)k - (uint32_t)K);
-    a.w[0] = (uint32_t)k;
+  const int d = k - (int)a.w[0];
+  if (d > 31) {
+    fx_shift(a, (uint32_t)d);
   } else {
-    const uint32_t sh = (uint32_t)K - (uint32_t)k;
-    f >>= sh < 63u ? sh : 63u;  // f < 2^63
+    const uint32_t up = d > 0 ? (uint32_t)d : 0u;
+#ifdef __CUDA_ARCH__
+    a.w[1] = __funnelshift_r(a.w[1], a.w[2], up);
+    a.w[2] = __funnelshift_r(a.w[2], a.w[3], up);
+    a.w[3] >>= up;
+#else
+    fx_shift(a, up);
+#endif
   }
+  a.w[0] = (uint32_t)(d > 0 ? k : (int)a.w[0]);
+  const uint32_t dn = d < 0 ? (uint32_t)-d : 0u;
+  f >>= dn < 63u ? dn : 63u;  // f < 2^63
+#ifdef __CUDA_ARCH__
+  asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
+      : "+r"(a.w[1]), "+r"(a.w[2]), "+r"(a.w[3]) : "r"((uint32_t)f), "r"((uint32_t)(f >> 32)));
+#else
   const uint64_t lo = ((uint64_t)a.w[2] << 32) | a.w[1];
   const uint64_t t = lo + f;
   a.w[3] += t < lo;
   a.w[1] = (uint32_t)t;
   a.w[2] = (uint32_t)(t >> 32);
+#endif
 }
 
 ACG_FX_HD void fx_add(FxLse& a, double x) {
@@ -281,6 +340,34 @@ ACG_FX_HD void fx_add(FxLse& a, double x) {
     fx_add_term(a, k, f);
   } else if (hi != 0xfff00000u) {  // (-inf adds nothing)
     a = fx_add_wide(a, x);
+  }
+}
+
+// fx_add with a table of 2^(j / 1024) (tab): |x| < 2^9, else fx_add.
+ACG_FX_HD void fx_add(FxLse& a, double x, const uint64_t* tab) {
+  const uint64_t b = fx_bits(x);
+  const uint32_t hi = (uint32_t)(b >> 32), t = hi & 0x7fffffffu;
+  if (t < 0x40800000u && !fx_wide(a)) {
+    // x as a float, and with 60 fraction bits modulo 2^64 (as fx_exp)
+    uint32_t fb = ((hi << 3) | ((uint32_t)b >> 29)) - 0xc0000000u;
+    fb = t < 0x3f000000u ? 0u : (fb | (hi & 0x80000000u));
+    float xf;
+    int n, k;
+#ifdef __CUDA_ARCH__
+    xf = __uint_as_float(fb);
+    n = __float_as_int(__fmaf_rn(xf, 1477.31972f, 12582912.f)) - 0x4b400000;
+#else
+    std::memcpy(&xf, &fb, 4);
+    n = (int)std::lrintf(xf * 1477.31972f);
+#endif
+    const uint64_t m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+    const int c = (int)(t >> 20) - 1015;
+    uint64_t X = c >= 0 ? m << c : (c > -53 ? m >> -c : 0ull);
+    if ((int32_t)hi < 0) X = 0ull - X;
+    const uint64_t f = fx_exp_tab(X, n, tab, k);
+    fx_add_term(a, k, f);
+  } else if (hi != 0xfff00000u) {
+    fx_add(a, x);
   }
 }
 

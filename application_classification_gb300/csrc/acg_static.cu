@@ -89,7 +89,9 @@ template <typename T, int NQV>
 __host__ __device__ constexpr bool src_staged() { return sizeof(T) == 4 && NQV == 1; }
 template <typename T, int NQV>
 __host__ __device__ constexpr size_t src_stage_smem() {
-  return src_staged<T, NQV>() ? (size_t)(kST / 32) * kSrcSlots * kSrcStageBytes : 0;
+  // (FP64: the exponential's table)
+  return sizeof(T) == 8 ? sizeof(uint64_t) * kFxTable
+         : src_staged<T, NQV>() ? (size_t)(kST / 32) * kSrcSlots * kSrcStageBytes : 0;
 }
 __device__ __forceinline__ void src_cp16(void* sdst, const void* gsrc) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
@@ -114,7 +116,7 @@ __device__ __forceinline__ void src_wait(int n) {
 // One range of a warp's items, [it, it_end).
 template <typename T, int NPOW, int NQV>
 __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it, const int it_end,
-                                                const int slot, const int qc) {
+                                                const int slot, const int qc, const uint64_t* tab) {
   using VT = typename SV<T>::type;
   constexpr int W = SV<T>::W;
   constexpr int S = 32 / NPOW;
@@ -182,6 +184,9 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
   constexpr bool kFx = sizeof(T) == 8;
   T mn[NQ], qx[NQ], sm[kFx ? 1 : NQ], sc[kFx ? 1 : NQ];
   FxLse fl[kFx ? NQ : 1];
+  constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
+  unsigned long long nb[kFx ? NQ : 1], qb[kFx ? NQ : 1];  // bits of min dE, min covered
+  int qlim32[kFx ? NQ : 1];                               // (edge ids are below 2^31)
   // quirk coverage of column q: original edge id < lim - q * De (no edge for
   // the columns q >= qcov, whose quirk value is never read)
   long long qlim[NQ];
@@ -191,12 +196,14 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
     qx[k] = neg_inf<T>();
     if constexpr (kFx) {
       fx_init(fl[k]);
+      nb[k] = qb[k] = kInfBits;
     } else {
       sm[k] = T(0);
       sc[k] = T(0);
     }
     const int q = (qc + NPOW * (k / W)) * W + k % W;
     qlim[k] = q < qcov ? __ldg(a.qlim_col + q) : 0;
+    if constexpr (kFx) qlim32[k] = (int)min(max(qlim[k], 0ll), 0x7fffffffll);
   }
   for (;;) {
     VT x[kSU][NQV];
@@ -261,9 +268,20 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
         for (int w = 0; w < W; ++w) {
           const T d = sg<T>(x[u][k], w);
           const int j = k * W + w;
-          mn[j] = fmin(mn[j], d);
-          if constexpr (kFx) fx_add(fl[j], -d);
-          else kahan_add(sm[j], sc[j], exp_fast(-d));
+          if constexpr (!kFx) mn[j] = fmin(mn[j], d);
+          if constexpr (kFx) {
+            // costs are not negative: minima (and the quirk maximum, as minus
+            // the minimum of the covered costs and zeros) in their bits' order
+            const bool cov = ecur[u] < qlim32[j];
+            const unsigned long long bd = (unsigned long long)__double_as_longlong(d);
+            const unsigned long long bc = cov ? bd : 0ull;
+            nb[j] = bd < nb[j] ? bd : nb[j];
+            qb[j] = bc < qb[j] ? bc : qb[j];
+            fx_add(fl[j], -d, tab);
+            continue;
+          } else {
+            kahan_add(sm[j], sc[j], exp_fast(-d));
+          }
           qx[j] = fmax(qx[j], (long long)ecur[u] < qlim[j] ? -d : T(0));
         }
     if (item_done) {
@@ -276,14 +294,18 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
       for (int o = NPOW; o < 32; o <<= 1)
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
-          mn[k] = fmin(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
-          qx[k] = fmax(qx[k], __shfl_xor_sync(0xffffffffu, qx[k], o));
           if constexpr (kFx) {
+            const unsigned long long on = __shfl_xor_sync(0xffffffffu, nb[k], o);
+            const unsigned long long oq = __shfl_xor_sync(0xffffffffu, qb[k], o);
+            nb[k] = on < nb[k] ? on : nb[k];
+            qb[k] = oq < qb[k] ? oq : qb[k];
             FxLse b;
 #pragma unroll
             for (int i = 0; i < 4; ++i) b.w[i] = __shfl_xor_sync(0xffffffffu, fl[k].w[i], o);
             fx_merge(fl[k], b);
           } else {
+            mn[k] = fmin(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+            qx[k] = fmax(qx[k], __shfl_xor_sync(0xffffffffu, qx[k], o));
             lsum[k] += __shfl_xor_sync(0xffffffffu, lsum[k], o);
           }
         }
@@ -295,6 +317,8 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
           if (slot == 0) fx_pair(fl[k], m, sv);
           lm[k] = m;
           lsum[k] = sv;
+          mn[k] = __longlong_as_double((long long)nb[k]);
+          qx[k] = __longlong_as_double((long long)(qb[k] ^ 0x8000000000000000ull));
         }
       } else {
 #pragma unroll
@@ -361,6 +385,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
         qx[k] = neg_inf<T>();
         if constexpr (kFx) {
           fx_init(fl[k]);
+          nb[k] = qb[k] = kInfBits;
         } else {
           sm[k] = T(0);
           sc[k] = T(0);
@@ -389,10 +414,17 @@ src_stats_kernel(const SrcStatsArgs<T> a) {
   const int slot = lane / NPOW, qc = lane % NPOW;
   const int nw = (int)gridDim.x * (kST / 32);
   const int gw = (blockIdx.x * kST + threadIdx.x) >> 5;
+  extern __shared__ __align__(16) unsigned char src_ring[];
+  const uint64_t* tab = reinterpret_cast<const uint64_t*>(src_ring);
+  if constexpr (sizeof(T) == 8) {
+    for (int t = threadIdx.x; t < kFxTable; t += kST)
+      reinterpret_cast<uint64_t*>(src_ring)[t] = fx_table_entry(t);
+    __syncthreads();
+  }
   for (int r = gw; r < a.nranges;) {
     int rn = a.nranges;
     if (a.ctr && lane == 0) rn = nw + atomicAdd(a.ctr, 1);
-    src_stats_range<T, NPOW, NQV>(a, __ldg(a.wsplit + r), __ldg(a.wsplit + r + 1), slot, qc);
+    src_stats_range<T, NPOW, NQV>(a, __ldg(a.wsplit + r), __ldg(a.wsplit + r + 1), slot, qc, tab);
     r = __shfl_sync(0xffffffffu, rn, 0);
   }
   if (a.ctr && lane == 0) {

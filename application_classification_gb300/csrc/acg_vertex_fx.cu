@@ -15,16 +15,19 @@
 // M <= LSE(Z + B)), |CV| <= LSE(dV), hence |MU_raw| <= LSE(dV) + the fills of
 // its edges, and f, r by the shifts on top.  With patterns of up to 48 vertices
 // and unit features Q is 48 to 50, finer than a double's last place above 8.
-// A stage that holds any other value (a finite one beyond 2^(60-Q), a NaN), and
-// a launch whose constants exceed 2^13 or are not finite, run the same steps in
-// FP64 (Fp64Ar); so every input the FP64 form took is handled as it was.
+// A stage that holds any other value, and a launch whose constants exceed 2^13
+// or are not finite, run the same steps in FP64 (Fp64Ar); so every input the
+// FP64 form took is handled as it was.
 //
 // A group of NW warps shares a stage of kFxVps vertices; the lanes of the group
 // own QPL columns each (QPL = 2 and NW up to 4 cover 256 pattern edges) and
 // PPL pattern vertices.  Two vertices per stage keep two blocks (16 warps) on
 // an SM; the stage of four of the FP32 kernel would leave one.
-// R-MAT 20, pattern 32/64 (1.05 M vertices, 3.5 GB): see the figures at the
-// launch below.
+// R-MAT 20, pattern 32/64 (1.05 M vertices, 3.5 GB, 0.52 ms at the copy
+// bandwidth): FP64 8.77 ms an iteration, with integer exponentials 5.9, in fixed
+// point 1.71, with the range checked on the words already in registers and the
+// larger exponential table 1.45.  ncu: 1,050 warp instructions per vertex, the
+// integer (ALU) pipe 63% busy, FP64 pipe 11%, DRAM 26%.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -47,13 +50,14 @@ constexpr int kFW = kFT / 32;
 __host__ __device__ inline size_t f16(size_t b) { return (b + 15) & ~size_t(15); }
 
 struct FxSmem {
-  size_t pat, sched, cst, mxd, amp, flags, ring, mu, total, stage, group_ring, mu_n;
+  size_t pat, sched, tab, cst, mxd, amp, flags, ring, mu, total, stage, group_ring, mu_n;
   int mu_row;
   __host__ __device__ FxSmem(int Pn, int Pe, int Pp, int Pnp, int nterms, int nw) {
     const int ng = kFW / nw;  // groups
     size_t o = 0;
     pat = o; o += f16(sizeof(int) * (size_t)(4 * Pe + 2 * (Pn + 1)));
     sched = o; o += f16(sizeof(uint32_t) * (size_t)nterms * 32 * nw);
+    tab = o; o += sizeof(uint64_t) * kFxTable;            // 2^(j / 1024)
     cst = o; o += f16(sizeof(double) * (size_t)6 * Pp);   // fF fR dF dR cF cR
     mxd = o; o += f16(sizeof(double) * (size_t)2 * Pp * ng);  // maxima of FP64 stages
     amp = o; o += f16(sizeof(float) * (size_t)2 * Pp);    // |F|, |R| bounds
@@ -102,12 +106,15 @@ __device__ __forceinline__ bool group_or(int group, bool x) {
 struct FxAr {
   using V = long long;
   int Q;
+  int32_t c;            // fx_scaled_factor(Q)
+  uint32_t lim;         // the high word of 2^(60 - Q)
+  const uint64_t* tab;
   __device__ __forceinline__ V in(double x) const { return fx_from_double(x, Q); }
   __device__ __forceinline__ double out(V v) const { return fx_to_double(v, Q); }
   __device__ __forceinline__ V max2(V a, V b) const { return a > b ? a : b; }
   __device__ __forceinline__ void add(FxLse& l, V x) const {
     int k;
-    const uint64_t f = fx_exp_scaled(x, Q, k);
+    const uint64_t f = fx_exp_scaled(x, Q, c, tab, k);
     fx_add_term(l, k, f);  // (a stage with a wide sum runs in FP64)
   }
 };
@@ -135,10 +142,15 @@ struct StageCtx {
   int gl, group, v0, nv, mu_row;
 };
 
-// One stage in arithmetic A.  c: the lane's column constants, mine: what the
-// lane owns.
+// One stage in arithmetic A; the column constants are the lane's.  In fixed
+// point it returns true, before anything but the stage's M, Y and CV rows is
+// changed, when the stage holds a value that fixed point does not cover: M or Y
+// at 2^(60 - Q) or beyond (low ones only lose to the fill, as -inf does), CV
+// outside +-2^(60 - Q), a NaN with a clear sign (fmax drops a NaN; a set sign
+// reads as a low value), or a sum that an FP64 stage took out of the integer
+// form.
 template <typename A, int QPL, int PPL, int NW>
-__device__ __forceinline__ void run_stage(const A ar, const StageCtx& x, const typename A::V (&fF)[QPL],
+__device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const typename A::V (&fF)[QPL],
                                           const typename A::V (&fR)[QPL], const typename A::V (&dF)[QPL],
                                           const typename A::V (&dR)[QPL], const typename A::V (&cF)[QPL],
                                           const typename A::V (&cR)[QPL], const int (&qd)[QPL],
@@ -152,6 +164,15 @@ __device__ __forceinline__ void run_stage(const A ar, const StageCtx& x, const t
   V* const smu = reinterpret_cast<V*>(x.smu);
   const int qo = x.gl * QPL;
   const bool qon = qo < Pp;
+  bool bad = false;
+  if constexpr (kFx) {
+    uint32_t wide = 0;
+#pragma unroll
+    for (int k = 0; k < QPL; ++k) wide |= S.lr[k].w[3] | S.lf[k].w[3];
+#pragma unroll
+    for (int j = 0; j < PPL; ++j) wide |= S.lmu[j].w[3];
+    bad = (int32_t)wide < 0;
+  }
   // ---- 1. F over M, R over Y; -CV in place
 #pragma unroll
   for (int jv = 0; jv < kFxVps; ++jv) {
@@ -166,6 +187,8 @@ __device__ __forceinline__ void run_stage(const A ar, const StageCtx& x, const t
       }
 #pragma unroll
       for (int k = 0; k < QPL; ++k) {
+        if constexpr (kFx)
+          bad |= __double2hiint(m[k]) >= (int)ar.lim || __double2hiint(y[k]) >= (int)ar.lim;
         // no in-edges: M = -inf; no out-edges: Y = -inf; the fill wins
         sv[im + k] = ar.max2(fF[k], ar.in(m[k]) - dF[k]);
         sv[iy + k] = ar.max2(fR[k], ar.in(y[k]) - dR[k]);
@@ -176,11 +199,17 @@ __device__ __forceinline__ void run_stage(const A ar, const StageCtx& x, const t
       const int p = x.gl + 32 * NW * j;
       if (p < Pn) {
         const int ic = G.oC + jv * Pnp + p;
-        sv[ic] = -ar.in(x.st[ic]);
+        const double cv = x.st[ic];
+        if constexpr (kFx) bad |= ((uint32_t)__double2hiint(cv) & 0x7fffffffu) >= ar.lim;
+        sv[ic] = -ar.in(cv);
       }
     }
   }
-  group_sync<NW>(x.group);
+  if constexpr (kFx) {
+    if (group_or<NW>(x.group, bad)) return true;
+  } else {
+    group_sync<NW>(x.group);
+  }
   // ---- 2. the sums MU_raw of the stage's (vertex, p) jobs
   {
     V s = V(0);
@@ -234,10 +263,14 @@ __device__ __forceinline__ void run_stage(const A ar, const StageCtx& x, const t
           if constexpr (kFx) {
             S.mxF[k] = ar.max2(S.mxF[k], f);
             S.mxR[k] = ar.max2(S.mxR[k], r);
-            if (__double2hiint(b) != (int)0xfff00000u) {  // no out-edges: adds nothing
+            const uint32_t hb = (uint32_t)__double2hiint(b);
+            if ((hb & 0x7fffffffu) < ar.lim) {
               const V bx = ar.in(b);
               ar.add(S.lr[k], f + bx);
               ar.add(S.lf[k], r + bx);
+            } else if (hb != 0xfff00000u) {  // (no out-edges, B = -inf: adds nothing)
+              S.lr[k] = fx_add_wide(S.lr[k], ar.out(f) + b);
+              S.lf[k] = fx_add_wide(S.lf[k], ar.out(r) + b);
             }
           } else {
             x.mxd[qo + k] = fmax(x.mxd[qo + k], f);
@@ -270,6 +303,7 @@ __device__ __forceinline__ void run_stage(const A ar, const StageCtx& x, const t
       }
     }
   }
+  return false;
 }
 
 template <int QPL, int PPL, int NW>
@@ -289,6 +323,7 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   for (int t = tid; t < 4 * Pe + 2 * (Pn + 1); t += kFT) s_pat[t] = a.pat[t];
   for (int t = tid; t < nterms * 32 * NW; t += kFT) s_sched[t] = a.vsched[t];
   for (int t = tid; t < 2 * Pp * kNG; t += kFT) s_mxd[t] = -CUDART_INF;
+  for (int t = tid; t < kFxTable; t += kFT) reinterpret_cast<uint64_t*>(smem + L.tab)[t] = fx_table_entry(t);
   if (tid < 2) s_bound[tid] = 0;
   __syncthreads();
   const int* s_psrc = s_pat;
@@ -352,12 +387,13 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   // every |MU_raw|, |f|, |r| is below the bound, so below 2^60 with Q fraction bits
   const float bound = (__int_as_float(s_bound[0]) + __int_as_float(s_bound[1])) * 1.001f + 64.f;
   const bool fixed = bound < 8192.f;
-  const int Q = fixed ? 60 - ((__float_as_int(bound) >> 23) - 126) : 47;
-  const uint32_t lim = (uint32_t)(1083 - Q) << 20;  // the high word of 2^(60 - Q)
+  // (at most 50: finer than a double from 4 on, and B, dEmin may reach 2^10)
+  const int Q = fixed ? min(50, 60 - ((__float_as_int(bound) >> 23) - 126)) : 47;
 
   const int gl = tid % (32 * NW), group = tid / (32 * NW);
   const int qo = gl * QPL;
-  const FxAr fx{Q};
+  uint64_t* s_tab = reinterpret_cast<uint64_t*>(smem + L.tab);
+  const FxAr fx{Q, fx_scaled_factor(Q), (uint32_t)(1083 - Q) << 20, s_tab};
   long long fFx[QPL], fRx[QPL], dFx[QPL], dRx[QPL], cFx[QPL], cRx[QPL];
   int qd[QPL], qs[QPL];
   LaneStats<QPL, PPL> S;
@@ -426,12 +462,19 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
     for (int c = gl; c < c16; c += 32 * NW)
       fcp16(st + G.oC * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.CV) + co + c * 16);
   };
-  // Whether one of the 16-byte chunks this thread copied holds a value fixed
-  // point does not cover: at 2^(60 - Q) or beyond, other than the infinity
-  // `inf` that stands for a vertex without edges.
-  auto outside = [&](const unsigned char* p, uint32_t inf) {
-    const uint4 w = *reinterpret_cast<const uint4*>(p);
-    return ((w.y & 0x7fffffffu) >= lim && w.y != inf) || ((w.w & 0x7fffffffu) >= lim && w.w != inf);
+  // The stage's M, Y and CV rows again, where fixed point had begun on them (Y's
+  // row in memory is rewritten at the end of its stage only).
+  auto restage = [&](int v0, int nv, unsigned char* st) {
+    const int n16 = (int)((size_t)nv * rowb / 16), c16 = (int)((size_t)nv * crow / 16);
+    for (int c = gl; c < n16; c += 32 * NW) {
+      *reinterpret_cast<uint4*>(st + G.oM * 8 + c * 16) =
+          *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.M) + (size_t)v0 * rowb + c * 16);
+      *reinterpret_cast<uint4*>(st + G.oY * 8 + c * 16) =
+          *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.vf) + (size_t)v0 * rowb + c * 16);
+    }
+    for (int c = gl; c < c16; c += 32 * NW)
+      *reinterpret_cast<uint4*>(st + G.oC * 8 + c * 16) =
+          *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.CV) + (size_t)v0 * crow + c * 16);
   };
   issue(vb, 0);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -444,25 +487,12 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
     x.st = reinterpret_cast<double*>(st);
     x.v0 = v0;
     x.nv = min(kFxVps, ve - v0);
-    uint32_t wide = 0;  // a sum that an FP64 stage took out of the integer form
-#pragma unroll
-    for (int k = 0; k < QPL; ++k) wide |= S.lr[k].w[3] | S.lf[k].w[3];
-#pragma unroll
-    for (int j = 0; j < PPL; ++j) wide |= S.lmu[j].w[3];
-    bool bad = !fixed || (int32_t)wide < 0;
-    {
-      const int n16 = (int)((size_t)x.nv * rowb / 16), c16 = (int)((size_t)x.nv * crow / 16);
-      for (int c = gl; c < n16; c += 32 * NW) {
-        bad |= outside(st + G.oM * 8 + c * 16, 0xfff00000u);
-        bad |= outside(st + G.oY * 8 + c * 16, 0xfff00000u);
-        bad |= outside(st + G.oE * 8 + c * 16, 0x7ff00000u);
-        bad |= outside(st + G.oB * 8 + c * 16, 0xfff00000u);
+    group_sync<NW>(group);
+    if (!fixed || run_stage<FxAr, QPL, PPL, NW>(fx, x, fFx, fRx, dFx, dRx, cFx, cRx, qd, qs, plast, S)) {
+      if (fixed) {
+        restage(v0, x.nv, st);
+        group_sync<NW>(group);
       }
-      for (int c = gl; c < c16; c += 32 * NW) bad |= outside(st + G.oC * 8 + c * 16, 0xffffffffu);
-    }
-    if (!group_or<NW>(group, bad)) {
-      run_stage<FxAr, QPL, PPL, NW>(fx, x, fFx, fRx, dFx, dRx, cFx, cRx, qd, qs, plast, S);
-    } else {
       double fF[QPL], fR[QPL], dF[QPL], dR[QPL], cF[QPL], cR[QPL];
 #pragma unroll
       for (int k = 0; k < QPL; ++k) {
