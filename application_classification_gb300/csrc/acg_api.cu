@@ -349,6 +349,7 @@ acg_status iterate(acg_plan* P, int t, double* mu_out, cudaStream_t s) {
                       (const T*)P->dE, (const T*)P->vr[(t - 1) & 1], (T*)P->M,
                       (T*)P->part_iter, Pp};
     ea.Pe = Pe;
+    ea.wide = P->edge_wide;
     ea.nranges = P->ew.nparts;
     ea.ctr = P->range_ctr;
     ea.pheavy = P->ew.pheavy;
@@ -395,6 +396,7 @@ vertex_phase:
     va.rec_ml = (T*)P->rec->ml[t];
   }
   va.lse_pos = P->gv + Pn;
+  va.wide = P->edge_wide;
   if constexpr (std::is_same_v<T, double>) ACG_TRY(launch_vertex_fx(va, P->vert_blocks, s));
   else ACG_TRY(launch_vertex_update<T>(va, P->vert_blocks, s));
   ACG_TRY(launch_finalize(P->bpart, P->vert_blocks,
@@ -448,7 +450,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
     ACG_TRY(launch_fill<T>((T*)P->Fq, nq, -inf, s));
     P->launches += 5;
   }
-  ACG_CUDA_TRY(cudaMemsetAsync(P->S_final, 0, sizeof(double) * Pn, s));
+  ACG_CUDA_TRY(cudaMemsetAsync(P->S_final, 0, sizeof(double) * (Pn + 1), s));  // and edge_wide
 
   // ---- cdist (ac.hxx:33-56 via main.cu:109-110) + column stats
   ranges.phase("cost matrices");
@@ -487,6 +489,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
                   (const T*)P->Fq, (const T*)P->B, (const T*)P->dEmin, (T*)P->vf,
                   (T*)P->vr[0], P->gv, P->ge, P->bpart, P->pat, De, lim, Dn, Pn, Pe, Pp,
                   P->Pnp, P->Pqc, P->qcov, P->qlim_col};
+    a.wide = P->edge_wide;
     const bool rec0 = P->rec && P->rec->has(0);
     if (rec0) {
       a.rec_f = (T*)P->rec->f[0];
@@ -567,6 +570,7 @@ acg_status run_cdist(acg_plan* P, acg_data* D, long long lim, const F* nf, int n
   // rows in dst-CSR order; with no data edges the kernel writes empty partials
   CdistRbArgs<T, F> ae{ef, gather ? D->dcsr.eid : nullptr, D->dcsr.eid, P->pe, (T*)P->dE,
                        nullptr, D->De, D->De, lim, D->Ke, efs, P->Pe, P->Pp, P->Pp};
+  if (std::is_same_v<T, double>) ae.wide = P->edge_wide;
   if constexpr (std::is_same_v<T, float> && std::is_same_v<F, float>) {
     if (P->cdist_tc && P->edge_costs_ready) {  // written while the features were uploaded
       P->edge_costs_ready = false;
@@ -726,7 +730,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
   alloc(sizeof(int) * spec.pat.size(), (void**)&P->pat);
   alloc(sizeof(int) * std::max(1, Pn), (void**)&P->iters_p);
   alloc(sizeof(long long) * Pp, (void**)&P->qlim_col);
-  alloc(sizeof(double) * std::max(1, Pn), (void**)&P->S_final);
+  alloc(sizeof(double) * (Pn + 1), (void**)&P->S_final);
   alloc(sizeof(int), (void**)&P->dev_err);
   if (P->prec == ACG_PREC_MIXED && o.cdist_kernel != 1) {
     P->cdist_tc = cdist_tc_eligible(D->Ke, (D->Ke + 3) / 4 * 4, Pe, Pp);
@@ -768,6 +772,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
     }
   }
   if (st != ACG_OK) return fail(st);
+  P->edge_wide = reinterpret_cast<int*>(P->S_final + Pn);
   std::vector<long long> qlim(Pp, 0);
   std::copy(spec.qlim.begin(), spec.qlim.end(), qlim.begin());
   ACG_CUDA_TRY(cudaMemcpyAsync(P->pat, spec.pat.data(), sizeof(int) * spec.pat.size(),

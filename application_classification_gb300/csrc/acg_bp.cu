@@ -300,6 +300,7 @@ init_vertex_kernel(const InitArgs<T> a) {
             const double fd = my_MU[s_pdst[q]] - F0;
             const T f = (T)fd;
             r = (T)(my_MU[s_psrc[q]] - R0);
+            if constexpr (sizeof(T) == 8) r = edge_word(r, a.wide);
             y = (T)(fd - (double)a.dEmin[vrow + q]);  // no out-edges: -inf
             const T b = a.B[vrow + q];
             mxF[k * W + w] = fmax(mxF[k * W + w], f);

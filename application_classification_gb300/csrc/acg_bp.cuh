@@ -72,6 +72,7 @@ struct InitArgs {
   T* rec_f = nullptr;
   T* rec_mh = nullptr;
   T* rec_ml = nullptr;
+  int* wide = nullptr;  // FP64: Z is stored as edge_word stores it
 };
 template <typename T>
 acg_status launch_init_vertex(const InitArgs<T>& a, GroupShape gs, int blocks, cudaStream_t s);

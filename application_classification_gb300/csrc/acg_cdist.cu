@@ -119,6 +119,8 @@ cdist_rb_kernel(const CdistRbArgs<T, F> a) {
       for (int j = 0; j < QB; ++j) {
         const int q = q0 + j;
         dist[j] = q < P ? sqrt(acc[i][j]) : T(0);
+        if constexpr (sizeof(T) == 8 && MODE == kCdistEdge)
+          if (a.wide && q < P) dist[j] = edge_word(dist[j], a.wide);
         if (q < P) {
           if (MODE == kCdistEdge) {
             if (q < qlim) l1[j].add(-dist[j]);

@@ -24,6 +24,7 @@ struct CdistRbArgs {
   long long De;
   long long lim;       // Pn * Dn
   int K, kstride, P, Pp, ostride;
+  int* wide = nullptr;  // FP64 edge costs: stored as edge_word stores them
 };
 
 template <typename T, typename F>

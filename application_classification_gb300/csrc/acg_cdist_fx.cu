@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
         if (q0 + j >= P) d[j] = 0.0;
         else if (big || fx_small(sh)) d[j] = pair_fp64(xr, a.y + (size_t)(q0 + j) * K, K);
         else d[j] = fx_root(sh, sc, sl, ax);
+        if (a.wide && q0 + j < P) d[j] = edge_word(d[j], a.wide);
       }
       *reinterpret_cast<double2*>(orow + q0) = make_double2(d[0], d[1]);
     }

@@ -165,6 +165,17 @@ struct OnlineLse<float> {
   __device__ __forceinline__ double sval() const { return (double)s - (double)c; }
 };
 
+// FP64 edge costs dE and messages Z are kept where the FP64 edge phase can read
+// their high words as floats (acg_iter.cu): magnitudes from 2^-100 (smaller
+// ones, and zeros, take 2^-100: 2^48 times below the last place of anything
+// they are added to) to 2^126; *wide is set where one is larger or a NaN, and
+// the edge phase then compares in FP64.
+__device__ __forceinline__ double edge_word(double x, int* wide) {
+  const uint32_t t = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+  if (t >= 0x47d00000u) *wide = 1;
+  return t < 0x39b00000u ? 0x1p-100 : x;
+}
+
 // (max, scaled sum) pair in FP64 for combining partial log-sum-exps.
 struct LseD {
   double m, s;

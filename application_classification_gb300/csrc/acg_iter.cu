@@ -108,85 +108,86 @@ __device__ __forceinline__ void heavy_finish(const T* partial, T* M, size_t b0, 
 // in FP64 occupy an SM for 32 cycles per warp (2 lanes per clock), which bounds
 // the FP64 edge phase at twice the time of its bytes.  Instead each element
 // x - y gets an interval [l, u] from the high words of x and y read as floats,
-// and a column keeps the pair (x, y) of its largest element so far with that
-// pair's interval.  Per step, the elements (and the pair kept) whose interval
-// reaches the largest lower bound are candidates; a single one is the new pair,
-// and only where there are more (two elements within 2^-18 of the operands) are
-// the differences formed in FP64 and compared.  The difference of the pair that
-// remains is formed once per item.  FP64 rounding is monotone, so the result
-// has the bits of the element-wise FP64 maximum.
-// R-MAT 20, pattern 32/64: 4.31 -> 1.99 ms an iteration (9.1 GB: 1.4 ms at the
-// copy bandwidth).
+// and a column keeps the pair (x, y) of its largest element so far.  Per step,
+// the elements (and the pair kept) whose interval reaches the largest lower
+// bound are candidates; a single one is the new pair, and only where there are
+// more (two elements within 2^-18 of the operands) are the differences formed
+// in FP64 and compared.  The difference of the pair that remains is formed once
+// per item.  FP64 rounding is monotone, so the result has the bits of the
+// element-wise FP64 maximum.
+// The integer pipe (shifts, logic, selects: 16 lanes a clock per scheduler) is
+// the next bound, so the values are stored within a float's range (edge_word)
+// and a high word becomes a float by one multiply-add.
+// R-MAT 20, pattern 32/64 (9.1 GB, 1.4 ms at the copy bandwidth): 4.31 ms an
+// iteration in FP64, 1.99 with intervals from clamped words, 1.78
+// so.
 struct LazyMax {
-  double x, y;  // the largest element so far is x - y
-  float l, u;   // bounds of it; none yet: x = l = u = -inf
+  double x, y;  // the largest element so far is x - y (none yet: about -2^127)
   __device__ __forceinline__ void init() {
-    x = -CUDART_INF;
-    y = 0.0;
-    l = u = -CUDART_INF_F;
+    x = -0x1p127;
+    y = 1.0;
   }
   __device__ __forceinline__ double value() const { return x - y; }
-  __device__ __forceinline__ void set(bool r, double nx, double ny, float nl, float nu) {
+  __device__ __forceinline__ void set(bool r, double nx, double ny) {
     x = r ? nx : x;
     y = r ? ny : y;
-    l = r ? nl : l;
-    u = r ? nu : u;
   }
 };
-// The float of a high word without sign: truncated toward zero to 20 mantissa
-// bits, 0 below 2^-126 and an infinity from 2^128 on (NaN included).
-__device__ __forceinline__ float trunc_magnitude(uint32_t hi) {
-  const uint32_t t = min(max(hi, 0x38000000u), 0x47f00000u);
-  return __uint_as_float(t * 8u - 0xc0000000u);
+// The float of a double's high word, truncated toward zero to 20 mantissa bits
+// (magnitudes of edge_word): the exponent rebased from 1023 to 127.  rebase is
+// 8; as a multiplier it keeps the shift off the integer pipe.
+__device__ __forceinline__ float high_float(double x, uint32_t rebase) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  return __uint_as_float((h * rebase + 0x40000000u) | (h & 0x80000000u));
 }
-// [l, u] of x - y for y >= 0; where a float cannot hold it, or y is a NaN, a
-// NaN in u (every comparison of a candidate then fails the other way, and FP64
-// decides).  Truncation is below 2^-20 of each operand (2^-126 absolute below
-// the float range), the roundings here below 2^-22.
-__device__ __forceinline__ void diff_bounds(double x, double y, float& l, float& u) {
-  const uint32_t hx = (uint32_t)__double2hiint(x), hy = (uint32_t)__double2hiint(y);
-  const float ax = trunc_magnitude(hx & 0x7fffffffu), fy = trunc_magnitude(hy);
-  const float fx = __uint_as_float(__float_as_uint(ax) | (hx & 0x80000000u));
-  const float d = fx - fy, w = fmaf(ax + fy, 0x1p-19f, 0x1p-124f);
-  l = d - w;
-  u = d + w;
+__device__ __forceinline__ float high_float_pos(double x, uint32_t rebase) {
+  return __uint_as_float((uint32_t)__double2hiint(x) * rebase + 0x40000000u);
 }
-// One step of a column: N elements x - y, ok where there is one, at positions
-// e, e + stride, ...; the whole warp calls it.  col: a pattern edge's column,
-// not one of the row's padding, whose zeros would tie with each other.  ARG:
-// pos, the first maximal position (-1: none yet).
+// [l, u] of x - y, y > 0: truncation is below 2^-20 of each operand, the
+// roundings here below 2^-22.
+__device__ __forceinline__ void diff_bounds(double x, double y, uint32_t rebase, float& l, float& u) {
+  const float fx = high_float(x, rebase), fy = high_float_pos(y, rebase);
+  const float d = fx - fy, w = fabsf(fx) + fy;
+  l = fmaf(w, -0x1p-19f, d);
+  u = fmaf(w, 0x1p-19f, d);
+}
+// One step of a column: N elements x - y, ok where there is one (below the
+// others' range where not), at positions e, e + stride, ...; the whole warp
+// calls it.  col: a pattern edge's column, not one of the row's padding, whose
+// zeros would tie with each other.  ARG: pos, the first maximal position.
 template <int N, bool ARG>
 __device__ __forceinline__ void lazy_step(LazyMax& b, int& pos, const double (&x)[N],
                                           const double (&y)[N], const bool (&ok)[N], bool col, int e,
-                                          int stride) {
-  float l[N], u[N], top = b.l;
+                                          int stride, uint32_t rebase) {
+  float l[N], u[N], top, bu;
+  diff_bounds(b.x, b.y, rebase, top, bu);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    diff_bounds(x[i], y[i], l[i], u[i]);
-    top = fmaxf(top, l[i]);  // (no element: l = -inf)
+    diff_bounds(x[i], y[i], rebase, l[i], u[i]);
+    top = fmaxf(top, l[i]);
   }
-  bool c[N];
-  int n = !(b.u < top);
+  bool c[N], any = bu >= top, two = false;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    c[i] = ok[i] && !(u[i] < top);
-    n += c[i];
+    c[i] = ok[i] && u[i] >= top;
+    two = two || (any && c[i]);
+    any = any || c[i];
   }
-  if (__any_sync(0xffffffffu, n > 1 && col)) {
+  if (__any_sync(0xffffffffu, two && col)) {
     // in FP64, in order (volatile: not computed ahead of the vote)
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       double v, m;
       asm volatile("sub.f64 %0, %1, %2;" : "=d"(v) : "d"(x[i]), "d"(y[i]));
       asm volatile("sub.f64 %0, %1, %2;" : "=d"(m) : "d"(b.x), "d"(b.y));
-      const bool r = ok[i] && (v > m || (ARG && pos < 0));
-      b.set(r, x[i], y[i], l[i], u[i]);
+      const bool r = ok[i] && v > m;
+      b.set(r, x[i], y[i]);
       if constexpr (ARG) pos = r ? e + i * stride : pos;
     }
   } else {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      b.set(c[i], x[i], y[i], l[i], u[i]);
+      b.set(c[i], x[i], y[i]);
       if constexpr (ARG) pos = c[i] ? e + i * stride : pos;
     }
   }
@@ -200,7 +201,7 @@ __device__ __forceinline__ double max_bits(double a, double b) {
 }
 
 // One range of a warp's items, [it, it_end).
-template <typename T, int NPOW, int NQV, bool ARG>
+template <typename T, int NPOW, int NQV, bool ARG, bool LAZY>
 __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, const int it_end,
                                                const int slot, const int qc) {
   using VT = typename VecT<T>::type;
@@ -223,7 +224,7 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
     const int e = base + slot + S * u;
     sidx[u] = e < item.z ? __ldg(a.src_of + e) : 0;
   }
-  constexpr bool kLazy = sizeof(T) == 8;
+  constexpr bool kLazy = LAZY;
   T acc[NQ];
   LazyMax best[kLazy ? NQ : 1];
   int pos[ARG ? NQ : 1];
@@ -249,8 +250,8 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
           x[u][k] = __ldg(reinterpret_cast<const VT*>(a.vr_in + (size_t)sidx[u] * Pp) + qv);
           y[u][k] = __ldcs(reinterpret_cast<const VT*>(a.dE + (size_t)e * Pp) + qv);
         } else {
-          x[u][k] = vfill<T>(neg_inf<T>());
-          y[u][k] = vfill<T>(T(0));
+          x[u][k] = vfill<T>(kLazy ? T(-0x1p127) : neg_inf<T>());
+          y[u][k] = vfill<T>(T(kLazy ? 1 : 0));
         }
       }
     }
@@ -283,7 +284,7 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
             xs[u] = vg<T>(x[u][k], w);
             ys[u] = vg<T>(y[u][k], w);
           }
-          lazy_step<kU, ARG>(best[j], pos[ARG ? j : 0], xs, ys, ok, col[j], base + slot, S);
+          lazy_step<kU, ARG>(best[j], pos[ARG ? j : 0], xs, ys, ok, col[j], base + slot, S, a.rebase);
         }
     } else {
 #pragma unroll
@@ -334,7 +335,7 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
 #pragma unroll
           for (int k = 0; k < NQ; ++k) {
             const T ob = __shfl_xor_sync(0xffffffffu, acc[k], o);
-            if constexpr (kLazy) acc[k] = max_bits(acc[k], ob);
+            if constexpr (sizeof(T) == 8) acc[k] = max_bits(acc[k], ob);
             else acc[k] = fmax(acc[k], ob);
           }
       }
@@ -389,11 +390,17 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
   }
 }
 
-// (FP64: three blocks per SM hide the longer chains, RMAT-20 78 -> 64 ms of edge
-// phases; the wide shapes keep what their registers allow.)
+// (FP64: four blocks per SM hide the longer chains; RMAT-20 edge phases 57.1 ms,
+// three blocks 60.3, two 67; the wide shapes keep what their registers allow.)
 template <typename T, int NQV>
 constexpr int edge_min_blocks() {
-  return sizeof(T) == 4 ? ACG_EDGE_MINB : NQV == 1 ? 3 : NQV == 2 ? 2 : 1;
+    #ifndef ACG_EDGE_MINB2
+#define ACG_EDGE_MINB2 2
+#endif
+#ifndef ACG_EDGE_MINB4
+#define ACG_EDGE_MINB4 1
+#endif
+  return sizeof(T) == 4 ? ACG_EDGE_MINB : NQV == 1 ? 4 : NQV == 2 ? ACG_EDGE_MINB2 : ACG_EDGE_MINB4;
 }
 template <typename T, int NPOW, int NQV, bool ARG>
 __global__ void __launch_bounds__(kAT, (edge_min_blocks<T, NQV>()))
@@ -402,6 +409,7 @@ edge_max_kernel(const EdgeMaxArgs<T> a) {
   const int slot = lane / NPOW, qc = lane % NPOW;
   const int nw = (int)gridDim.x * (kAT / 32);
   const int gw = (blockIdx.x * kAT + threadIdx.x) >> 5;
+  const bool wide = sizeof(T) == 8 && *a.wide != 0;
   // The warp's own range first, then claimed ones (the claim of the next is in
   // flight while this one runs): warps that finish early keep taking work, so
   // the SMs stay full until the last ranges instead of waiting on the slowest
@@ -409,7 +417,13 @@ edge_max_kernel(const EdgeMaxArgs<T> a) {
   for (int r = gw; r < a.nranges;) {
     int rn = a.nranges;
     if (a.ctr && lane == 0) rn = nw + atomicAdd(a.ctr, 1);
-    edge_max_range<T, NPOW, NQV, ARG>(a, __ldg(a.wsplit + r), __ldg(a.wsplit + r + 1), slot, qc);
+    const int it = __ldg(a.wsplit + r), it_end = __ldg(a.wsplit + r + 1);
+    if constexpr (sizeof(T) == 8) {
+      if (wide) edge_max_range<T, NPOW, NQV, ARG, false>(a, it, it_end, slot, qc);
+      else edge_max_range<T, NPOW, NQV, ARG, true>(a, it, it_end, slot, qc);
+    } else {
+      edge_max_range<T, NPOW, NQV, ARG, false>(a, it, it_end, slot, qc);
+    }
     r = __shfl_sync(0xffffffffu, rn, 0);
   }
   if (a.ctr && lane == 0) {

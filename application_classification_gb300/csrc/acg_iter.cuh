@@ -43,6 +43,11 @@ struct EdgeMaxArgs {
   const int* hvert = nullptr;
   int* hcnt = nullptr;
   int Pe = 0;          // columns of Pp that are pattern edges
+  // FP64: *wide is nonzero where a cost or message is not as edge_word keeps
+  // them in range; rebase is 8 (a multiplier the compiler must not see as a
+  // shift, see high_float)
+  const int* wide = nullptr;
+  uint32_t rebase = 8;
 };
 
 // Column statistics of one iteration (FP64), double-buffered across iterations:
@@ -87,6 +92,7 @@ struct VertexUpdArgs {
   const uint32_t* vsched = nullptr;
   int vterms = 0;
   const double* lse_pos = nullptr;  // [Pn] LSE_v(dV), which bounds |CV| (FP64 only)
+  int* wide = nullptr;              // FP64: Z is stored as edge_word stores it
 };
 // The warp form's schedule for a pattern (pat: the incidence arrays of
 // build_incidence): per lane, the terms of its (staged vertex, pattern vertex)

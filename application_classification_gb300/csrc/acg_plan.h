@@ -79,6 +79,7 @@ struct acg_plan {
   int* pat = nullptr;          // pattern incidence (device)
   int* iters_p = nullptr;      // [Pn] iteration count of each vertex's pattern
   long long* qlim_col = nullptr;  // [Pp] quirk coverage of each column
+  int* edge_wide = nullptr;    // FP64: costs or messages out of edge_word's range (after S_final)
   double* S_final = nullptr;   // [Pn] column LSE of MU_raw at each vertex's last iteration
   bool is_union = false;       // several patterns (the output is scattered)
   bool fill_at_run = false;    // workspaces shared with other plans: refill per match

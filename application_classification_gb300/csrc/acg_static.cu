@@ -750,7 +750,8 @@ init_warp_kernel(const InitArgs<T> a) {
             if (hout) R0 = fmax(R0, ((q < qcov ? cur.rq[k] : T(0)) - lbh[k]) - lbl[k]);
             if (hin) F0 = fmax(F0, ((q < qcov ? cur.fq[k] : T(0)) - lbh[k]) - lbl[k]);
             const T f = (smu[qd[k]] - F0) + smu[32 * PPL + qd[k]];
-            const T r = (smu[qs[k]] - R0) + smu[32 * PPL + qs[k]];
+            T r = (smu[qs[k]] - R0) + smu[32 * PPL + qs[k]];
+            if constexpr (sizeof(T) == 8) r = edge_word(r, a.wide);
             mxF[k] = fmax(mxF[k], f);
             mxR[k] = fmax(mxR[k], r);
             lr[k].add_fast(f + cur.b[k]);

@@ -283,6 +283,8 @@ __device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const t
           fo[k] = ar.out(f);
           yo[k] = fo[k] - em;
           zo[k] = ar.out(r);
+          if constexpr (kFx) zo[k] = r == 0 ? 0x1p-100 : zo[k];  // (edge_word)
+          else zo[k] = edge_word(zo[k], a.wide);
         }
       }
       double* gy = a.vf + v * Pp + qo;

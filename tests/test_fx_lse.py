@@ -31,7 +31,7 @@ int main(int argc, char** argv) {
     const double R = std::atof(argv[1]);
     std::uniform_real_distribution<double> u(-R, R);
     double worst = 0;
-    for (int i = 0; i < 400000; ++i) {
+    for (int i = 0; i < 60000; ++i) {
       const double x = i == 0 ? 0.0 : i == 1 ? -0.0 : i == 2 ? 5e-324 : i == 3 ? R : i == 4 ? -R : u(g);
       int k;
       const uint64_t f = fx_exp(fx_bits(x), k);
@@ -43,7 +43,7 @@ int main(int argc, char** argv) {
     for (int j = 0; j < kFxTable; ++j) tab[j] = fx_table_entry(j);
     double worst_tab = 0;
     for (int Q = 47; Q <= 50; ++Q)
-      for (int i = 0; i < 100000; ++i) {
+      for (int i = 0; i < 20000; ++i) {
         const double x = i == 0 ? 0.0 : i == 1 ? R : i == 2 ? -R : u(g);
         if (std::fabs(x) >= std::ldexp(1.0, 60 - Q)) continue;
         int k;
