@@ -158,7 +158,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
       VT* dst = ring + (size_t)(issued % kSrcSlots) * (kSrcStageBytes / 16);
 #pragma unroll
       for (int i = 0; i < kSU; ++i) {
-        const int c = lane + 32 * i, row = c / NPOW, qv = c % NPOW;
+        const int c = lane + 32 * i, row = c / NPOW, qv = a.col0 + c % NPOW;
         const int e = P0 + issued * STEP + row;
         if (e < P1 && qv * W < Pp)
           src_cp16(dst + c, reinterpret_cast<const VT*>(a.dE + (size_t)nrow[i] * Pp) + qv);
@@ -225,7 +225,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
         const int rel = e - P0, j = rel / STEP;
         (void)jlo;
         x[u][0] = (okv[u] && qc * W < Pp)
-                      ? ring[(size_t)(j % kSrcSlots) * (kSrcStageBytes / 16) + (rel - j * STEP) * NPOW + qc]
+                      ? ring[(size_t)(j % kSrcSlots) * (kSrcStageBytes / 16) + (rel - j * STEP) * NPOW + qc - a.col0]
                       : sfill<T>(pos_inf<T>());
       }
     } else {
@@ -411,7 +411,7 @@ template <typename T, int NPOW, int NQV>
 __global__ void __launch_bounds__(kST, src_staged<T, NQV>() ? 2 : (ACG_SRC_MINB > 0 ? ACG_SRC_MINB : 1))
 src_stats_kernel(const SrcStatsArgs<T> a) {
   const int lane = threadIdx.x & 31;
-  const int slot = lane / NPOW, qc = lane % NPOW;
+  const int slot = lane / NPOW, qc = a.col0 + lane % NPOW;
   const int nw = (int)gridDim.x * (kST / 32);
   const int gw = (blockIdx.x * kST + threadIdx.x) >> 5;
   extern __shared__ __align__(16) unsigned char src_ring[];
@@ -831,22 +831,32 @@ bool init_warp_shape(int pn, int pp, F&& f) {
 
 }  // namespace
 
-#define ACG_SRC_LAUNCH(NP_, NQ_)                                                            \
-  if (ws.npow == NP_ && ws.nqv == NQ_) {                                                    \
-    constexpr size_t sm = src_stage_smem<T, NQ_>();                                         \
+#define ACG_SRC_SHAPES(X) X(1) X(2) X(4) X(8) X(16) X(32)
+#define ACG_SRC_LAUNCH(NP_)                                                                 \
+  if (ws.npow == NP_) {                                                                     \
+    constexpr size_t sm = src_stage_smem<T, 1>();                                           \
     if (sm > 48 * 1024)                                                                     \
-      ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_kernel<T, NP_, NQ_>,                      \
+      ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_kernel<T, NP_, 1>,                        \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-    src_stats_kernel<T, NP_, NQ_><<<blocks, kST, sm, s>>>(a);                               \
+    src_stats_kernel<T, NP_, 1><<<blocks, kST, sm, s>>>(a);                                 \
     ACG_LAUNCH_CHECK();                                                                     \
-    return ACG_OK;                                                                          \
+    continue;                                                                               \
   }
 
+// Rows of more than 32 vectors (above 128 FP32 or 64 FP64 columns) in launches of
+// 32 each: two or four vectors a lane cost registers, so warps in flight (R-MAT
+// 18 with 120 FP64 columns 7.9 -> 3.8 ms, R-MAT 16 with 250 8.5 -> 2.1 ms, with
+// 250 FP32 columns 0.82 -> 0.41 ms).
 template <typename T>
-acg_status launch_src_stats(const SrcStatsArgs<T>& a, WarpShape ws, int blocks, cudaStream_t s) {
-  if (a.nitems == 0) return ACG_OK;
-  ACG_STATIC_SHAPES(ACG_SRC_LAUNCH)
-  return set_error(ACG_ERR_UNSUPPORTED, "no source-side kernel for npow=%d nqv=%d", ws.npow, ws.nqv);
+acg_status launch_src_stats(const SrcStatsArgs<T>& args, WarpShape ws, int blocks, cudaStream_t s) {
+  if (args.nitems == 0) return ACG_OK;
+  SrcStatsArgs<T> a = args;
+  if (ws.nqv > 1) blocks *= 2;  // (split for one block per SM, two fit; ranges are claimed)
+  for (a.col0 = 0; a.col0 * SV<T>::W < a.Pp; a.col0 += 32) {
+    ACG_SRC_SHAPES(ACG_SRC_LAUNCH)
+    return set_error(ACG_ERR_UNSUPPORTED, "no source-side kernel for npow=%d", ws.npow);
+  }
+  return ACG_OK;
 }
 
 template <typename T>
@@ -880,13 +890,13 @@ acg_status launch_dst_quirk(const DstQuirkArgs<T>& a, WarpShape ws, int blocks, 
   return set_error(ACG_ERR_UNSUPPORTED, "no quirk kernel for npow=%d nqv=%d", ws.npow, ws.nqv);
 }
 
-#define ACG_SRC_OCC(NP_, NQ_)                                                           \
-  if (ws.npow == NP_ && ws.nqv == NQ_) {                                                \
-    constexpr size_t sm = src_stage_smem<T, NQ_>();                                     \
+#define ACG_SRC_OCC(NP_)                                                                \
+  if (ws.npow == NP_) {                                                                 \
+    constexpr size_t sm = src_stage_smem<T, 1>();                                       \
     if (sm > 48 * 1024)                                                                 \
-      cudaFuncSetAttribute(src_stats_kernel<T, NP_, NQ_>,                               \
+      cudaFuncSetAttribute(src_stats_kernel<T, NP_, 1>,                                 \
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);       \
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, src_stats_kernel<T, NP_, NQ_>, \
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, src_stats_kernel<T, NP_, 1>, \
                                                       kST, sm) != cudaSuccess)          \
       nb = 1;                                                                           \
   }
@@ -894,7 +904,10 @@ acg_status launch_dst_quirk(const DstQuirkArgs<T>& a, WarpShape ws, int blocks, 
 template <typename T>
 int src_stats_blocks_per_sm(WarpShape ws) {
   int nb = 1;
-  ACG_STATIC_SHAPES(ACG_SRC_OCC)
+  // wide rows: item ranges, and with them the hubs' chunks (whose sums are formed
+  // one by one), for one block per SM
+  if (ws.nqv > 1) return 1;
+  ACG_SRC_SHAPES(ACG_SRC_OCC)
   return nb < 1 ? 1 : nb;
 }
 

@@ -46,6 +46,7 @@ struct SrcStatsArgs {
   // ranges from ctr (two zeroed ints, reset by the last warp to finish)
   int nranges = 0;
   int* ctr = nullptr;
+  int col0 = 0;  // first 16-byte column of the launch (rows wider than 32: several)
 };
 template <typename T>
 acg_status launch_src_stats(const SrcStatsArgs<T>& a, WarpShape ws, int blocks, cudaStream_t s);
