@@ -127,7 +127,10 @@ struct OnlineLse<float> {
   // statistics: m' = max(m, x); s = s e^(m - m') + e^(x - m').  Terms near the
   // running maximum dominate the sum and carry ~1e-7 relative error.
   __device__ __forceinline__ void add_fast(float x) {
-    if (!(x > -CUDART_INF_F)) return;
+    if (x > -CUDART_INF_F) add_fast_some(x);
+  }
+  // the same for x known to be above -inf
+  __device__ __forceinline__ void add_fast_some(float x) {
     const float mn = fmaxf(m, x);
     const float sc = __expf(m - mn);  // m = -inf -> 0
     s *= sc;

@@ -1360,6 +1360,7 @@ bool warp_form(int pn, int pp, F&& f) {
 
 template <typename T>
 acg_status launch_vertex_update(const VertexUpdArgs<T>& a, int blocks, cudaStream_t s) {
+  if (a.Pp > 64) return launch_vertex_wide(a, blocks, s);
   cudaError_t le = cudaSuccess;
   if (a.vsched == nullptr && a.Pn > 0 && a.Pn <= 64 && a.Pp <= 64)
     return set_error(ACG_ERR_INVALID_ARGUMENT, "vertex phase: no schedule for the warp form");

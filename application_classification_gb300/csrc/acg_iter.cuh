@@ -101,6 +101,11 @@ struct VertexUpdArgs {
 int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
 // The vertex phase of FP64 plans (acg_vertex_fx.cu), every pattern size: its
 // schedule (nonzero for every pattern), launch and grid.
+// The vertex phase of FP32 plans with more than 64 padded edge columns
+// (acg_vertex_wide.cu): its schedule and launch; blocks as vertex_update_blocks
+// gives them.
+int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
+acg_status launch_vertex_wide(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s);
 int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
 int vertex_fx_warps(int pn, int pp);  // warps that share a stage
 acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s);

@@ -48,13 +48,13 @@ struct VwStage {
 // psrc[pe], pdst[pe], in_off[pn + 1], in_q[pe], out_off[pn + 1], out_q[pe])
 // are at pat, for stages of vps vertices.  Returns the terms per lane (a
 // multiple of 4) and fills out[terms * nlanes] for nlanes lanes (32, or the
-// lanes of a group of warps); 0 when the pattern has more than two vertices or
-// two padded edge columns per lane, or the stage is too large for the word's
+// lanes of a group of warps); 0 when the pattern has more than per_lane
+// vertices or padded edge columns per lane, or the stage is too large for the word's
 // fields.
 inline int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, int vps,
-                                std::vector<uint32_t>* out, int nlanes = 32) {
+                                std::vector<uint32_t>* out, int nlanes = 32, int per_lane = 2) {
   out->clear();
-  if (pn <= 0 || pn > 2 * nlanes || pp > 2 * nlanes || vps <= 0) return 0;
+  if (pn <= 0 || pn > per_lane * nlanes || pp > per_lane * nlanes || vps <= 0) return 0;
   const int row = (pn + 31) / 32 * 32 + 1;  // a vertex's MU_raw row
   const VwStage G(pp, pnp, false, vps);  // offsets of M, Y, CV (the same for FP32 and FP64)
   // every offset and slot must fit its field of the word
