@@ -397,16 +397,36 @@ vertex_phase:
   }
   va.lse_pos = P->gv + Pn;
   va.wide = P->edge_wide;
+  const bool wide = sizeof(T) == 4 && Pp > 64;
+  if constexpr (sizeof(T) == 4) va.rowpart = (float*)P->rowpart;
+  // Beside the next edge phase where that lasts long enough to hide them and the
+  // two waits between streams: an R-MAT of 65,536 vertices and 32 columns (134 MB
+  // of costs) 1,833 -> 1,724 us a match, a uniform graph of 20,000 and 30 FP64
+  // columns (98 MB) 1,759 -> 1,685; one of 1,000 (1.6 MB) 480 -> 514.  Recording
+  // copies the statistics on s, and phase timing includes them.
+  const bool beside = !P->rec && !P->kernel_timing && (double)D->De * Pp * sizeof(T) >= 90e6;
+  if (beside && t > 1) ACG_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_stats, 0));
   if constexpr (std::is_same_v<T, double>) ACG_TRY(launch_vertex_fx(va, P->vert_blocks, s));
   else ACG_TRY(launch_vertex_update<T>(va, P->vert_blocks, s));
+  const cudaStream_t fs = beside ? P->side : s;
+  if (beside) {
+    ACG_CUDA_TRY(cudaEventRecord(P->ev_vertex, s));
+    ACG_CUDA_TRY(cudaStreamWaitEvent(fs, P->ev_vertex, 0));
+  }
+  if constexpr (sizeof(T) == 4)
+    if (wide) ACG_TRY(launch_wide_partials(va, P->vert_blocks, fs));
   ACG_TRY(launch_finalize(P->bpart, P->vert_blocks,
-                          StatSpec{2 * Pe, 2 * Pe + Pn, P->prec != ACG_PREC_FP64}, P->gi[t & 1], s));
-  ACG_TRY(launch_capture_s(P->gi[t & 1] + 4 * Pe, P->iters_p, t, P->S_final, Pn, s));
+                          StatSpec{2 * Pe, 2 * Pe + Pn, P->prec != ACG_PREC_FP64}, P->gi[t & 1], fs,
+                          StatCapture{P->iters_p, P->S_final, 4 * Pe, t}));
+  if (beside) {
+    ACG_CUDA_TRY(cudaEventRecord(P->ev_stats, fs));
+    if (t == P->iters) ACG_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_stats, 0));
+  }
   if (rec)
     ACG_CUDA_TRY(cudaMemcpyAsync(P->rec->glob[t], P->gi[t & 1], sizeof(double) * glob_doubles(Pn, Pe),
                                  cudaMemcpyDeviceToDevice, s));
   if (P->kernel_timing) cudaEventRecord(P->kev[3 * (t - 1) + 2], s);
-  P->launches += 3;
+  P->launches += 2 + wide;
   return ACG_OK;
 }
 
@@ -682,6 +702,14 @@ static acg_status get_work(acg_data* D, int which, int nwarps, int step, WarpWor
   return ACG_OK;
 }
 
+void side_free(acg_plan* P) {
+  if (P->side) cudaStreamDestroy(P->side);
+  if (P->ev_vertex) cudaEventDestroy(P->ev_vertex);
+  if (P->ev_stats) cudaEventDestroy(P->ev_stats);
+  P->side = nullptr;
+  P->ev_vertex = P->ev_stats = nullptr;
+}
+
 acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& o, cudaStream_t s,
                             bool deferred, acg_plan** out) {
   std::unique_ptr<acg_plan> P(new acg_plan());
@@ -694,6 +722,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
         if (e) cudaEventDestroy(e);
       for (auto& e : p->kev)
         if (e) cudaEventDestroy(e);
+      side_free(p);
     }
   } guard{P.get()};
   P->data = D;
@@ -870,6 +899,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
   big((size_t)Dn * P->Pnp * eb, &P->CV);
   if (P->prec == ACG_PREC_MIXED) big((size_t)Dn * P->Pnp * eb, &P->CVlo);
   big(vrow, &P->M);
+  big(sizeof(float) * std::max<size_t>(1, eb == 4 ? wide_rowpart_floats(Pp, P->vert_blocks) : 0), &P->rowpart);
   big((size_t)std::max(1, P->ew.npartial) * Pp * eb, &P->part_iter);
   big((size_t)std::max(1, P->sw.npartial) * (3 * Pp + P->Pqc) * eb, &P->part_src);
   if (!deferred && st == ACG_OK) {
@@ -905,6 +935,13 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
   if (st != ACG_OK) return fail(st);
   for (auto& e : P->ev)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(set_error(ACG_ERR_CUDA, "cudaEventCreate failed"));
+  {  // the highest priority: its few blocks start before the edge phase's fill the SMs
+    int lo = 0, hi = 0;
+    ACG_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    ACG_CUDA_TRY(cudaStreamCreateWithPriority(&P->side, cudaStreamNonBlocking, hi));
+    ACG_CUDA_TRY(cudaEventCreateWithFlags(&P->ev_vertex, cudaEventDisableTiming));
+    ACG_CUDA_TRY(cudaEventCreateWithFlags(&P->ev_stats, cudaEventDisableTiming));
+  }
   P->kernel_timing = o.kernel_timing;
   if (P->kernel_timing) {
     P->kev.assign(3 * (size_t)P->iters, nullptr);
@@ -1064,6 +1101,7 @@ acg_status acg_plan_destroy(acg_plan* P) {
   for (auto& e : P->kev)
     if (e) cudaEventDestroy(e);
   dev_free_all(&P->owned);
+  side_free(P);
   delete P;
   return ACG_OK;
 }

@@ -131,7 +131,7 @@ __device__ void block_partials_out(const double* red, int nwarps, StatSpec spec,
 // ------------------------------------------------------------- finalize
 __global__ void __launch_bounds__(256)
 stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spec,
-                     double* __restrict__ out) {
+                     double* __restrict__ out, const StatCapture cap) {
   __shared__ double sm[8], ss[8];
   const int o = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -174,7 +174,10 @@ stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spe
     if (threadIdx.x == 0) {
       double t = 0.0;
       for (int k = 0; k < 8; ++k) t += ss[k];
-      out[o] = (m > -CUDART_INF && t > 0.0) ? m + log(t) : -CUDART_INF;
+      const double r = (m > -CUDART_INF && t > 0.0) ? m + log(t) : -CUDART_INF;
+      out[o] = r;
+      const int p = o - cap.first;
+      if (cap.iters_p && p >= 0 && cap.iters_p[p] == cap.t) cap.S_final[p] = r;
     }
   }
 }
@@ -398,10 +401,10 @@ acg_status launch_init_vertex(const InitArgs<T>& a, GroupShape gs, int blocks, c
 }
 
 acg_status launch_finalize(const double* bpart, int nblocks, StatSpec spec, double* out,
-                           cudaStream_t s) {
+                           cudaStream_t s, const StatCapture& cap) {
   const int n = spec.outs();
   if (n == 0) return ACG_OK;
-  stat_finalize_kernel<<<n, 256, 0, s>>>(bpart, nblocks, spec, out);
+  stat_finalize_kernel<<<n, 256, 0, s>>>(bpart, nblocks, spec, out, cap);
   ACG_LAUNCH_CHECK();
   return ACG_OK;
 }

@@ -33,8 +33,15 @@ struct GroupShape {
 };
 GroupShape choose_shape(int elem_bytes, int pp, int pn);
 
+// Also, from output `first` on (S[p], the column log-sum-exp of MU_raw):
+// S_final[p] = S[p] where iteration t is the last of pattern vertex p.
+struct StatCapture {
+  const int* iters_p = nullptr;
+  double* S_final = nullptr;
+  int first = 0, t = 0;
+};
 acg_status launch_finalize(const double* bpart, int nblocks, StatSpec spec, double* out,
-                           cudaStream_t s);
+                           cudaStream_t s, const StatCapture& cap = StatCapture());
 
 // dst[i][k] = (float)src[row ? row[i] : i][k] for k < K, zero up to kstride.
 acg_status launch_convert_rows(const double* src, const int* row, long long n, int K, float* dst,

@@ -1242,12 +1242,6 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
   write_block_partials(red, kVw, nmax, nlse, a.bpart, gridDim.x, blockIdx.x, sizeof(T) == 4);
 }
 
-__global__ void capture_s_kernel(const double* __restrict__ S, const int* __restrict__ iters_p,
-                                 int t, double* __restrict__ S_final, int Pn) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < Pn && iters_p[p] == t) S_final[p] = S[p];
-}
-
 template <typename T>
 __global__ void fill_kernel(T* __restrict__ p, size_t n, T v) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -1401,14 +1395,6 @@ int vertex_update_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sm
 
 int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out) {
   return vertex_warp_schedule(pat, pn, pe, pp, pnp, kVps, out);
-}
-
-acg_status launch_capture_s(const double* S, const int* iters_p, int t, double* S_final, int Pn,
-                            cudaStream_t s) {
-  if (Pn == 0) return ACG_OK;
-  capture_s_kernel<<<ceil_div(Pn, 128), 128, 0, s>>>(S, iters_p, t, S_final, Pn);
-  ACG_LAUNCH_CHECK();
-  return ACG_OK;
 }
 
 template <typename T>

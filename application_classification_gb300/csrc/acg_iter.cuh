@@ -91,6 +91,7 @@ struct VertexUpdArgs {
   // MU_raw sums of one stage, [vterms][32] (vertex_warp_schedule)
   const uint32_t* vsched = nullptr;
   int vterms = 0;
+  float* rowpart = nullptr;  // acg_vertex_wide.cu: the rows' statistics (wide_rowpart_floats)
   const double* lse_pos = nullptr;  // [Pn] LSE_v(dV), which bounds |CV| (FP64 only)
   int* wide = nullptr;              // FP64: Z is stored as edge_word stores it
 };
@@ -106,15 +107,13 @@ int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::v
 // gives them.
 int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
 acg_status launch_vertex_wide(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s);
+size_t wide_rowpart_floats(int pp, int blocks);
+// The block partials (bpart) of a wide launch from its rows' statistics.
+acg_status launch_wide_partials(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s);
 int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
 int vertex_fx_warps(int pn, int pp);  // warps that share a stage
 acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s);
 int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms);
-// S_final[p] = S[p] of this iteration where it is p's last (S = the column
-// log-sum-exp of MU_raw in the statistics just finalised).
-acg_status launch_capture_s(const double* S, const int* iters_p, int t, double* S_final, int Pn,
-                            cudaStream_t s);
-
 // Edge phase of FP32 plans with the costs recomputed on the tensor cores
 // (acg_edge_tc.cu): M[v][q] = max over in-edges e of z[s_e][q] - ||x_e - y_q||,
 // d formed as the tensor-core edge cost matrix forms it.  One CTA per part of

@@ -109,6 +109,7 @@ struct acg_plan {
   void* M = nullptr;           // [Dn][Pp] edge-phase maxima
   void* part_iter = nullptr;
   void* part_src = nullptr;    // [sw.npartial][3 Pp + Pqc] chunk rows of the source-side pass
+  void* rowpart = nullptr;     // wide FP32 vertex phase: its rows' statistics
   double* bpart = nullptr;
   double* gv = nullptr;        // [3 Pn]
   double* ge = nullptr;        // [max(Pe, Pqc)]
@@ -119,6 +120,11 @@ struct acg_plan {
   cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   int kernel_timing = 0;
   std::vector<cudaEvent_t> kev;  // [3 * iters] around each iteration's phases
+  // The statistics of an iteration are combined on `side`, beside the next edge
+  // phase, which does not read them: it waits for ev_vertex, and the next vertex
+  // phase (and the output) for ev_stats.
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_vertex = nullptr, ev_stats = nullptr;
   cudaStream_t last_stream = nullptr;
   int64_t launches = 0;
   bool ran = false;
@@ -192,6 +198,9 @@ acg_status run_iteration_any(acg_plan* P, int t, double* mu_out, cudaStream_t s)
 // The C-null term of a plan with the cnull option (acg_cnull.cu), from its dE.
 acg_status run_cnull(acg_plan* P, cudaStream_t s);
 int cnull_blocks(int num_sms);
+
+// Destroys a plan's side stream and its events (no work pending on them).
+void side_free(acg_plan* P);
 
 // Frees the adjoint's buffers of a plan (acg_adjoint.cu).
 void adj_free(acg_plan* P);

@@ -15,7 +15,11 @@
 // A thread's columns, rows and pattern vertices, and the order of every sum, are
 // those of the tile form: a block of V = 256 / (Pp / 4) rows walks the tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ...
-// R-MAT 18, pattern 40/120 (0.84 GB, 124 us at the copy bandwidth): WIDE_FIGURES.
+// R-MAT 18, pattern 40/120 (0.84 GB, 124 us at the copy bandwidth): 458 us an
+// iteration as block tiles, 234 so (and 100 of merges beside the edge phase);
+// 131,072 vertices, patterns of 132 to 192 columns: 284 -> 190 us.  Two columns a
+// lane with twice the warps was slower (435 us: the copies, the schedule and the
+// barriers are per warp), and so were constants held in registers (326).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -45,9 +49,7 @@ struct WideSmem {
     cst = o; o += w16(sizeof(float) * (size_t)10 * Pp);
     stage = sizeof(float) * (size_t)VwStage(Pp, Pnp, true, kWv).n;
     row_ring = 2 * stage;
-    // the ring becomes the reduction area: 6 doubles per row and lane, or 2 per thread
-    const size_t red = sizeof(double) * std::max((size_t)6 * V * (Pp / 4), (size_t)2 * kTileThreads);
-    ring = o; o += w16(std::max(red, V * row_ring));
+    ring = o; o += w16(V * row_ring);
     mu_row = (Pn + 31) / 32 * 32 + 1;  // (the schedule's slots)
     mu_n = (size_t)kWv * mu_row;
     mu = o; o += w16(sizeof(float) * 2 * 2 * V * mu_n);  // two stages: hi, lo of each row
@@ -337,47 +339,53 @@ __global__ void __launch_bounds__(kThreads, kBlocks) vertex_wide_kernel(const Ve
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 
-  // ---- block partials: mVF, mVR (max), lR, lF, S (lse); rows combined in order
-  double* s_red = reinterpret_cast<double*>(smem + L.ring);
-  const int nmax = 2 * Pe;
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    __syncthreads();
-    if (qon) {
-      double* e = s_red + (size_t)(row * nvec + gl) * 6;
-      e[0] = (double)mxF[w];
-      e[1] = (double)mxR[w];
-      e[2] = lr[w].mval();
-      e[3] = lr[w].sval();
-      e[4] = lf[w].mval();
-      e[5] = lf[w].sval();
-    }
-    __syncthreads();
-    for (int c = tid; c < 2 * nvec; c += nt) {  // (vector, statistic): VF's, VR's
-      const int i = c >> 1, k = c & 1, q = i * 4 + w;
-      if (q >= Pe) continue;
-      double f = -CUDART_INF, m = -CUDART_INF, s = 0;
-      for (int j = 0; j < V; ++j) {
-        const double* x = s_red + (size_t)(j * nvec + i) * 6;
-        f = fmax(f, x[k]);
-        lse_merge(m, s, x[2 + 2 * k], x[3 + 2 * k]);
-      }
-      a.bpart[(size_t)(k * Pe + q) * gx + bx] = f;
-      a.bpart[(size_t)(nmax + 2 * (k * Pe + q)) * gx + bx] = m;
-      a.bpart[(size_t)(nmax + 2 * (k * Pe + q) + 1) * gx + bx] = s;
-    }
+  // ---- the rows' statistics, merged by wide_partials_kernel
+  if (qon) {
+    float* rp = a.rowpart + (size_t)(bx * V + row) * 8 * Pp + qo;
+    auto put = [&](int i, float x0, float x1, float x2, float x3) { st4(rp + (size_t)i * Pp, {x0, x1, x2, x3}); };
+    put(0, mxF[0], mxF[1], mxF[2], mxF[3]);
+    put(1, lr[0].m, lr[1].m, lr[2].m, lr[3].m);
+    put(2, lr[0].s, lr[1].s, lr[2].s, lr[3].s);
+    put(3, lr[0].c, lr[1].c, lr[2].c, lr[3].c);
+    put(4, mxR[0], mxR[1], mxR[2], mxR[3]);
+    put(5, lf[0].m, lf[1].m, lf[2].m, lf[3].m);
+    put(6, lf[0].s, lf[1].s, lf[2].s, lf[3].s);
+    put(7, lf[0].c, lf[1].c, lf[2].c, lf[3].c);
   }
-  __syncthreads();
   if (tid < kTileThreads) {
-    s_red[tid * 2] = lmu.mval();
-    s_red[tid * 2 + 1] = lmu.sval();
+    float* rm = a.rowpart + (size_t)gx * V * 8 * Pp + (size_t)bx * 3 * kTileThreads + tid;
+    rm[0] = lmu.m;
+    rm[kTileThreads] = lmu.s;
+    rm[2 * kTileThreads] = lmu.c;
   }
-  __syncthreads();
-  for (int p = tid; p < Pn; p += nt) {
+}
+
+// Block b's partials from its rows' statistics: mVF, mVR (max), lR, lF, S (lse),
+// rows combined in order.  The merges are FP64 exponentials, 37 us of the FP64
+// pipe at 120 columns; as a launch of their own they run beside the next edge
+// phase, which does not read them.
+__global__ void __launch_bounds__(256)
+wide_partials_kernel(const float* __restrict__ rowpart, int V, int Pe, int Pn, int Pp,
+                     double* __restrict__ bpart) {
+  const int bx = blockIdx.x, gx = gridDim.x, nmax = 2 * Pe, prows = kTileThreads / Pn;
+  for (int j = threadIdx.x; j < 2 * Pe + Pn; j += 256) {
     double m = -CUDART_INF, s = 0;
-    for (int j = 0; j < prows; ++j) lse_merge(m, s, s_red[(j * Pn + p) * 2], s_red[(j * Pn + p) * 2 + 1]);
-    a.bpart[(size_t)(nmax + 2 * (2 * Pe + p)) * gx + bx] = m;
-    a.bpart[(size_t)(nmax + 2 * (2 * Pe + p) + 1) * gx + bx] = s;
+    if (j < 2 * Pe) {
+      const int k = j >= Pe, q = j - k * Pe;
+      double f = -CUDART_INF;
+      const float* rp = rowpart + (size_t)bx * V * 8 * Pp + (size_t)4 * k * Pp + q;
+      for (int r = 0; r < V; ++r, rp += 8 * Pp) {
+        f = fmax(f, (double)rp[0]);
+        lse_merge(m, s, (double)rp[Pp], (double)rp[2 * Pp] - (double)rp[3 * Pp]);
+      }
+      bpart[(size_t)j * gx + bx] = f;
+    } else {
+      const float* rm = rowpart + (size_t)gx * V * 8 * Pp + (size_t)bx * 3 * kTileThreads + (j - 2 * Pe);
+      for (int r = 0; r < prows; ++r, rm += Pn)
+        lse_merge(m, s, (double)rm[0], (double)rm[kTileThreads] - (double)rm[2 * kTileThreads]);
+    }
+    bpart[(size_t)(nmax + 2 * j) * gx + bx] = m;
+    bpart[(size_t)(nmax + 2 * j + 1) * gx + bx] = s;
   }
 }
 
@@ -398,6 +406,16 @@ acg_status launch_wide(const VertexUpdArgs<float>& a, int V, int blocks, cudaStr
 
 int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out) {
   return vertex_warp_schedule(pat, pn, pe, pp, pnp, kWv, out, 32 * wide_warps(pp), 4);
+}
+
+size_t wide_rowpart_floats(int pp, int blocks) {
+  return pp <= 64 ? 0 : (size_t)blocks * ((size_t)kTileThreads / (pp / 4) * 8 * pp + 3 * kTileThreads);
+}
+
+acg_status launch_wide_partials(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s) {
+  wide_partials_kernel<<<blocks, 256, 0, s>>>(a.rowpart, kTileThreads / (a.Pp / 4), a.Pe, a.Pn, a.Pp, a.bpart);
+  ACG_LAUNCH_CHECK();
+  return ACG_OK;
 }
 
 acg_status launch_vertex_wide(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s) {
