@@ -134,7 +134,7 @@ __device__ __forceinline__ T ag(const typename AV<T>::type& v, int w) {
   return reinterpret_cast<const T*>(&v)[w];
 }
 __device__ __forceinline__ float ex(float x) { return expf(x); }
-__device__ __forceinline__ double ex(double x) { return exp(x); }
+__device__ __forceinline__ double ex(double x) { return fx_expd(x); }  // (integer pipes)
 
 // ------------------------------------------------------------ column helpers
 // Block partials of per-lane column values: red[warp][col] in shared memory is
@@ -382,6 +382,12 @@ struct StepAArgs {
   const double* cnull;  // [Pe] the C-null term subtracted from both fills (option cnull), or null
 };
 
+// Vertices whose rows a warp loads together in the step kernels.
+template <typename T, int QPL>
+constexpr int step_unroll() {
+  return sizeof(T) * QPL <= 4 ? 4 : 2;
+}
+
 template <typename T, int QPL, int PPL>
 __global__ void __launch_bounds__(kT) adj_stepA_kernel(const StepAArgs<T> a) {
   extern __shared__ __align__(16) unsigned char sm[];
@@ -431,52 +437,86 @@ __global__ void __launch_bounds__(kT) adj_stepA_kernel(const StepAArgs<T> a) {
   }
   const long long nw = (long long)gridDim.x * kW, gw = (long long)blockIdx.x * kW + wib;
   const int vb = (int)(gw * a.Dn / nw), ve = (int)((gw + 1) * a.Dn / nw);
-  for (int v = vb; v < ve; ++v) {
+  // The rows of kUn vertices are loaded before the first is worked on: one
+  // vertex at a time waited out a memory latency each (R-MAT 16, 24 columns: step
+  // A 58 -> 45 us, step B 61 -> 28 us).
+  constexpr int kUn = step_unroll<T, QPL>();
+  for (int v0 = vb; v0 < ve; v0 += kUn) {
+    T mu[kUn][PPL], cv[kUn][PPL], gf[kUn][QPL], gr[kUn][QPL], fv[kUn][QPL], rv_[kUn][QPL], em[kUn][QPL],
+        mv[kUn][QPL], ge[kUn][QPL];
 #pragma unroll
-    for (int j = 0; j < PPL; ++j) {
-      const int p = lane + 32 * j;
-      if (p < Pn) {
-        const T x = a.gMU[(size_t)v * Pn + p];
-        sg[p] = x;
-        a.gCV[(size_t)v * Pn + p] -= x;
+    for (int u = 0; u < kUn; ++u) {
+      const int v = v0 + u;
+      const bool on = v < ve;
+#pragma unroll
+      for (int j = 0; j < PPL; ++j) {
+        const int p = lane + 32 * j;
+        const bool ok = on && p < Pn;
+        mu[u][j] = ok ? a.gMU[(size_t)v * Pn + p] : T(0);
+        cv[u][j] = ok ? a.gCV[(size_t)v * Pn + p] : T(0);
+      }
+#pragma unroll
+      for (int k = 0; k < QPL; ++k) {
+        const bool ok = on && qo + k < Pe;
+        const size_t i = (size_t)v * Pp + qo + k;
+        gf[u][k] = ok && a.gFd ? a.gFd[i] : T(0);
+        gr[u][k] = ok && a.gRd ? a.gRd[i] : T(0);
+        fv[u][k] = ok ? a.f[i] : T(0);
+        rv_[u][k] = ok ? a.r[i] : T(0);
+        em[u][k] = ok ? a.dEmin[i] : T(0);
+        mv[u][k] = ok ? a.M[i] : T(0);
+        ge[u][k] = ok ? a.gdEmin[i] : T(0);
       }
     }
-    __syncwarp();
 #pragma unroll
-    for (int k = 0; k < QPL; ++k) {
-      const int q = qo + k;
-      if (q >= Pe) continue;
-      const size_t i = (size_t)v * Pp + q;
-      const T gF = sg[qd[k]] + (a.gFd ? a.gFd[i] : T(0));
-      const T gR = sg[qs[k]] + (a.gRd ? a.gRd[i] : T(0));
-      const T f = a.f[i], r = a.r[i];
-      const T Y = f - a.dEmin[i];
-      const bool sR = ((Y - dRh[k]) - dRl[k]) > fR[k];
-      const bool sF = ((a.M[i] - dFh[k]) - dFl[k]) > fF[k];
-      const T gb = sR ? gR : T(0), gm = sF ? gF : T(0);
-      a.gbR[i] = gb;
-      a.gM[i] = gm;
-      // the maximum's -dE term: each (edge, column) is the maximum of one vertex
-      if (gm != T(0)) {
-        const int e = __ldg(a.A + i);
-        a.gdE[(size_t)e * Pp + q] -= gm;
-        atomicOr(a.emask + e, 1ull << q);
+    for (int u = 0; u < kUn; ++u) {
+      const int v = v0 + u;
+      if (v >= ve) break;
+#pragma unroll
+      for (int j = 0; j < PPL; ++j) {
+        const int p = lane + 32 * j;
+        if (p < Pn) {
+          sg[p] = mu[u][j];
+          a.gCV[(size_t)v * Pn + p] = cv[u][j] - mu[u][j];
+        }
       }
-      a.gdEmin[i] -= gb;
-      sa[k][0] += sR ? 0.0 : (double)gR;
-      sa[k][1] += sF ? 0.0 : (double)gF;
-      sa[k][2] += (double)gb;
-      sa[k][3] += (double)gm;
-      if (af[k] < 0 || f > bf[k]) {
-        bf[k] = f;
-        af[k] = v;
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < QPL; ++k) {
+        const int q = qo + k;
+        if (q >= Pe) continue;
+        const size_t i = (size_t)v * Pp + q;
+        const T gF = sg[qd[k]] + gf[u][k];
+        const T gR = sg[qs[k]] + gr[u][k];
+        const T f = fv[u][k], r = rv_[u][k];
+        const T Y = f - em[u][k];
+        const bool sR = ((Y - dRh[k]) - dRl[k]) > fR[k];
+        const bool sF = ((mv[u][k] - dFh[k]) - dFl[k]) > fF[k];
+        const T gb = sR ? gR : T(0), gm = sF ? gF : T(0);
+        a.gbR[i] = gb;
+        a.gM[i] = gm;
+        // the maximum's -dE term: each (edge, column) is the maximum of one vertex
+        if (gm != T(0)) {
+          const int e = __ldg(a.A + i);
+          a.gdE[(size_t)e * Pp + q] -= gm;
+          atomicOr(a.emask + e, 1ull << q);
+        }
+        a.gdEmin[i] = ge[u][k] - gb;
+        sa[k][0] += sR ? 0.0 : (double)gR;
+        sa[k][1] += sF ? 0.0 : (double)gF;
+        sa[k][2] += (double)gb;
+        sa[k][3] += (double)gm;
+        if (af[k] < 0 || f > bf[k]) {
+          bf[k] = f;
+          af[k] = v;
+        }
+        if (ar[k] < 0 || r > br[k]) {
+          br[k] = r;
+          ar[k] = v;
+        }
       }
-      if (ar[k] < 0 || r > br[k]) {
-        br[k] = r;
-        ar[k] = v;
-      }
+      __syncwarp();
     }
-    __syncwarp();
   }
 #pragma unroll
   for (int k = 0; k < QPL; ++k) {
@@ -588,43 +628,71 @@ __global__ void __launch_bounds__(kT) adj_stepB_kernel(const StepBArgs<T> a) {
   __syncthreads();
   const long long nw = (long long)gridDim.x * kW, gw = (long long)blockIdx.x * kW + wib;
   const int vb = (int)(gw * a.Dn / nw), ve = (int)((gw + 1) * a.Dn / nw);
-  for (int v = vb; v < ve; ++v) {
+  constexpr int kUn = step_unroll<T, QPL>();
+  for (int v0 = vb; v0 < ve; v0 += kUn) {
+    T bv[kUn][QPL], fv[kUn][QPL], rv[kUn][QPL], gbr[kUn][QPL], gvre[kUn][QPL], gbv[kUn][QPL], hv[kUn][PPL],
+        lv[kUn][PPL];
 #pragma unroll
-    for (int k = 0; k < QPL; ++k) {
-      const int q = qo + k;
-      if (q >= Pp) continue;
-      const size_t i = (size_t)v * Pp + q;
-      T gvf = T(0), gvr = T(0);
-      if (q < Pe) {
-        const T b = a.B[i];
-        // softmax weights of the log-sum-exps (no out-edges: B = -inf, weight 0)
-        const bool hb = b > neg_inf<T>();
-        const T wR = hb ? ex(((a.f[i] + b) - dRh[k]) - dRl[k]) : T(0);
-        const T wF = hb ? ex(((a.r[i] + b) - dFh[k]) - dFl[k]) : T(0);
-        gvf = a.gbR[i] + (v == vfa[k] ? gaR[k] : T(0)) + glR[k] * wR;
-        gvr = a.gVRe[i] + (v == vra[k] ? gaF[k] : T(0)) + glF[k] * wF;
-        a.gB[i] += glR[k] * wR + glF[k] * wF;
-      }
-      a.gFd[i] = -gvf;
-      a.gRd[i] = -gvr;
-      sgr[q] = gvf;
-      sgr[32 * QPL + q] = gvr;
-    }
-    __syncwarp();
+    for (int u = 0; u < kUn; ++u) {
+      const int v = v0 + u;
+      const bool on = v < ve;
 #pragma unroll
-    for (int j = 0; j < PPL; ++j) {
-      const int p = lane + 32 * j;
-      if (p >= Pn) continue;
-      T acc = T(0);
-      const int* inc = s_inc + j * maxdeg * 32 + lane;
-      for (int t = 0; t < maxdeg; ++t) acc += sgr[inc[t * 32]];
-      if (a.mh) {
-        const size_t i = (size_t)v * Pn + p;
-        acc += gS[j] * ex((a.mh[i] - Sh[j]) + (a.ml[i] - Sl[j]));
+      for (int k = 0; k < QPL; ++k) {
+        const bool ok = on && qo + k < Pe;
+        const size_t i = (size_t)v * Pp + qo + k;
+        bv[u][k] = ok ? a.B[i] : T(0);
+        fv[u][k] = ok ? a.f[i] : T(0);
+        rv[u][k] = ok ? a.r[i] : T(0);
+        gbr[u][k] = ok ? a.gbR[i] : T(0);
+        gvre[u][k] = ok ? a.gVRe[i] : T(0);
+        gbv[u][k] = ok ? a.gB[i] : T(0);
       }
-      a.gMU[(size_t)v * Pn + p] = acc;
+#pragma unroll
+      for (int j = 0; j < PPL; ++j) {
+        const int p = lane + 32 * j;
+        const bool ok = on && p < Pn && a.mh;
+        hv[u][j] = ok ? a.mh[(size_t)v * Pn + p] : T(0);
+        lv[u][j] = ok ? a.ml[(size_t)v * Pn + p] : T(0);
+      }
     }
-    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kUn; ++u) {
+      const int v = v0 + u;
+      if (v >= ve) break;
+#pragma unroll
+      for (int k = 0; k < QPL; ++k) {
+        const int q = qo + k;
+        if (q >= Pp) continue;
+        const size_t i = (size_t)v * Pp + q;
+        T gvf = T(0), gvr = T(0);
+        if (q < Pe) {
+          const T b = bv[u][k];
+          // softmax weights of the log-sum-exps (no out-edges: B = -inf, weight 0)
+          const bool hb = b > neg_inf<T>();
+          const T wR = hb ? ex(((fv[u][k] + b) - dRh[k]) - dRl[k]) : T(0);
+          const T wF = hb ? ex(((rv[u][k] + b) - dFh[k]) - dFl[k]) : T(0);
+          gvf = gbr[u][k] + (v == vfa[k] ? gaR[k] : T(0)) + glR[k] * wR;
+          gvr = gvre[u][k] + (v == vra[k] ? gaF[k] : T(0)) + glF[k] * wF;
+          a.gB[i] = gbv[u][k] + (glR[k] * wR + glF[k] * wF);
+        }
+        a.gFd[i] = -gvf;
+        a.gRd[i] = -gvr;
+        sgr[q] = gvf;
+        sgr[32 * QPL + q] = gvr;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < PPL; ++j) {
+        const int p = lane + 32 * j;
+        if (p >= Pn) continue;
+        T acc = T(0);
+        const int* inc = s_inc + j * maxdeg * 32 + lane;
+        for (int t = 0; t < maxdeg; ++t) acc += sgr[inc[t * 32]];
+        if (a.mh) acc += gS[j] * ex((hv[u][j] - Sh[j]) + (lv[u][j] - Sl[j]));
+        a.gMU[(size_t)v * Pn + p] = acc;
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -835,7 +903,10 @@ __global__ void __launch_bounds__(kT) adj_quirk_dst_kernel(const QuirkArgs<T> a)
         const size_t i = (size_t)e * Pp + q;
         const T d = a.dE[i];
         const T buf = c ? -d : T(0);
-        if (c) a.gdE[i] -= (T)(gl[k] * exp((double)buf - lb[k]));
+        if (c) {
+          if constexpr (sizeof(T) == 8) a.gdE[i] -= gl[k] * ex(buf - lb[k]);
+          else a.gdE[i] -= (T)(gl[k] * exp((double)buf - lb[k]));
+        }
         if (pos[k] < 0 || buf > best[k]) {
           best[k] = buf;
           pos[k] = e;
@@ -1067,14 +1138,15 @@ __global__ void adj_dv_kernel(T* __restrict__ gMU0, const T* __restrict__ gCV, c
 }
 
 // ------------------------------------------------------------------ cdist
-// One thread per row r of d = ||x_row(r) - y_q||: recomputes d in the forward's
-// arithmetic, writes rr = g / d in place of g (0 where d = 0) and the row's
+// One thread per row r of d = ||x_row(r) - y_q||: recomputes d (FP64 edges: reads
+// the forward's, which halves the FP64 instructions a pair; R-MAT 14, 24 columns
+// 902 -> 560 us), writes rr = g / d in place of g (0 where d = 0) and the row's
 // feature gradient sum_q rr (x - y_q) to out[orow(r)] (FP64).
 template <typename T, typename F, int KM>
 __global__ void __launch_bounds__(kT)
 adj_cdist_rows_kernel(const F* __restrict__ x, const int* __restrict__ row, int kstride, int K,
                       const double* __restrict__ y, int P, T* __restrict__ g, int ldg, long long nrows,
-                      const int* __restrict__ orow, double* __restrict__ out) {
+                      const int* __restrict__ orow, double* __restrict__ out, const T* __restrict__ dist) {
   extern __shared__ __align__(16) unsigned char sm[];
   T* s_y = reinterpret_cast<T*>(sm);  // [P][KM]
   for (int t = threadIdx.x; t < P * KM; t += kT) {
@@ -1092,14 +1164,31 @@ adj_cdist_rows_kernel(const F* __restrict__ x, const int* __restrict__ row, int 
     }
     T* gr = g + (size_t)r * ldg;
     for (int q = 0; q < P; ++q) {
-      T acc = T(0);
+      T rr;
+      if constexpr (sizeof(T) == 8) {
+        const T d = dist ? dist[(size_t)r * ldg + q] : T(0);
+        if (dist && d > T(0x1p-99)) {
+          rr = gr[q] / d;
+        } else {
+          T acc = T(0);
 #pragma unroll
-      for (int k = 0; k < KM; ++k) {
-        const T t = xr[k] - s_y[q * KM + k];
-        acc = fma(t, t, acc);
+          for (int k = 0; k < KM; ++k) {
+            const T t = xr[k] - s_y[q * KM + k];
+            acc = fma(t, t, acc);
+          }
+          const T d1 = sqrt(acc);
+          rr = d1 > T(0) ? gr[q] / d1 : T(0);
+        }
+      } else {
+        T acc = T(0);
+#pragma unroll
+        for (int k = 0; k < KM; ++k) {
+          const T t = xr[k] - s_y[q * KM + k];
+          acc = fma(t, t, acc);
+        }
+        const T d = sqrt(acc);
+        rr = d > T(0) ? gr[q] / d : T(0);
       }
-      const T d = sqrt(acc);
-      const T rr = d > T(0) ? gr[q] / d : T(0);
       gr[q] = rr;
 #pragma unroll
       for (int k = 0; k < KM; ++k) gx[k] += rr * (xr[k] - s_y[q * KM + k]);
@@ -1541,7 +1630,7 @@ struct Adj {
     T* g = (T*)(vertex ? W->gMU : W->gdE);
     const double* y = vertex ? P->pv : P->pe;
     if (K == 0 || nrows == 0 || P_ == 0) return ACG_OK;
-    const int km = (K + 3) / 4 * 4;
+    const int km = sizeof(T) == 8 ? (K + 1) / 2 * 2 : (K + 3) / 4 * 4;
     const size_t sm = sizeof(T) * (size_t)P_ * km;
     const int blocks = std::max(1, std::min(ceil_div(std::max<long long>(1, nrows), kT), nsm * 8));
     // data features: the FP32 copies (mixed; edges in destination-CSR order) or
@@ -1555,12 +1644,17 @@ struct Adj {
       constexpr int KM = decltype(kmc)::value;
       if constexpr (sizeof(T) == 4) {
         const float* x = vertex ? D->nf32 : D->ef32;
-        adj_cdist_rows_kernel<T, float, KM><<<blocks, kT, sm, s>>>(x, row, kstride, K, y, P_, g, ld, nrows, orow, gx);
+        adj_cdist_rows_kernel<T, float, KM><<<blocks, kT, sm, s>>>(x, row, kstride, K, y, P_, g, ld, nrows, orow, gx, nullptr);
       } else {
         const double* x = vertex ? D->node_feats : D->edge_feats;
-        adj_cdist_rows_kernel<T, double, KM><<<blocks, kT, sm, s>>>(x, row, kstride, K, y, P_, g, ld, nrows, orow, gx);
+        // the edge distances are at hand (row stride Pp, as the gradient's)
+        adj_cdist_rows_kernel<T, double, KM><<<blocks, kT, sm, s>>>(x, row, kstride, K, y, P_, g, ld, nrows,
+                                                                    orow, gx, vertex ? nullptr : (const T*)P->dE);
       }
       le = cudaGetLastError();
+    };
+    auto launch_even = [&](auto kmc) {
+      if constexpr (sizeof(T) == 8) launch(kmc);
     };
     switch (km) {
       case 4: launch(std::integral_constant<int, 4>{}); break;
@@ -1571,6 +1665,15 @@ struct Adj {
       case 24: launch(std::integral_constant<int, 24>{}); break;
       case 28: launch(std::integral_constant<int, 28>{}); break;
       case 32: launch(std::integral_constant<int, 32>{}); break;
+      // (FP64: two features a step, an unused one costs four FP64 instructions a pair)
+      case 2: launch_even(std::integral_constant<int, 2>{}); break;
+      case 6: launch_even(std::integral_constant<int, 6>{}); break;
+      case 10: launch_even(std::integral_constant<int, 10>{}); break;
+      case 14: launch_even(std::integral_constant<int, 14>{}); break;
+      case 18: launch_even(std::integral_constant<int, 18>{}); break;
+      case 22: launch_even(std::integral_constant<int, 22>{}); break;
+      case 26: launch_even(std::integral_constant<int, 26>{}); break;
+      case 30: launch_even(std::integral_constant<int, 30>{}); break;
       default: return set_error(ACG_ERR_UNSUPPORTED, "acg_backward: feature dimension %d above 32", K);
     }
     if (le != cudaSuccess) return set_error(ACG_ERR_CUDA, "adj_cdist_rows: %s", cudaGetErrorString(le));

@@ -328,6 +328,13 @@ acg_status acg::build_warp_work(const Csr& c, int nwarps, int step, WarpWork* ou
 
 namespace {
 
+// Whether an edge phase lasts long enough to hide the statistics beside it and the
+// two waits between streams, by the bytes of its costs: an R-MAT of 65,536
+// vertices and 32 columns (134 MB) 1,833 -> 1,724 us a match, a uniform graph of
+// 20,000 and 30 FP64 columns (98 MB) 1,759 -> 1,685; one of 1,000 (1.6 MB) 480 ->
+// 514.
+bool side_worthwhile(long long De, int Pp, int elem) { return (double)De * Pp * elem >= 90e6; }
+
 template <typename T>
 acg_status iterate(acg_plan* P, int t, double* mu_out, cudaStream_t s) {
   acg_data* D = P->data;
@@ -399,12 +406,9 @@ vertex_phase:
   va.wide = P->edge_wide;
   const bool wide = sizeof(T) == 4 && Pp > 64;
   if constexpr (sizeof(T) == 4) va.rowpart = (float*)P->rowpart;
-  // Beside the next edge phase where that lasts long enough to hide them and the
-  // two waits between streams: an R-MAT of 65,536 vertices and 32 columns (134 MB
-  // of costs) 1,833 -> 1,724 us a match, a uniform graph of 20,000 and 30 FP64
-  // columns (98 MB) 1,759 -> 1,685; one of 1,000 (1.6 MB) 480 -> 514.  Recording
-  // copies the statistics on s, and phase timing includes them.
-  const bool beside = !P->rec && !P->kernel_timing && (double)D->De * Pp * sizeof(T) >= 90e6;
+  // Beside the next edge phase (side_worthwhile); recording copies the statistics
+  // on s, and phase timing includes them.
+  const bool beside = P->side && !P->rec && !P->kernel_timing;
   if (beside && t > 1) ACG_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_stats, 0));
   if constexpr (std::is_same_v<T, double>) ACG_TRY(launch_vertex_fx(va, P->vert_blocks, s));
   else ACG_TRY(launch_vertex_update<T>(va, P->vert_blocks, s));
@@ -935,7 +939,8 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
   if (st != ACG_OK) return fail(st);
   for (auto& e : P->ev)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(set_error(ACG_ERR_CUDA, "cudaEventCreate failed"));
-  {  // the highest priority: its few blocks start before the edge phase's fill the SMs
+  if (side_worthwhile(De, Pp, eb)) {
+    // the highest priority: its few blocks start before the edge phase's fill the SMs
     int lo = 0, hi = 0;
     ACG_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     ACG_CUDA_TRY(cudaStreamCreateWithPriority(&P->side, cudaStreamNonBlocking, hi));

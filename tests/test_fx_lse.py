@@ -37,6 +37,10 @@ int main(int argc, char** argv) {
       const uint64_t f = fx_exp(fx_bits(x), k);
       const long double e = expl((long double)x - (long double)k * kLn2);
       worst = std::fmax(worst, (double)fabsl(ldexpl((long double)f, -61) / e - 1));
+      if (std::fabs(x) < 1000) {  // as a double: half a last place more
+        const long double w = expl((long double)x), r = (long double)fx_expd(x);
+        if (w > 0x1p-1000L && w < 0x1p1023L && fabsl(r / w - 1) > 4e-16L + (long double)std::fabs(x) * 0x1p-63L) worst = 1;
+      }
     }
     // the table form of fixed-point values, every scale in use
     static uint64_t tab[kFxTable];
