@@ -32,18 +32,26 @@ cnull_stats_kernel(const T* __restrict__ dE, long long De, int Pe, int Pp, int c
   const int c = threadIdx.x % cw, rl = threadIdx.x / cw;
   const int q = blockIdx.y * cw + c;
   const long long r0 = De * blockIdx.x / nb, r1 = De * (blockIdx.x + 1) / nb;
-  double mx = -CUDART_INF, lm, ls;
-  OnlineLse<double> l;  // integer arithmetic: no FP64 exponential per element
-  l.init();
+  double mx = -CUDART_INF, lm = -CUDART_INF, ls = 0.0;
   if (rl < rs && q < Pe) {
-    for (long long r = r0 + rl; r < r1; r += rs) {
-      const double x = (double)dE[(size_t)r * Pp + q];
-      mx = fmax(mx, x);
-      l.add(x);
+    if constexpr (sizeof(T) == 8) {
+      OnlineLse<double> l;  // integer arithmetic: no FP64 exponential per element
+      l.init();
+      for (long long r = r0 + rl; r < r1; r += rs) {
+        const double x = dE[(size_t)r * Pp + q];
+        mx = fmax(mx, x);
+        l.add(x);
+      }
+      lm = l.mval();
+      ls = l.sval();
+    } else {
+      for (long long r = r0 + rl; r < r1; r += rs) {
+        const double x = (double)dE[(size_t)r * Pp + q];
+        mx = fmax(mx, x);
+        lse_merge(lm, ls, x, 1.0);
+      }
     }
   }
-  lm = l.mval();
-  ls = l.sval();
   s_m[threadIdx.x] = mx;
   s_l[threadIdx.x] = lm;
   s_s[threadIdx.x] = ls;
