@@ -328,17 +328,38 @@ acg_status acg::build_warp_work(const Csr& c, int nwarps, int step, WarpWork* ou
 
 namespace {
 
-// Whether an edge phase lasts long enough to hide the statistics beside it and the
-// two waits between streams, by the bytes of its costs: an R-MAT of 65,536
-// vertices and 32 columns (134 MB) 1,833 -> 1,724 us a match, a uniform graph of
-// 20,000 and 30 FP64 columns (98 MB) 1,759 -> 1,685; one of 1,000 (1.6 MB) 480 ->
-// 514.
-bool side_worthwhile(long long De, int Pp, int elem) { return (double)De * Pp * elem >= 90e6; }
+// Whether to combine an iteration's statistics beside the next edge phase: in a
+// batch, whose captured graph makes the fork and join free, where that phase lasts
+// long enough (by the bytes of its costs).  R-MAT 17, 12 patterns: 187 -> 173 ms.
+// Launched one by one, the two waits between streams cost what they hide and keep
+// the next kernels from starting early (early_launches): R-MAT 18 with 120
+// columns 31.4 ms beside, 30.6 in line; a uniform graph of 30,011 FP64 4.48 and
+// 4.60.
+bool side_worthwhile(bool batch, long long De, int Pp, int elem) {
+  return batch && (double)De * Pp * elem >= 90e6;
+}
+
+// Whether kernels may start early (launch_kernel).  Not in plans whose statistics
+// run beside the edge phase: blocks of it waiting for their turn would keep those
+// off the SMs (R-MAT 17 batch 173 -> 189 ms).  And where the passes are short enough
+// for the gaps between them to count: R-MAT 16 mixed (134 MB of costs) 1.78 -> 1.70
+// ms, R-MAT 18 mixed (537 MB) 4.59 -> 4.51, 40/120 patterns on R-MAT 18 (2 GB)
+// 30.85 -> 30.75; but R-MAT 20 FP64 (8.6 GB) 132 -> 162 ms and R-MAT 22 mixed
+// (16.7 GB) 174 -> 180, where the blocks that wait take the place of running ones
+// for longer than a gap.
+template <typename T>
+bool early_launches(const acg_plan* P) {
+  return !P->side && (double)P->data->De * P->Pp * sizeof(T) < 3e9;
+}
 
 template <typename T>
 acg_status iterate(acg_plan* P, int t, double* mu_out, cudaStream_t s) {
   acg_data* D = P->data;
   const int Dn = D->Dn, Pn = P->Pn, Pe = P->Pe, Pp = P->Pp;
+  // Statistics beside the next edge phase (side_worthwhile); recording copies them
+  // on s, and phase timing includes them.
+  const bool beside = P->side && !P->rec && !P->kernel_timing;
+  const bool early = early_launches<T>(P) && !P->rec;
   if (P->kernel_timing) cudaEventRecord(P->kev[3 * (t - 1)], s);
   if constexpr (std::is_same_v<T, float>) {
     if (Pe > 0 && P->edge_tc && !P->rec) {  // costs recomputed on the tensor cores
@@ -356,6 +377,7 @@ acg_status iterate(acg_plan* P, int t, double* mu_out, cudaStream_t s) {
                       (const T*)P->dE, (const T*)P->vr[(t - 1) & 1], (T*)P->M,
                       (T*)P->part_iter, Pp};
     ea.Pe = Pe;
+    ea.early = early;
     ea.wide = P->edge_wide;
     ea.nranges = P->ew.nparts;
     ea.ctr = P->range_ctr;
@@ -381,7 +403,7 @@ acg_status iterate(acg_plan* P, int t, double* mu_out, cudaStream_t s) {
                                    cudaMemcpyDeviceToDevice, s));
     } else if (!inside) {
       ACG_TRY(launch_heavy_combine<T>((const T*)P->part_iter, P->ew.hbase, P->ew.hcount,
-                                      P->ew.hvert, P->ew.nheavy, Pp, (T*)P->M, s));
+                                      P->ew.hvert, P->ew.nheavy, Pp, (T*)P->M, early, s));
     }
     P->launches += 1 + (!inside && P->ew.nheavy > 0);
   }
@@ -404,11 +426,9 @@ vertex_phase:
   }
   va.lse_pos = P->gv + Pn;
   va.wide = P->edge_wide;
+  va.early = early;
   const bool wide = sizeof(T) == 4 && Pp > 64;
   if constexpr (sizeof(T) == 4) va.rowpart = (float*)P->rowpart;
-  // Beside the next edge phase (side_worthwhile); recording copies the statistics
-  // on s, and phase timing includes them.
-  const bool beside = P->side && !P->rec && !P->kernel_timing;
   if (beside && t > 1) ACG_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_stats, 0));
   if constexpr (std::is_same_v<T, double>) ACG_TRY(launch_vertex_fx(va, P->vert_blocks, s));
   else ACG_TRY(launch_vertex_update<T>(va, P->vert_blocks, s));
@@ -420,7 +440,7 @@ vertex_phase:
   if constexpr (sizeof(T) == 4)
     if (wide) ACG_TRY(launch_wide_partials(va, P->vert_blocks, fs));
   ACG_TRY(launch_finalize(P->bpart, P->vert_blocks,
-                          StatSpec{2 * Pe, 2 * Pe + Pn, P->prec != ACG_PREC_FP64}, P->gi[t & 1], fs,
+                          StatSpec{2 * Pe, 2 * Pe + Pn, P->prec == ACG_PREC_FP64 ? kMergeFx : kMergeF32, early}, P->gi[t & 1], fs,
                           StatCapture{P->iters_p, P->S_final, 4 * Pe, t}));
   if (beside) {
     ACG_CUDA_TRY(cudaEventRecord(P->ev_stats, fs));
@@ -462,6 +482,8 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
   const int Dn = D->Dn, Pn = P->Pn, Pe = P->Pe, Pp = P->Pp;
   const long long De = D->De;
   const long long lim = (long long)Pn * (long long)Dn;
+  const int once_merge = sizeof(T) == 8 ? kMergeFx : kMergeF64;
+  const bool early = early_launches<T>(P);
   P->launches = 0;
   cudaEventRecord(P->ev[0], s);
   if (P->fill_at_run) {  // shared workspaces: rows that no pass writes
@@ -489,6 +511,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
                        (T*)P->part_src, P->qlim_col, De, lim, Pp, P->Pqc, P->qcov};
     sa.nranges = P->sw.nparts;
     sa.ctr = P->range_ctr;
+    sa.early = early;
     ACG_TRY(launch_src_stats<T>(sa, P->ws, P->src_blocks, s));
     ACG_TRY(launch_src_stats_combine<T>(sa, P->sw, s));
     DstQuirkArgs<T> qa{P->ew.items, P->ew.nitems, P->ew.wsplit, D->dcsr.eid,
@@ -496,14 +519,15 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
                        (T*)P->Fq, (T*)P->part_iter, P->bpart, P->qlim_col, De, lim, Pp,
                        P->Pqc, P->qcov, P->ew.nparts};
     qa.dstride = P->dEq_cols;
+    qa.early = early;
     ACG_TRY(launch_dst_quirk<T>(qa, P->qws, P->edge_blocks, s));
     if (P->qcov > 0 && P->ew.nitems > 0) {  // ge[q < Pqc]; the later columns stay -inf
-      ACG_TRY(launch_finalize(P->bpart, P->edge_blocks, StatSpec{0, P->Pqc}, P->ge, s));
+      ACG_TRY(launch_finalize(P->bpart, P->edge_blocks, StatSpec{0, P->Pqc, once_merge, early}, P->ge, s));
       P->launches += 1;
     }
     if (P->qcov > 0)
       ACG_TRY(launch_heavy_combine<T>((const T*)P->part_iter, P->ew.hbase, P->ew.hcount,
-                                      P->ew.hvert, P->ew.nheavy, P->Pqc, (T*)P->Fq, s));
+                                      P->ew.hvert, P->ew.nheavy, P->Pqc, (T*)P->Fq, early, s));
     P->launches += 2 + (P->sw.nheavy > 0) + (P->qcov > 0 && P->ew.nheavy > 0);
   }
   // ---- init vertex pass
@@ -514,6 +538,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
                   (T*)P->vr[0], P->gv, P->ge, P->bpart, P->pat, De, lim, Dn, Pn, Pe, Pp,
                   P->Pnp, P->Pqc, P->qcov, P->qlim_col};
     a.wide = P->edge_wide;
+    a.early = early;
     const bool rec0 = P->rec && P->rec->has(0);
     if (rec0) {
       a.rec_f = (T*)P->rec->f[0];
@@ -527,7 +552,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
     // S = 0 (MU0 is normalised) and shifts 0 for the first pass
     ACG_CUDA_TRY(cudaMemsetAsync(P->gi[0] + 4 * Pe, 0,
                                  sizeof(double) * (glob_doubles(Pn, Pe) - 4 * Pe), s));
-    ACG_TRY(launch_finalize(P->bpart, P->init_blocks, StatSpec{2 * Pe, 2 * Pe}, P->gi[0], s));
+    ACG_TRY(launch_finalize(P->bpart, P->init_blocks, StatSpec{2 * Pe, 2 * Pe, once_merge, early}, P->gi[0], s));
     P->launches += 2;
     if (rec0) {
       ACG_CUDA_TRY(cudaMemcpyAsync(P->rec->r[0], P->vr[0], sizeof(T) * (size_t)Dn * Pp,
@@ -544,7 +569,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
   cudaEventRecord(P->ev[3], s);
   // ---- output [Dn][Pn] (main.cu:247 transpose is implicit in the layout)
   if (P->iters > 0 && !P->is_union) {
-    ACG_TRY(launch_mu_output(mu_out, P->S_final, Dn, Pn, s));
+    ACG_TRY(launch_mu_output(mu_out, P->S_final, Dn, Pn, early, s));
   } else if (P->iters == 0) {
     const long long n = (long long)Dn * Pn;
     if (n > 0) {
@@ -568,6 +593,7 @@ acg_status run_match(acg_plan* P, double* mu_out, cudaStream_t s, const UnionOut
 template <typename T, typename F>
 acg_status run_cdist(acg_plan* P, acg_data* D, long long lim, const F* nf, int nfs, const F* ef,
                      int efs, bool gather, cudaStream_t s) {
+  const bool early = early_launches<T>(P);
   int vcols = P->cv_blocks;  // partial columns of the vertex statistics
   bool vdone = false;
   if constexpr (std::is_same_v<T, float> && std::is_same_v<F, float>) {
@@ -581,6 +607,7 @@ acg_status run_cdist(acg_plan* P, acg_data* D, long long lim, const F* nf, int n
     if (cdist_fx_eligible(D->Kv)) {
       CdistRbArgs<double, double> av{nf, nullptr, nullptr, P->pv, (double*)P->CV, P->bpart, D->Dn, D->De, lim,
                                      D->Kv, nfs, P->Pn, P->Pnp, P->Pnp};
+      av.early = early;
       ACG_TRY(launch_cdist_vertex_fx(av, P->cv_blocks, s));
       vdone = true;
     }
@@ -590,11 +617,12 @@ acg_status run_cdist(acg_plan* P, acg_data* D, long long lim, const F* nf, int n
                          D->Kv, nfs, P->Pn, P->Pnp, P->Pnp};
     ACG_TRY(launch_cdist_rb(av, kCdistVertex, P->cv_blocks, s));
   }
-  ACG_TRY(launch_finalize(P->bpart, vcols, StatSpec{P->Pn, 2 * P->Pn}, P->gv, s));
+  ACG_TRY(launch_finalize(P->bpart, vcols, StatSpec{P->Pn, 2 * P->Pn, sizeof(T) == 8 ? kMergeFx : kMergeF64, early}, P->gv, s));
   // rows in dst-CSR order; with no data edges the kernel writes empty partials
   CdistRbArgs<T, F> ae{ef, gather ? D->dcsr.eid : nullptr, D->dcsr.eid, P->pe, (T*)P->dE,
                        nullptr, D->De, D->De, lim, D->Ke, efs, P->Pe, P->Pp, P->Pp};
   if (std::is_same_v<T, double>) ae.wide = P->edge_wide;
+  ae.early = early;
   if constexpr (std::is_same_v<T, float> && std::is_same_v<F, float>) {
     if (P->cdist_tc && P->edge_costs_ready) {  // written while the features were uploaded
       P->edge_costs_ready = false;
@@ -866,7 +894,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
       ACG_CUDA_TRY(cudaMemcpyAsync(P->vsched, vs.data(), sizeof(uint32_t) * vs.size(),
                                    cudaMemcpyHostToDevice, s));
     }
-    P->vert_blocks = eb == 8 ? vertex_fx_blocks(Pn, Pe, Pp, P->Pnp, P->vterms, nsm)
+    P->vert_blocks = eb == 8 ? vertex_fx_blocks(Pn, Pe, Pp, P->Pnp, P->vterms, nsm, Dn)
                              : vertex_update_blocks<float>(Pn, Pe, Pp, P->Pnp, P->vterms, nsm, Dn);
     if (o.vertex_blocks_per_sm > 0)
       P->vert_blocks = std::min(P->vert_blocks, nsm * o.vertex_blocks_per_sm);
@@ -939,7 +967,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
   if (st != ACG_OK) return fail(st);
   for (auto& e : P->ev)
     if (cudaEventCreate(&e) != cudaSuccess) return fail(set_error(ACG_ERR_CUDA, "cudaEventCreate failed"));
-  if (side_worthwhile(De, Pp, eb)) {
+  if (side_worthwhile(deferred, De, Pp, eb)) {
     // the highest priority: its few blocks start before the edge phase's fill the SMs
     int lo = 0, hi = 0;
     ACG_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));

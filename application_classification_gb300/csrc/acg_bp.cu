@@ -125,7 +125,7 @@ __device__ __forceinline__ void warp_group_lse(double& m, double& s) {
 // warps in order and write the block's partials [slot][ncols].
 __device__ void block_partials_out(const double* red, int nwarps, StatSpec spec,
                                    double* bpart, int ncols, int col) {
-  write_block_partials(red, nwarps, spec.nmax, spec.nlse, bpart, ncols, col);
+  write_block_partials(red, nwarps, spec.nmax, spec.nlse, bpart, ncols, col, spec.mode);
 }
 
 // ------------------------------------------------------------- finalize
@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(256)
 stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spec,
                      double* __restrict__ out, const StatCapture cap) {
   __shared__ double sm[8], ss[8];
+  dep_launch();
+  dep_wait();
   const int o = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (o < spec.nmax) {
@@ -166,7 +168,7 @@ stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spe
     double s = 0.0;
     if (m > -CUDART_INF)
       for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-        if (lse_nonempty(pm[b], ps[b])) s += ps[b] * merge_exp(pm[b] - m, spec.f32 != 0);
+        if (lse_nonempty(pm[b], ps[b])) s += ps[b] * merge_exp(pm[b] - m, spec.mode);
 #pragma unroll
     for (int k = 16; k >= 1; k >>= 1) s += shfl_xor_d(s, k);
     if (lane == 0) ss[w] = s;
@@ -317,7 +319,7 @@ init_vertex_kernel(const InitArgs<T> a) {
       }
     __syncwarp(gr.mask);
   }
-  const StatSpec spec{2 * Pe, 2 * Pe};
+  const StatSpec spec{2 * Pe, 2 * Pe, sizeof(T) == 8 ? kMergeFx : kMergeF64};
   const int slots = spec.slots();
   double* red = s_red + (size_t)(threadIdx.x >> 5) * slots;
 #pragma unroll
@@ -346,6 +348,8 @@ init_vertex_kernel(const InitArgs<T> a) {
 
 __global__ void mu_output_kernel(double* __restrict__ mu, const double* __restrict__ S,
                                  long long n, int Pn) {
+  dep_launch();
+  dep_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) mu[i] -= S[i % Pn];
 }
@@ -404,8 +408,7 @@ acg_status launch_finalize(const double* bpart, int nblocks, StatSpec spec, doub
                            cudaStream_t s, const StatCapture& cap) {
   const int n = spec.outs();
   if (n == 0) return ACG_OK;
-  stat_finalize_kernel<<<n, 256, 0, s>>>(bpart, nblocks, spec, out, cap);
-  ACG_LAUNCH_CHECK();
+  ACG_CUDA_TRY(launch_kernel(spec.early, stat_finalize_kernel, n, 256, 0, s, bpart, nblocks, spec, out, cap));
   return ACG_OK;
 }
 
@@ -434,11 +437,10 @@ acg_status launch_inverse_perm(const int* perm, long long n, int* pos, cudaStrea
   return ACG_OK;
 }
 
-acg_status launch_mu_output(double* mu, const double* S, long long Dn, int Pn, cudaStream_t s) {
+acg_status launch_mu_output(double* mu, const double* S, long long Dn, int Pn, bool early, cudaStream_t s) {
   const long long n = Dn * Pn;
   if (n == 0) return ACG_OK;
-  mu_output_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(mu, S, n, Pn);
-  ACG_LAUNCH_CHECK();
+  ACG_CUDA_TRY(launch_kernel(early, mu_output_kernel, (int)((n + 255) / 256), 256, 0, s, mu, S, n, Pn));
   return ACG_OK;
 }
 

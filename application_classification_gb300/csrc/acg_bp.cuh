@@ -21,7 +21,8 @@ __host__ __device__ inline int pattern_ints(int pn, int pe) { return 4 * pe + 2 
 struct StatSpec {
   int nmax;
   int nlse;
-  int f32 = 0;  // merge with the FP32 exponential (statistics of FP32 kernels)
+  int mode = 0;  // the merges' exponential (MergeExp)
+  bool early = false;  // finalize launched early (early_launches)
   __host__ __device__ int slots() const { return nmax + 2 * nlse; }
   __host__ __device__ int outs() const { return nmax + nlse; }
 };
@@ -80,11 +81,12 @@ struct InitArgs {
   T* rec_mh = nullptr;
   T* rec_ml = nullptr;
   int* wide = nullptr;  // FP64: Z is stored as edge_word stores it
+  bool early = false;   // (early_launches)
 };
 template <typename T>
 acg_status launch_init_vertex(const InitArgs<T>& a, GroupShape gs, int blocks, cudaStream_t s);
 
 // mu[v][p] -= S[p]
-acg_status launch_mu_output(double* mu, const double* S, long long Dn, int Pn, cudaStream_t s);
+acg_status launch_mu_output(double* mu, const double* S, long long Dn, int Pn, bool early, cudaStream_t s);
 
 }  // namespace acg

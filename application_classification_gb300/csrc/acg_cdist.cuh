@@ -25,6 +25,7 @@ struct CdistRbArgs {
   long long lim;       // Pn * Dn
   int K, kstride, P, Pp, ostride;
   int* wide = nullptr;  // FP64 edge costs: stored as edge_word stores them
+  bool early = false;   // (early_launches)
 };
 
 template <typename T, typename F>

@@ -43,6 +43,8 @@ __device__ __noinline__ double pair_fp64(const double* __restrict__ x, const dou
 
 template <int KM>
 __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double, double> a) {
+  dep_launch();
+  dep_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   FxPart* s_y = reinterpret_cast<FxPart*>(smem);  // [Pp][KM], zero past P and K
   __shared__ int s_exp, s_bad;
@@ -124,6 +126,8 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
 // t / P + 256 / P, ... of the block's contiguous rows.
 __global__ void __launch_bounds__(kXT)
 cdist_stats_kernel(const double* __restrict__ d, long long nrows, int P, int stride, double* __restrict__ part) {
+  dep_launch();
+  dep_wait();
   __shared__ FxLse s_p[kXT], s_n[kXT];
   __shared__ double s_m[kXT];
   const int nb = gridDim.x, rs = kXT / P;
@@ -171,8 +175,7 @@ cdist_stats_kernel(const double* __restrict__ d, long long nrows, int P, int str
     if (sm > 48 * 1024)                                                                          \
       ACG_CUDA_TRY(cudaFuncSetAttribute(cdist_fx_kernel<KM_>,                                    \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));  \
-    cdist_fx_kernel<KM_><<<blocks, kXT, sm, s>>>(a);                                             \
-    ACG_LAUNCH_CHECK();                                                                          \
+    ACG_CUDA_TRY(launch_kernel(a.early, cdist_fx_kernel<KM_>, blocks, kXT, sm, s, a));                 \
     return ACG_OK;                                                                               \
   }
 
@@ -192,8 +195,7 @@ acg_status launch_cdist_vertex_fx(const CdistRbArgs<double, double>& a, int bloc
   if (a.P == 0) return ACG_OK;
   if (a.P > kXT) return set_error(ACG_ERR_UNSUPPORTED, "cdist: %d columns", a.P);
   ACG_TRY(launch_cdist_fx(a, std::max(1, std::min(ceil_div(a.nrows, kXT), blocks * 4)), s));
-  cdist_stats_kernel<<<blocks, kXT, 0, s>>>(a.out, a.nrows, a.P, a.ostride, a.bpart);
-  ACG_LAUNCH_CHECK();
+  ACG_CUDA_TRY(launch_kernel(a.early, cdist_stats_kernel, blocks, kXT, 0, s, a.out, a.nrows, a.P, a.ostride, a.bpart));
   return ACG_OK;
 }
 

@@ -29,6 +29,31 @@
 
 namespace acg {
 
+// Programmatic dependent launch: a kernel launched early may start while the one
+// before it in the stream still runs; until dep_wait() returns (the
+// one before has completed and its writes are visible) it touches only what no
+// kernel of a match writes.  dep_launch() lets the next such kernel start early.
+// An iteration of a small graph is four to five kernels of about 8 us, so the
+// gaps between them and their prologues count (1,000 vertices: FP64 571 -> 451 us a
+// match, mixed 480 -> 406).
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... KA, typename... A>
+cudaError_t launch_kernel(bool early, void (*kernel)(KA...), int blocks, int threads, size_t smem,
+                                cudaStream_t s, const A&... args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3((unsigned)blocks);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, KA(args)...);
+}
+
 constexpr int kNumSMs = 152;  // GB300: 2 dies x 76 SMs
 
 template <typename T>
@@ -213,11 +238,14 @@ __device__ __forceinline__ void lse_merge(double& m, double& s, double m2, doubl
 }
 
 // exp(d) for d <= 0, the factor that rescales a partial sum when partial
-// log-sum-exps are merged.  FP64 for FP64 statistics; the FP32 exponential
-// (relative error ~1e-7, that of the FP32 partial sums it scales) for the
-// statistics of FP32 kernels -- FP64 transcendentals are slow on this GPU.
-__device__ __forceinline__ double merge_exp(double d, bool f32) {
-  return f32 ? (double)expf((float)d) : exp(d);
+// log-sum-exps are merged: kMergeF32, the FP32 exponential (relative error ~1e-7,
+// that of the FP32 partial sums it scales) for the iterations' statistics of FP32
+// kernels; kMergeF64, CUDA's FP64 exponential, for what FP32 plans form once per
+// match; kMergeFx, the integer pipes', for FP64 plans (FP64 transcendentals are
+// slow on this GPU).
+enum MergeExp { kMergeF64 = 0, kMergeF32 = 1, kMergeFx = 2 };
+__device__ __forceinline__ double merge_exp(double d, int mode) {
+  return mode == kMergeF32 ? (double)expf((float)d) : mode == kMergeFx ? fx_expd(d) : exp(d);
 }
 // A partial (m, s) that holds no term: m = -inf or s = 0.
 __device__ __forceinline__ bool lse_nonempty(double m, double s) {
@@ -231,7 +259,7 @@ __device__ __forceinline__ bool lse_nonempty(double m, double s) {
 // s_w exp(m_w - m)): one independent exponential per partial, no chain.
 __device__ __forceinline__ void write_block_partials(const double* red, int nwarps, int nmax,
                                                      int nlse, double* bpart, int ncols,
-                                                     int col, bool f32 = false) {
+                                                     int col, int mode = kMergeF64) {
   const int slots = nmax + 2 * nlse;
   for (int j = threadIdx.x; j < nmax + nlse; j += blockDim.x) {
     if (j < nmax) {
@@ -248,7 +276,7 @@ __device__ __forceinline__ void write_block_partials(const double* red, int nwar
       if (m > -CUDART_INF) {
         for (int w = 0; w < nwarps; ++w) {
           const double m2 = red[w * slots + sm], s2 = red[w * slots + sm + 1];
-          if (lse_nonempty(m2, s2)) s += s2 * merge_exp(m2 - m, f32);
+          if (lse_nonempty(m2, s2)) s += s2 * merge_exp(m2 - m, mode);
         }
       }
       bpart[(size_t)sm * ncols + col] = m;

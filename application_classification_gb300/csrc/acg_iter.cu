@@ -403,6 +403,8 @@ edge_max_kernel(const EdgeMaxArgs<T> a) {
   const int slot = lane / NPOW, qc = lane % NPOW;
   const int nw = (int)gridDim.x * (kAT / 32);
   const int gw = (blockIdx.x * kAT + threadIdx.x) >> 5;
+  dep_launch();
+  dep_wait();
   const bool wide = sizeof(T) == 8 && *a.wide != 0;
   // The warp's own range first, then claimed ones (the claim of the next is in
   // flight while this one runs): warps that finish early keep taking work, so
@@ -445,6 +447,8 @@ heavy_combine_kernel(const T* __restrict__ partial, const int* __restrict__ hbas
                      const int* __restrict__ hcount, const int* __restrict__ hvert, int Pp,
                      T* __restrict__ M) {
   __shared__ T part[8][kHeavyCols];
+  dep_launch();
+  dep_wait();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const T* p0 = partial + (size_t)hbase[blockIdx.x] * Pp;
   const int cnt = hcount[blockIdx.x];
@@ -945,6 +949,8 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
   for (int t = tid; t < 4 * Pe + 2 * (Pn + 1); t += kBT) s_pat[t] = a.pat[t];
   for (int t = tid; t < nterms * 32; t += kBT) s_sched[t] = a.vsched[t];
   __syncthreads();
+  dep_launch();
+  dep_wait();
   const int* s_psrc = s_pat;
   const int* s_pdst = s_pat + Pe;
 
@@ -1239,7 +1245,8 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
     }
   }
   __syncthreads();
-  write_block_partials(red, kVw, nmax, nlse, a.bpart, gridDim.x, blockIdx.x, sizeof(T) == 4);
+  write_block_partials(red, kVw, nmax, nlse, a.bpart, gridDim.x, blockIdx.x,
+                       sizeof(T) == 4 ? kMergeF32 : kMergeFx);
 }
 
 template <typename T>
@@ -1275,10 +1282,9 @@ WarpShape choose_warp_shape(int elem_bytes, int pp) {
 #define ACG_EDGE_LAUNCH(NP_, NQ_)                                           \
   if (ws.npow == NP_ && ws.nqv == NQ_) {                                    \
     if (a.argpos)                                                           \
-      edge_max_kernel<T, NP_, NQ_, true><<<blocks, kAT, 0, s>>>(a);         \
+      ACG_CUDA_TRY(launch_kernel(a.early, edge_max_kernel<T, NP_, NQ_, true>, blocks, kAT, 0, s, a));  \
     else                                                                    \
-      edge_max_kernel<T, NP_, NQ_, false><<<blocks, kAT, 0, s>>>(a);        \
-    ACG_LAUNCH_CHECK();                                                     \
+      ACG_CUDA_TRY(launch_kernel(a.early, edge_max_kernel<T, NP_, NQ_, false>, blocks, kAT, 0, s, a)); \
     return ACG_OK;                                                          \
   }
 
@@ -1316,11 +1322,10 @@ acg_status launch_heavy_combine_arg(const T* partial, const int* ppos, const int
 }
 template <typename T>
 acg_status launch_heavy_combine(const T* partial, const int* hbase, const int* hcount,
-                                const int* hvert, int nheavy, int Pp, T* M, cudaStream_t s) {
+                                const int* hvert, int nheavy, int Pp, T* M, bool early, cudaStream_t s) {
   if (nheavy == 0) return ACG_OK;
   if (Pp > kHeavyCols) return set_error(ACG_ERR_UNSUPPORTED, "heavy vertices: %d columns", Pp);
-  heavy_combine_kernel<T><<<nheavy, 256, 0, s>>>(partial, hbase, hcount, hvert, Pp, M);
-  ACG_LAUNCH_CHECK();
+  ACG_CUDA_TRY(launch_kernel(early, heavy_combine_kernel<T>, nheavy, 256, 0, s, partial, hbase, hcount, hvert, Pp, M));
   return ACG_OK;
 }
 
@@ -1360,8 +1365,7 @@ acg_status launch_vertex_update(const VertexUpdArgs<T>& a, int blocks, cudaStrea
     return set_error(ACG_ERR_INVALID_ARGUMENT, "vertex phase: no schedule for the warp form");
   const bool warp = warp_form(a.Pn, a.Pp, [&]<int QPL, int PPL>() {
     const size_t sm = vertex_warp_setup<T, QPL, PPL>(a.Pn, a.Pe, a.Pp, a.Pnp, a.vterms);
-    vertex_warp_kernel<T, QPL, PPL><<<blocks, kBT, sm, s>>>(a);
-    le = cudaGetLastError();
+    le = launch_kernel(a.early, vertex_warp_kernel<T, QPL, PPL>, blocks, kBT, sm, s, a);
   });
   if (warp) {
     if (le != cudaSuccess)
@@ -1421,8 +1425,8 @@ template acg_status launch_edge_max<double>(const EdgeMaxArgs<double>&, WarpShap
 template acg_status launch_edge_max<float>(const EdgeMaxArgs<float>&, WarpShape, int, cudaStream_t);
 template acg_status launch_heavy_combine_arg<double>(const double*, const int*, const int*, const int*, const int*, int, int, double*, int*, cudaStream_t);
 template acg_status launch_heavy_combine_arg<float>(const float*, const int*, const int*, const int*, const int*, int, int, float*, int*, cudaStream_t);
-template acg_status launch_heavy_combine<double>(const double*, const int*, const int*, const int*, int, int, double*, cudaStream_t);
-template acg_status launch_heavy_combine<float>(const float*, const int*, const int*, const int*, int, int, float*, cudaStream_t);
+template acg_status launch_heavy_combine<double>(const double*, const int*, const int*, const int*, int, int, double*, bool, cudaStream_t);
+template acg_status launch_heavy_combine<float>(const float*, const int*, const int*, const int*, int, int, float*, bool, cudaStream_t);
 template acg_status launch_vertex_update<float>(const VertexUpdArgs<float>&, int, cudaStream_t);
 template int edge_max_blocks_per_sm<double>(WarpShape);
 template int edge_max_blocks_per_sm<float>(WarpShape);

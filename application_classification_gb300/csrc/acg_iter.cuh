@@ -43,6 +43,7 @@ struct EdgeMaxArgs {
   const int* hvert = nullptr;
   int* hcnt = nullptr;
   int Pe = 0;          // columns of Pp that are pattern edges
+  bool early = false;  // (early_launches)
   // FP64: *wide is nonzero where a cost or message is not as edge_word keeps
   // them in range; rebase is 8 (a multiplier the compiler must not see as a
   // shift, see high_float)
@@ -91,6 +92,7 @@ struct VertexUpdArgs {
   // MU_raw sums of one stage, [vterms][32] (vertex_warp_schedule)
   const uint32_t* vsched = nullptr;
   int vterms = 0;
+  bool early = false;        // (early_launches)
   float* rowpart = nullptr;  // acg_vertex_wide.cu: the rows' statistics (wide_rowpart_floats)
   const double* lse_pos = nullptr;  // [Pn] LSE_v(dV), which bounds |CV| (FP64 only)
   int* wide = nullptr;              // FP64: Z is stored as edge_word stores it
@@ -113,7 +115,7 @@ acg_status launch_wide_partials(const VertexUpdArgs<float>& a, int blocks, cudaS
 int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
 int vertex_fx_warps(int pn, int pp);  // warps that share a stage
 acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s);
-int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms);
+int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms, int dn);
 // Edge phase of FP32 plans with the costs recomputed on the tensor cores
 // (acg_edge_tc.cu): M[v][q] = max over in-edges e of z[s_e][q] - ||x_e - y_q||,
 // d formed as the tensor-core edge cost matrix forms it.  One CTA per part of
@@ -155,7 +157,7 @@ template <typename T>
 acg_status launch_edge_max(const EdgeMaxArgs<T>& a, WarpShape ws, int blocks, cudaStream_t s);
 template <typename T>
 acg_status launch_heavy_combine(const T* partial, const int* hbase, const int* hcount,
-                                const int* hvert, int nheavy, int Pp, T* M, cudaStream_t s);
+                                const int* hvert, int nheavy, int Pp, T* M, bool early, cudaStream_t s);
 // The same with the argmax positions of the chunks (earlier chunks win ties).
 template <typename T>
 acg_status launch_heavy_combine_arg(const T* partial, const int* ppos, const int* hbase,

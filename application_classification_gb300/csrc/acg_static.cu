@@ -421,6 +421,8 @@ src_stats_kernel(const SrcStatsArgs<T> a) {
       reinterpret_cast<uint64_t*>(src_ring)[t] = fx_table_entry(t);
     __syncthreads();
   }
+  dep_launch();
+  dep_wait();
   for (int r = gw; r < a.nranges;) {
     int rn = a.nranges;
     if (a.ctr && lane == 0) rn = nw + atomicAdd(a.ctr, 1);
@@ -450,6 +452,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 src_stats_combine_kernel(const SrcStatsArgs<T> a, const int* __restrict__ hbase,
                          const int* __restrict__ hcount, const int* __restrict__ hvert) {
+  dep_launch();
+  dep_wait();
   extern __shared__ __align__(16) unsigned char comb_sm[];
   const int Pp = a.Pp, Pqc = a.Pqc;
   double* s_m = reinterpret_cast<double*>(comb_sm);  // [8][Pp]
@@ -493,6 +497,8 @@ src_stats_combine_kernel(const SrcStatsArgs<T> a, const int* __restrict__ hbase,
 template <typename T, int NPOW, int NQV>
 __global__ void __launch_bounds__(kST)
 dst_quirk_kernel(const DstQuirkArgs<T> a) {
+  dep_launch();
+  dep_wait();
   using VT = typename SV<T>::type;
   constexpr int W = SV<T>::W;
   constexpr int S = 32 / NPOW;
@@ -594,7 +600,8 @@ dst_quirk_kernel(const DstQuirkArgs<T> a) {
     }
   }
   __syncthreads();
-  write_block_partials(red, kST / 32, 0, Pqc, a.bpart, gridDim.x, blockIdx.x);
+  write_block_partials(red, kST / 32, 0, Pqc, a.bpart, gridDim.x, blockIdx.x,
+                       sizeof(T) == 8 ? kMergeFx : kMergeF64);
 }
 
 // ------------------------------------------------------------ init, warp form
@@ -631,6 +638,8 @@ init_warp_kernel(const InitArgs<T> a) {
   T* smu = s_mu + (size_t)wib * 64 * PPL;  // hi | lo
   for (int t = tid; t < npat; t += kST) s_pat[t] = a.pat[t];
   __syncthreads();
+  dep_launch();
+  dep_wait();
   const int* s_psrc = s_pat;
   const int* s_pdst = s_pat + Pe;
   const double* gv = a.gv;  // [maxneg(Pn) | lse_pos(Pn) | lse_neg(Pn)]
@@ -790,7 +799,8 @@ init_warp_kernel(const InitArgs<T> a) {
     }
   }
   __syncthreads();
-  write_block_partials(red, kW, nmax, nlse, a.bpart, gridDim.x, blockIdx.x);
+  write_block_partials(red, kW, nmax, nlse, a.bpart, gridDim.x, blockIdx.x,
+                       sizeof(T) == 8 ? kMergeFx : kMergeF64);
 }
 
 template <typename T, int QPL, int PPL>
@@ -838,8 +848,7 @@ bool init_warp_shape(int pn, int pp, F&& f) {
     if (sm > 48 * 1024)                                                                     \
       ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_kernel<T, NP_, 1>,                        \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-    src_stats_kernel<T, NP_, 1><<<blocks, kST, sm, s>>>(a);                                 \
-    ACG_LAUNCH_CHECK();                                                                     \
+    ACG_CUDA_TRY(launch_kernel(a.early, src_stats_kernel<T, NP_, 1>, blocks, kST, sm, s, a));     \
     continue;                                                                               \
   }
 
@@ -867,8 +876,7 @@ acg_status launch_src_stats_combine(const SrcStatsArgs<T>& a, const WarpWork& w,
   if (sm > 48 * 1024)
     ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_combine_kernel<T>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  src_stats_combine_kernel<T><<<w.nheavy, 256, sm, s>>>(a, w.hbase, w.hcount, w.hvert);
-  ACG_LAUNCH_CHECK();
+  ACG_CUDA_TRY(launch_kernel(a.early, src_stats_combine_kernel<T>, w.nheavy, 256, sm, s, a, w.hbase, w.hcount, w.hvert));
   return ACG_OK;
 }
 
@@ -878,8 +886,7 @@ acg_status launch_src_stats_combine(const SrcStatsArgs<T>& a, const WarpWork& w,
     if (sm > 48 * 1024)                                                           \
       ACG_CUDA_TRY(cudaFuncSetAttribute(dst_quirk_kernel<T, NP_, NQ_>,            \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-    dst_quirk_kernel<T, NP_, NQ_><<<blocks, kST, sm, s>>>(a);                     \
-    ACG_LAUNCH_CHECK();                                                           \
+    ACG_CUDA_TRY(launch_kernel(a.early, dst_quirk_kernel<T, NP_, NQ_>, blocks, kST, sm, s, a)); \
     return ACG_OK;                                                                \
   }
 
@@ -927,8 +934,7 @@ acg_status launch_init_warp(const InitArgs<T>& a, int blocks, cudaStream_t s) {
   const bool ok = init_warp_shape<T>(a.Pn, a.Pp, [&]<int QPL, int PPL>() {
     size_t sm = 0;
     init_warp_fit<T, QPL, PPL>(a.Pn, a.Pe, &sm);
-    init_warp_kernel<T, QPL, PPL><<<blocks, kST, sm, s>>>(a);
-    le = cudaGetLastError();
+    le = launch_kernel(a.early, init_warp_kernel<T, QPL, PPL>, blocks, kST, sm, s, a);
   });
   if (!ok) return set_error(ACG_ERR_UNSUPPORTED, "init warp form: pattern too large");
   if (le != cudaSuccess) return set_error(ACG_ERR_CUDA, "init_warp_kernel launch: %s", cudaGetErrorString(le));

@@ -47,6 +47,7 @@ struct SrcStatsArgs {
   int nranges = 0;
   int* ctr = nullptr;
   int col0 = 0;  // first 16-byte column of the launch (rows wider than 32: several)
+  bool early = false;  // (early_launches)
 };
 template <typename T>
 acg_status launch_src_stats(const SrcStatsArgs<T>& a, WarpShape ws, int blocks, cudaStream_t s);
@@ -75,6 +76,7 @@ struct DstQuirkArgs {
                        // does ranges w, w + warps, ...
   int dstride = 0;     // row stride of dE as given: Pp, or Pqc for the compact
                        // copy of the covered columns (0: Pp)
+  bool early = false;  // (early_launches)
 };
 template <typename T>
 acg_status launch_dst_quirk(const DstQuirkArgs<T>& a, WarpShape ws, int blocks, cudaStream_t s);

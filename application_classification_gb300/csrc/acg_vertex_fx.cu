@@ -328,6 +328,8 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   for (int t = tid; t < kFxTable; t += kFT) reinterpret_cast<uint64_t*>(smem + L.tab)[t] = fx_table_entry(t);
   if (tid < 2) s_bound[tid] = 0;
   __syncthreads();
+  dep_launch();
+  dep_wait();
   const int* s_psrc = s_pat;
   const int* s_pdst = s_pat + Pe;
 
@@ -591,15 +593,14 @@ acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStre
       le = cudaFuncSetAttribute(vertex_fx_kernel<QPL, PPL, NW>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (le != cudaSuccess) return;
-    vertex_fx_kernel<QPL, PPL, NW><<<blocks, kFT, sm, s>>>(a);
-    le = cudaGetLastError();
+    le = launch_kernel(a.early, vertex_fx_kernel<QPL, PPL, NW>, blocks, kFT, sm, s, a);
   });
   if (le != cudaSuccess)
     return set_error(ACG_ERR_CUDA, "vertex_fx_kernel launch: %s", cudaGetErrorString(le));
   return ACG_OK;
 }
 
-int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms) {
+int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms, int dn) {
   int nb = 0;
   fx_form(pn, pp, [&]<int QPL, int PPL, int NW>() {
     const size_t sm = FxSmem(pn, pe, pp, pnp, nterms, NW).total;
@@ -610,7 +611,9 @@ int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms) {
         cudaSuccess)
       nb = 1;
   });
-  return num_sms * (nb < 1 ? 1 : nb);
+  // (a stage per group at least: fewer partials to finalise on small graphs)
+  const int per = kFxVps * kFW / vertex_fx_warps(pn, pp);
+  return std::min(num_sms * (nb < 1 ? 1 : nb), std::max(1, ceil_div(dn, per)));
 }
 
 }  // namespace acg

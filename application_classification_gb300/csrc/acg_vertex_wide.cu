@@ -362,8 +362,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) vertex_wide_kernel(const Ve
 
 // Block b's partials from its rows' statistics: mVF, mVR (max), lR, lF, S (lse),
 // rows combined in order.  The merges are FP64 exponentials, 37 us of the FP64
-// pipe at 120 columns; as a launch of their own they run beside the next edge
-// phase, which does not read them.
+// pipe at 120 columns; as a launch of their own they spread over all threads of a
+// block, and in a batch run beside the next edge phase, which does not read them.
 __global__ void __launch_bounds__(256)
 wide_partials_kernel(const float* __restrict__ rowpart, int V, int Pe, int Pn, int Pp,
                      double* __restrict__ bpart) {

@@ -25,25 +25,29 @@ def test_wide_vertex_phase(cuda, dn, pn, pe):
     assert np.abs(mu - ref).max() <= 1e-4
 
 
-# large enough for the statistics to run beside the edge phase: the same bits on
-# another stream, on a reused plan, with two plans' matches in flight, and with
-# phase timing (statistics in line)
-@pytest.mark.parametrize("precision,pn,pe", [("mixed", 16, 32), ("mixed", 20, 90), ("fp64", 16, 32)])
-def test_side_stream(cuda, precision, pn, pe):
+# large enough for a batch to combine the statistics beside the edge phase: a
+# pattern that forms a group of its own has the bits of its single match, on the
+# first call (captured), on the relaunch, and on another stream; and single plans
+# give the same bits with two matches in flight and with phase timing
+@pytest.mark.parametrize("precision,pn,pe", [("mixed", 16, 60), ("mixed", 20, 90), ("fp64", 16, 60)])
+def test_statistics_beside_edge_phase(cuda, precision, pn, pe):
     import torch
 
     d, p, _ = graph.workload(f"rmat16_{pn}_{pe}")
     data = matcher.DataGraph(d)
-    plans = [matcher.Plan(data, p, precision) for _ in range(2)]
-    timed = matcher.Plan(data, p, precision, kernel_timing=True)
-    want = timed.run()
+    want = matcher.Plan(data, p, precision, kernel_timing=True).run()
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    plans = [matcher.Plan(data, p, precision) for _ in range(2)]
     outs = []
-    for _ in range(2):
-        for plan, st in zip(plans, streams):
-            with torch.cuda.stream(st):
-                outs.append(plan.run(stream=st))
+    for plan, st in zip(plans * 2, streams * 2):
+        with torch.cuda.stream(st):
+            outs.append(plan.run(stream=st))
+    batch = matcher.Batch(data, [p, p], precision)
+    for st in (streams[0], streams[0], streams[1]):
+        with torch.cuda.stream(st):
+            outs += [o.clone() for o in batch.run(stream=st)]
+        st.synchronize()
     torch.cuda.synchronize()
     for o in outs:
         assert torch.equal(o, want)
