@@ -869,7 +869,7 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
 // double-buffered ring (kVps vertices per stage) with cp.async, so a warp never
 // waits on another.  Per stage:
 //   1. F, R of each staged vertex from its M, Y rows, written over them in the
-//      stage (the CV rows are negated in place);
+//      stage;
 //   2. the compensated sums MU_raw[v][p] = -CV[v][p] + sum F + sum R of all
 //      staged vertices through a per-lane schedule built on the host
 //      (vertex_warp_schedule): each (vertex, p) sum is one job whose terms are
@@ -882,20 +882,17 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
 // Every sum keeps its terms and their order, so the results do not depend on
 // how the jobs are spread.  Vertices without in-edges have M rows of -inf (set
 // once, never written by phase A).
-#ifndef ACG_VTX_VPS
-#define ACG_VTX_VPS 4
-#endif
-constexpr int kVps = ACG_VTX_VPS;  // vertices per stage
+constexpr int kVps = 4;  // vertices per stage (one add4_fast per column)
 constexpr int kVw = kBT / 32;
-template <typename T, int QPL, int PPL>
+template <int PPL>
 struct VwSmem {
   size_t pat, sched, ring, mu, total, stage, warp_ring, mu_n;
   __host__ __device__ VwSmem(int Pn, int Pe, int Pp, int Pnp, int nterms) {
-    const size_t sz = sizeof(T);
+    const size_t sz = sizeof(float);
     size_t o = 0;
     pat = o; o += a16(sizeof(int) * (size_t)(4 * Pe + 2 * (Pn + 1)));
     sched = o; o += a16(sizeof(uint32_t) * (size_t)nterms * 32);
-    stage = (size_t)VwStage(Pp, Pnp, sz == 4, kVps).n * sz;  // row sizes are 16-byte multiples
+    stage = (size_t)VwStage(Pp, Pnp, true, kVps).n * sz;  // row sizes are 16-byte multiples
     warp_ring = 2 * stage;
     const size_t red = sizeof(double) * (size_t)kVw * (6 * Pe + 2 * Pn);  // aliases the rings
     ring = o; o += a16(red > kVw * warp_ring ? red : kVw * warp_ring);
@@ -905,44 +902,50 @@ struct VwSmem {
   }
 };
 
-template <typename T, int N>
-__device__ __forceinline__ void lds_n(const T* p, T (&x)[N]) {
-  if constexpr (N == 2 && sizeof(T) == 4) {
+// Two FP32 additions or subtractions in one instruction, each rounded to nearest
+// as by itself; the last step of a message, ((u - c) - m) + (l - cl), on pairs.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+      " add.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n"
+      " sub.rn.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 message2(float2 u, float2 c, float2 m, float2 l, float2 cl) {
+  return add2(sub2(sub2(u, c), m), sub2(l, cl));
+}
+
+template <int N>
+__device__ __forceinline__ void lds_n(const float* p, float (&x)[N]) {
+  if constexpr (N == 2) {
     const float2 v = *reinterpret_cast<const float2*>(p);
     x[0] = v.x;
     x[1] = v.y;
-  } else if constexpr (N == 2 && sizeof(T) == 8) {
-    const double2 v = *reinterpret_cast<const double2*>(p);
-    x[0] = v.x;
-    x[1] = v.y;
   } else {
-#pragma unroll
-    for (int k = 0; k < N; ++k) x[k] = p[k];
+    x[0] = *p;
   }
 }
-template <typename T, int N>
-__device__ __forceinline__ void st_n(T* p, const T (&x)[N]) {
-  if constexpr (N == 2 && sizeof(T) == 4) {
-    *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
-  } else if constexpr (N == 2 && sizeof(T) == 8) {
-    *reinterpret_cast<double2*>(p) = make_double2(x[0], x[1]);
-  } else {
-#pragma unroll
-    for (int k = 0; k < N; ++k) p[k] = x[k];
-  }
+template <int N>
+__device__ __forceinline__ void st_n(float* p, const float (&x)[N]) {
+  if constexpr (N == 2) *reinterpret_cast<float2*>(p) = make_float2(x[0], x[1]);
+  else *p = x[0];
 }
 
 // Two blocks per SM bounds the registers at 128
-#ifndef ACG_VTX_MINB
-#define ACG_VTX_MINB 2
-#endif
-template <typename T, int QPL, int PPL>
-__global__ void __launch_bounds__(kBT, ACG_VTX_MINB)
-vertex_warp_kernel(const VertexUpdArgs<T> a) {
+template <int QPL, int PPL, bool REC>
+__global__ void __launch_bounds__(kBT, 2)
+vertex_warp_kernel(const VertexUpdArgs<float> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int Pe = a.Pe, Pn = a.Pn, Pp = a.Pp, Pnp = a.Pnp, Dn = a.Dn, nterms = a.vterms;
-  const VwSmem<T, QPL, PPL> L(Pn, Pe, Pp, Pnp, nterms);
-  const VwStage G(Pp, Pnp, sizeof(T) == 4, kVps);
+  const VwSmem<PPL> L(Pn, Pe, Pp, Pnp, nterms);
+  const VwStage G(Pp, Pnp, true, kVps);
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
   int* s_pat = reinterpret_cast<int*>(smem + L.pat);
   uint32_t* s_sched = reinterpret_cast<uint32_t*>(smem + L.sched);
@@ -959,12 +962,12 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
   const int x0 = 4 * Pe + Pn;
   const int qo = lane * QPL;
   const bool qon = qo < Pp;
-  T fF[QPL], fR[QPL], dFh[QPL], dFl[QPL], dRh[QPL], dRl[QPL], cRh[QPL], cRl[QPL], cFh[QPL], cFl[QPL];
+  float fF[QPL], fR[QPL], dFh[QPL], dFl[QPL], dRh[QPL], dRl[QPL], cRh[QPL], cRl[QPL], cFh[QPL], cFl[QPL];
   int qd[QPL], qs[QPL];
 #pragma unroll
   for (int k = 0; k < QPL; ++k) {
     const int q = qo + k;
-    fF[k] = fR[k] = dFh[k] = dFl[k] = dRh[k] = dRl[k] = cRh[k] = cRl[k] = cFh[k] = cFl[k] = T(0);
+    fF[k] = fR[k] = dFh[k] = dFl[k] = dRh[k] = dRl[k] = cRh[k] = cRl[k] = cFh[k] = cFl[k] = 0.f;
     qd[k] = qs[k] = 0;
     if (q < Pe) {
       qd[k] = s_pdst[q];
@@ -977,21 +980,21 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
         fr -= a.cnull[q];
         ff -= a.cnull[q];
       }
-      fR[k] = (T)fr;
-      fF[k] = (T)ff;
-      dRh[k] = (T)dR;
-      dRl[k] = (T)(dR - (double)dRh[k]);
-      dFh[k] = (T)dF;
-      dFl[k] = (T)(dF - (double)dFh[k]);
+      fR[k] = (float)fr;
+      fF[k] = (float)ff;
+      dRh[k] = (float)dR;
+      dRl[k] = (float)(dR - (double)dRh[k]);
+      dFh[k] = (float)dF;
+      dFl[k] = (float)(dF - (double)dFh[k]);
       const double lRp = cRu + dR, lFp = cFu + dF;
       double cRn = a.first ? lRp : g[x0 + 2 * Pe + q];
       double cFn = a.first ? lFp : g[x0 + 3 * Pe + q];
       if (!isfinite(cRn)) cRn = 0.0;
       if (!isfinite(cFn)) cFn = 0.0;
-      cRh[k] = (T)cRn;
-      cRl[k] = (T)(cRn - (double)cRh[k]);
-      cFh[k] = (T)cFn;
-      cFl[k] = (T)(cFn - (double)cFh[k]);
+      cRh[k] = (float)cRn;
+      cRl[k] = (float)(cRn - (double)cRh[k]);
+      cFh[k] = (float)cFn;
+      cFl[k] = (float)(cFn - (double)cFh[k]);
       if (blockIdx.x == 0 && wib == 0) {
         double* o = a.glob_out;
         o[x0 + q] = (double)cRh[k] + (double)cRl[k];
@@ -1001,12 +1004,13 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
       }
     }
   }
-  T mxF[QPL], mxR[QPL];
-  OnlineLse<T> lr[QPL], lf[QPL], lmu[PPL];
+  float mxF[QPL], mxR[QPL];
+  OnlineLse<float> lr[QPL], lf[QPL], lmu[PPL];
+  bool any_last = false;
   bool plast[PPL];  // this iteration is the last of pattern vertex p's pattern
 #pragma unroll
   for (int k = 0; k < QPL; ++k) {
-    mxF[k] = mxR[k] = neg_inf<T>();
+    mxF[k] = mxR[k] = neg_inf<float>();
     lr[k].init();
     lf[k].init();
   }
@@ -1015,18 +1019,20 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
     lmu[j].init();
     const int p = lane + 32 * j;
     plast[j] = p < Pn && __ldg(a.iters_p + p) == a.t;
+    any_last = any_last || plast[j];
   }
+  any_last = __any_sync(0xffffffffu, any_last);  // (one branch a vertex, none of the FP64 sums)
 
   const long long nw = (long long)gridDim.x * kVw;
   const long long gw = (long long)blockIdx.x * kVw + wib;
   const int vb = (int)(gw * Dn / nw), ve = (int)((gw + 1) * Dn / nw);
   unsigned char* ring = smem + L.ring + (size_t)wib * L.warp_ring;
-  T* smu = reinterpret_cast<T*>(smem + L.mu) + (size_t)wib * L.mu_n;
+  float* smu = reinterpret_cast<float*>(smem + L.mu) + (size_t)wib * L.mu_n;
   // MU_raw rows of the staged vertices, one word apart in bank order so that
   // the lanes ending jobs of one p for different vertices do not collide
   constexpr int kMuRow = 32 * PPL + 1;
   constexpr int kMuLo = kVps * kMuRow;  // the low parts after the high parts
-  const size_t rowb = (size_t)Pp * sizeof(T), crow = (size_t)Pnp * sizeof(T);
+  const size_t rowb = (size_t)Pp * sizeof(float), crow = (size_t)Pnp * sizeof(float);
   auto issue = [&](int v0, int buf) {
     const int nv = min(kVps, ve - v0);
     if (nv <= 0) return;
@@ -1034,17 +1040,16 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
     const int n16 = (int)((size_t)nv * rowb / 16);
     const size_t go = (size_t)v0 * rowb;
     for (int c = lane; c < n16; c += 32) {
-      cp16(st + G.oM * sizeof(T) + c * 16, reinterpret_cast<const unsigned char*>(a.M) + go + c * 16);
-      cp16(st + G.oY * sizeof(T) + c * 16, reinterpret_cast<const unsigned char*>(a.vf) + go + c * 16);
-      cp16(st + G.oE * sizeof(T) + c * 16, reinterpret_cast<const unsigned char*>(a.dEmin) + go + c * 16);
-      cp16(st + G.oB * sizeof(T) + c * 16, reinterpret_cast<const unsigned char*>(a.B) + go + c * 16);
+      cp16(st + G.oM * sizeof(float) + c * 16, reinterpret_cast<const unsigned char*>(a.M) + go + c * 16);
+      cp16(st + G.oY * sizeof(float) + c * 16, reinterpret_cast<const unsigned char*>(a.vf) + go + c * 16);
+      cp16(st + G.oE * sizeof(float) + c * 16, reinterpret_cast<const unsigned char*>(a.dEmin) + go + c * 16);
+      cp16(st + G.oB * sizeof(float) + c * 16, reinterpret_cast<const unsigned char*>(a.B) + go + c * 16);
     }
     const int c16 = (int)((size_t)nv * crow / 16);
     const size_t co = (size_t)v0 * crow;
     for (int c = lane; c < c16; c += 32) {
-      cp16(st + G.oC * sizeof(T) + c * 16, reinterpret_cast<const unsigned char*>(a.CV) + co + c * 16);
-      if constexpr (sizeof(T) == 4)
-        cp16(st + G.oCl * sizeof(T) + c * 16, reinterpret_cast<const unsigned char*>(a.CVlo) + co + c * 16);
+      cp16(st + G.oC * sizeof(float) + c * 16, reinterpret_cast<const unsigned char*>(a.CV) + co + c * 16);
+      cp16(st + G.oCl * sizeof(float) + c * 16, reinterpret_cast<const unsigned char*>(a.CVlo) + co + c * 16);
     }
   };
   issue(vb, 0);
@@ -1055,35 +1060,32 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
     cp_commit();
     cp_wait1();
     __syncwarp();
-    T* st = reinterpret_cast<T*>(ring + (size_t)buf * L.stage);
+    float* st = reinterpret_cast<float*>(ring + (size_t)buf * L.stage);
     const int nv = min(kVps, ve - v0);
-    // ---- 1. F over M, R over Y; -CV (and its low part) in place
+    // ---- 1. F over M, R over Y (a vertex past the stage's: unused)
+    if (qon) {
 #pragma unroll
-    for (int jv = 0; jv < kVps; ++jv) {
-      if (jv >= nv) break;
-      if (qon) {
-        T m[QPL], y[QPL], F[QPL], R[QPL];
-        T* sm_ = st + G.oM + jv * Pp + qo;
-        T* sy_ = st + G.oY + jv * Pp + qo;
-        lds_n<T, QPL>(sm_, m);
-        lds_n<T, QPL>(sy_, y);
-#pragma unroll
-        for (int k = 0; k < QPL; ++k) {
-          // no in-edges: M = -inf; no out-edges: Y = -inf; the fill wins
-          F[k] = fmax(fF[k], (m[k] - dFh[k]) - dFl[k]);
-          R[k] = fmax(fR[k], (y[k] - dRh[k]) - dRl[k]);
+      for (int jv = 0; jv < kVps; ++jv) {
+        float m[QPL], y[QPL];
+        float* sm_ = st + G.oM + jv * Pp + qo;
+        float* sy_ = st + G.oY + jv * Pp + qo;
+        lds_n<QPL>(sm_, m);
+        lds_n<QPL>(sy_, y);
+        // no in-edges: M = -inf; no out-edges: Y = -inf; the fill wins
+        if constexpr (QPL == 2) {
+          const float2 f2 = sub2(sub2({m[0], m[1]}, {dFh[0], dFh[1]}), {dFl[0], dFl[1]});
+          const float2 r2 = sub2(sub2({y[0], y[1]}, {dRh[0], dRh[1]}), {dRl[0], dRl[1]});
+          m[0] = fmaxf(fF[0], f2.x);
+          m[1] = fmaxf(fF[1], f2.y);
+          y[0] = fmaxf(fR[0], r2.x);
+          y[1] = fmaxf(fR[1], r2.y);
+        } else {
+          const float2 v = sub2(sub2({m[0], y[0]}, {dFh[0], dRh[0]}), {dFl[0], dRl[0]});
+          m[0] = fmaxf(fF[0], v.x);
+          y[0] = fmaxf(fR[0], v.y);
         }
-        st_n<T, QPL>(sm_, F);
-        st_n<T, QPL>(sy_, R);
-      }
-#pragma unroll
-      for (int j = 0; j < PPL; ++j) {
-        const int p = lane + 32 * j;
-        if (p < Pn) {
-          T* c = st + G.oC + jv * Pnp + p;
-          *c = -*c;
-          if constexpr (sizeof(T) == 4) c[G.oCl - G.oC] = -c[G.oCl - G.oC];
-        }
+        st_n<QPL>(sm_, m);
+        st_n<QPL>(sy_, y);
       }
     }
     __syncwarp();
@@ -1091,131 +1093,121 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
     // per step: their schedule words in one 16-byte load, their values loaded
     // before the dependent additions
     {
-      T hi = T(0), lo = T(0);
+      float hi = 0.f, lo = 0.f;
       const uint4* sch = reinterpret_cast<const uint4*>(s_sched) + lane;
       for (int t4 = 0; t4 < nterms / 4; ++t4) {
         const uint4 w4 = sch[t4 * 32];
         const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-        T x[4], xl[4];
+        float x[4], xl[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const T* xp = st + (w[u] & 0xfffu);
+          const float* xp = st + (w[u] & 0xfffu);
           x[u] = *xp;
-          if constexpr (sizeof(T) == 4) xl[u] = (w[u] & kSchedStart) ? xp[G.oCl - G.oC] : T(0);
+          xl[u] = 0.f;
+          if (w[u] & kSchedStart) xl[u] = xp[G.oCl - G.oC];
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
+          // a job starts from (-CV_hi, -CV_lo)
           const bool first = (w[u] & kSchedStart) != 0;
-          const T h0 = first ? T(0) : hi;
-          if constexpr (sizeof(T) == 4) {
-            // a job starts from (0, -CV_lo) and adds -CV_hi: exactly (-CV_hi, -CV_lo)
-            const T l0 = first ? xl[u] : lo;
-            const T sm = h0 + x[u];
-            const T bp = sm - h0;
-            lo = l0 + ((h0 - (sm - bp)) + (x[u] - bp));
-            hi = sm;
-          } else {
-            hi = h0 + x[u];
-          }
+          const float sm = hi + x[u];
+          const float bp = sm - hi;
+          const float l = lo + ((hi - (sm - bp)) + (x[u] - bp));
+          hi = first ? -x[u] : sm;
+          lo = first ? -xl[u] : l;
           if (w[u] & kSchedEnd) {
             const int slot = (int)((w[u] >> 16) & 0x1ffu);
             smu[slot] = hi;
-            if constexpr (sizeof(T) == 4) smu[kMuLo + slot] = lo;
+            smu[kMuLo + slot] = lo;
           }
         }
       }
     }
     __syncwarp();
-    // ---- 3. per staged vertex: MU_raw outputs, new Y and Z; the FP32 column
-    // log-sum-exps take the stage's values four at a time
-    constexpr bool kBatch = sizeof(T) == 4 && kVps == 4;
-    T lrv[QPL][kVps], lfv[QPL][kVps], muh[PPL][kVps], mul[PPL][kVps];
+    // ---- 3. per staged vertex: MU_raw outputs, new Y and Z; the column
+    // log-sum-exps take the stage's values four at a time (-inf: nothing)
+    float lrv[QPL][kVps], lfv[QPL][kVps], muh[PPL][kVps], mul[PPL][kVps];
 #pragma unroll
     for (int jv = 0; jv < kVps; ++jv) {
 #pragma unroll
-      for (int k = 0; k < QPL; ++k) lrv[k][jv] = lfv[k][jv] = neg_inf<T>();
+      for (int k = 0; k < QPL; ++k) lrv[k][jv] = lfv[k][jv] = neg_inf<float>();
 #pragma unroll
       for (int j = 0; j < PPL; ++j) {
-        muh[j][jv] = neg_inf<T>();
-        mul[j][jv] = T(0);
+        muh[j][jv] = neg_inf<float>();
+        mul[j][jv] = 0.f;
       }
     }
 #pragma unroll
     for (int jv = 0; jv < kVps; ++jv) {
       if (jv >= nv) break;
-      const int v = v0 + jv;
-      const T* mu_hi = smu + jv * kMuRow;
+      const size_t v = v0 + jv;
+      const float* mu_hi = smu + jv * kMuRow;
 #pragma unroll
       for (int j = 0; j < PPL; ++j) {
         const int p = lane + 32 * j;
-        if (p < Pn) {
-          const T h = mu_hi[p];
-          const T l = sizeof(T) == 4 ? mu_hi[kMuLo + p] : T(0);
-          if constexpr (kBatch) {
-            muh[j][jv] = h;
-            mul[j][jv] = l;
-          } else {
-            lmu[j].add2_fast(h, l);
-          }
-          if (plast[j]) a.mu_raw[(size_t)v * Pn + p] = (double)h + (double)l;
-          if (a.rec_mh) {
-            a.rec_mh[(size_t)v * Pn + p] = h;
-            a.rec_ml[(size_t)v * Pn + p] = l;
+        const bool pon = p < Pn;
+        const float h = mu_hi[p], l = mu_hi[kMuLo + p];
+        muh[j][jv] = pon ? h : neg_inf<float>();
+        mul[j][jv] = pon ? l : 0.f;
+        if (any_last && pon && plast[j]) a.mu_raw[v * Pn + p] = (double)h + (double)l;
+        if constexpr (REC) {
+          if (pon && a.rec_mh) {
+            a.rec_mh[v * Pn + p] = h;
+            a.rec_ml[v * Pn + p] = l;
           }
         }
       }
       if (!a.last && qon) {
-        T F[QPL], R[QPL], em[QPL], b[QPL], yo[QPL], zo[QPL], fo[QPL];
-        lds_n<T, QPL>(st + G.oM + jv * Pp + qo, F);
-        lds_n<T, QPL>(st + G.oY + jv * Pp + qo, R);
-        lds_n<T, QPL>(st + G.oE + jv * Pp + qo, em);
-        lds_n<T, QPL>(st + G.oB + jv * Pp + qo, b);
+        float F[QPL], R[QPL], em[QPL], b[QPL], f[QPL], r[QPL], yo[QPL];
+        lds_n<QPL>(st + G.oM + jv * Pp + qo, F);
+        lds_n<QPL>(st + G.oY + jv * Pp + qo, R);
+        lds_n<QPL>(st + G.oE + jv * Pp + qo, em);
+        lds_n<QPL>(st + G.oB + jv * Pp + qo, b);
+        // f = VF' - cR, r = VR' - cF: the shift comes off the compensated
+        // MU_raw first, the small message after
+        if constexpr (QPL == 2) {
+          const float2 f2 = message2({mu_hi[qd[0]], mu_hi[qd[1]]}, {cRh[0], cRh[1]}, {F[0], F[1]},
+                                     {mu_hi[kMuLo + qd[0]], mu_hi[kMuLo + qd[1]]}, {cRl[0], cRl[1]});
+          const float2 r2 = message2({mu_hi[qs[0]], mu_hi[qs[1]]}, {cFh[0], cFh[1]}, {R[0], R[1]},
+                                     {mu_hi[kMuLo + qs[0]], mu_hi[kMuLo + qs[1]]}, {cFl[0], cFl[1]});
+          f[0] = f2.x;
+          f[1] = f2.y;
+          r[0] = r2.x;
+          r[1] = r2.y;
+        } else {
+          const float2 v2 = message2({mu_hi[qd[0]], mu_hi[qs[0]]}, {cRh[0], cFh[0]}, {F[0], R[0]},
+                                     {mu_hi[kMuLo + qd[0]], mu_hi[kMuLo + qs[0]]}, {cRl[0], cFl[0]});
+          f[0] = v2.x;
+          r[0] = v2.y;
+        }
 #pragma unroll
         for (int k = 0; k < QPL; ++k) {
-          // f = VF' - cR, r = VR' - cF: the shift comes off the compensated
-          // MU_raw first, the small message after
-          T f, r;
-          if constexpr (sizeof(T) == 4) {
-            f = ((mu_hi[qd[k]] - cRh[k]) - F[k]) + (mu_hi[kMuLo + qd[k]] - cRl[k]);
-            r = ((mu_hi[qs[k]] - cFh[k]) - R[k]) + (mu_hi[kMuLo + qs[k]] - cFl[k]);
-          } else {
-            f = (mu_hi[qd[k]] - cRh[k]) - F[k];
-            r = (mu_hi[qs[k]] - cFh[k]) - R[k];
-          }
           if (qo + k < Pe) {
-            mxF[k] = fmax(mxF[k], f);
-            mxR[k] = fmax(mxR[k], r);
-            if constexpr (kBatch) {
-              lrv[k][jv] = f + b[k];
-              lfv[k][jv] = r + b[k];
-            } else {
-              lr[k].add_fast(f + b[k]);
-              lf[k].add_fast(r + b[k]);
-            }
-            yo[k] = f - em[k];  // no out-edges: dEmin = +inf, Y = -inf
-            zo[k] = r;
-            fo[k] = f;
-          } else {
-            yo[k] = zo[k] = fo[k] = T(0);
+            mxF[k] = fmaxf(mxF[k], f[k]);
+            mxR[k] = fmaxf(mxR[k], r[k]);
+            lrv[k][jv] = f[k] + b[k];
+            lfv[k][jv] = r[k] + b[k];
+          }
+          yo[k] = qo + k < Pe ? f[k] - em[k] : 0.f;  // no out-edges: dEmin = +inf, Y = -inf
+          if (qo + k >= Pe) f[k] = r[k] = 0.f;
+        }
+        st_n<QPL>(a.vf + v * Pp + qo, yo);
+        st_n<QPL>(a.vr_out + v * Pp + qo, r);
+        if constexpr (REC) {
+          if (a.rec_f) {
+            st_n<QPL>(a.rec_f + v * Pp + qo, f);
+            st_n<QPL>(a.rec_r + v * Pp + qo, r);
           }
         }
-        st_n<T, QPL>(a.vf + (size_t)v * Pp + qo, yo);
-        st_n<T, QPL>(a.vr_out + (size_t)v * Pp + qo, zo);
-        if (a.rec_f) {
-          st_n<T, QPL>(a.rec_f + (size_t)v * Pp + qo, fo);
-          st_n<T, QPL>(a.rec_r + (size_t)v * Pp + qo, zo);
-        }
       }
     }
-    if constexpr (kBatch) {
 #pragma unroll
-      for (int k = 0; k < QPL; ++k) {
-        lr[k].add4_fast(lrv[k][0], lrv[k][1], lrv[k][2], lrv[k][3]);
-        lf[k].add4_fast(lfv[k][0], lfv[k][1], lfv[k][2], lfv[k][3]);
-      }
-#pragma unroll
-      for (int j = 0; j < PPL; ++j) lmu[j].add2x4_fast(muh[j], mul[j]);
+    for (int k = 0; k < QPL; ++k) {
+      lr[k].add4_fast(lrv[k][0], lrv[k][1], lrv[k][2], lrv[k][3]);
+      lf[k].add4_fast(lfv[k][0], lfv[k][1], lfv[k][2], lfv[k][3]);
     }
+#pragma unroll
+    for (int j = 0; j < PPL; ++j) lmu[j].add2x4_fast(muh[j], mul[j]);
     __syncwarp();  // this stage's buffer is free for the stage after next
   }
   cp_wait0();
@@ -1246,7 +1238,7 @@ vertex_warp_kernel(const VertexUpdArgs<T> a) {
   }
   __syncthreads();
   write_block_partials(red, kVw, nmax, nlse, a.bpart, gridDim.x, blockIdx.x,
-                       sizeof(T) == 4 ? kMergeF32 : kMergeFx);
+                       kMergeF32);
 }
 
 template <typename T>
@@ -1336,11 +1328,11 @@ size_t vertex_update_smem(int pn, int pe, int pp) {
   return UpdSmem(kBT / nvec, pn, pe, pp, pnp, sizeof(T)).total;
 }
 
-template <typename T, int QPL, int PPL>
+template <int QPL, int PPL, bool REC>
 size_t vertex_warp_setup(int pn, int pe, int pp, int pnp, int nterms) {
-  const size_t sm = VwSmem<T, QPL, PPL>(pn, pe, pp, pnp, nterms).total;
+  const size_t sm = VwSmem<PPL>(pn, pe, pp, pnp, nterms).total;
   if (sm > 48 * 1024)
-    cudaFuncSetAttribute(vertex_warp_kernel<T, QPL, PPL>,
+    cudaFuncSetAttribute(vertex_warp_kernel<QPL, PPL, REC>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   return sm;
 }
@@ -1364,8 +1356,12 @@ acg_status launch_vertex_update(const VertexUpdArgs<T>& a, int blocks, cudaStrea
   if (a.vsched == nullptr && a.Pn > 0 && a.Pn <= 64 && a.Pp <= 64)
     return set_error(ACG_ERR_INVALID_ARGUMENT, "vertex phase: no schedule for the warp form");
   const bool warp = warp_form(a.Pn, a.Pp, [&]<int QPL, int PPL>() {
-    const size_t sm = vertex_warp_setup<T, QPL, PPL>(a.Pn, a.Pe, a.Pp, a.Pnp, a.vterms);
-    le = launch_kernel(a.early, vertex_warp_kernel<T, QPL, PPL>, blocks, kBT, sm, s, a);
+    auto go = [&]<bool REC>() {
+      const size_t sm = vertex_warp_setup<QPL, PPL, REC>(a.Pn, a.Pe, a.Pp, a.Pnp, a.vterms);
+      le = launch_kernel(a.early, vertex_warp_kernel<QPL, PPL, REC>, blocks, kBT, sm, s, a);
+    };
+    if (a.rec_f || a.rec_mh) go.template operator()<true>();
+    else go.template operator()<false>();
   });
   if (warp) {
     if (le != cudaSuccess)
@@ -1385,8 +1381,8 @@ template <typename T>
 int vertex_update_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms, int dn) {
   int nb = 0;
   const bool warp = warp_form(pn, pp, [&]<int QPL, int PPL>() {
-    const size_t sm = vertex_warp_setup<T, QPL, PPL>(pn, pe, pp, pnp, nterms);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, vertex_warp_kernel<T, QPL, PPL>, kBT,
+    const size_t sm = vertex_warp_setup<QPL, PPL, false>(pn, pe, pp, pnp, nterms);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, vertex_warp_kernel<QPL, PPL, false>, kBT,
                                                       sm) != cudaSuccess)
       nb = 1;
   });

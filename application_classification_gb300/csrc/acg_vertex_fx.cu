@@ -580,7 +580,7 @@ void fx_form(int pn, int pp, F&& f) {
 int vertex_fx_warps(int pn, int pp) { return pp <= 64 && pn <= 64 ? 1 : pp <= 128 ? 2 : 4; }
 
 int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out) {
-  return vertex_warp_schedule(pat, pn, pe, pp, pnp, kFxVps, out, 32 * vertex_fx_warps(pn, pp));
+  return vertex_warp_schedule(pat, pn, pe, pp, pnp, kFxVps, out, 32 * vertex_fx_warps(pn, pp), 2, 8);
 }
 
 acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s) {
