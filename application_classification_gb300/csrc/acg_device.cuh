@@ -285,6 +285,36 @@ __device__ __forceinline__ void write_block_partials(const double* red, int nwar
   }
 }
 
+// The same for FP32 statistics, maxima kept as floats: warp w's are red_m[w * (nmax +
+// nlse) ...], its sums red_s[w * nlse ...].  The results are write_block_partials'
+// with kMergeF32, bit for bit: a difference of two floats rounds to FP32 alike from
+// FP64 and from the exact value.
+__device__ __forceinline__ void write_block_partials_f32(const float* red_m, const double* red_s,
+                                                         int nwarps, int nmax, int nlse,
+                                                         double* bpart, int ncols, int col) {
+  const int nm = nmax + nlse;
+  for (int j = threadIdx.x; j < nm; j += blockDim.x) {
+    float m = -CUDART_INF_F;
+    if (j < nmax) {
+      for (int w = 0; w < nwarps; ++w) m = fmaxf(m, red_m[w * nm + j]);
+      bpart[(size_t)j * ncols + col] = (double)m;
+    } else {
+      const int i = j - nmax;
+      double s = 0.0;
+      auto nonempty = [&](int w) {
+        return red_m[w * nm + j] > -CUDART_INF_F && (__double_as_longlong(red_s[w * nlse + i]) << 1) != 0;
+      };
+      for (int w = 0; w < nwarps; ++w)
+        if (nonempty(w)) m = fmaxf(m, red_m[w * nm + j]);
+      if (m > -CUDART_INF_F)
+        for (int w = 0; w < nwarps; ++w)
+          if (nonempty(w)) s += red_s[w * nlse + i] * (double)expf(red_m[w * nm + j] - m);
+      bpart[(size_t)(nmax + 2 * i) * ncols + col] = (double)m;
+      bpart[(size_t)(nmax + 2 * i + 1) * ncols + col] = s;
+    }
+  }
+}
+
 // Compensated running sum for FP32 (TwoSum: hi + lo carries the exact sum of
 // the added terms to within one rounding); plain sum for FP64.
 template <typename T>

@@ -957,53 +957,71 @@ vertex_warp_kernel(const VertexUpdArgs<float> a) {
   const int* s_psrc = s_pat;
   const int* s_pdst = s_pat + Pe;
 
-  // per-q constants of the lane's columns (see the tile form for the algebra)
+  // per-q constants (see the tile form for the algebra), formed once per block: FP64
+  // arithmetic, 16 cycles an instruction and SM.  By every warp for its lanes they
+  // were 8 us of a launch at 64 columns, whatever the graph's size.
   const double* g = a.glob_in;
   const int x0 = 4 * Pe + Pn;
   const int qo = lane * QPL;
   const bool qon = qo < Pp;
-  float fF[QPL], fR[QPL], dFh[QPL], dFl[QPL], dRh[QPL], dRl[QPL], cRh[QPL], cRl[QPL], cFh[QPL], cFl[QPL];
-  int qd[QPL], qs[QPL];
-#pragma unroll
-  for (int k = 0; k < QPL; ++k) {
-    const int q = qo + k;
-    fF[k] = fR[k] = dFh[k] = dFl[k] = dRh[k] = dRl[k] = cRh[k] = cRl[k] = cFh[k] = cFl[k] = 0.f;
-    qd[k] = qs[k] = 0;
+  float* s_cst = reinterpret_cast<float*>(smem + L.mu);  // [10][Pp], before the first sums
+  for (int q = tid; q < Pp; q += kBT) {
+    float c[10] = {};
     if (q < Pe) {
-      qd[k] = s_pdst[q];
-      qs[k] = s_psrc[q];
       const double cRu = g[x0 + q], cFu = g[x0 + Pe + q];
       const double dR = g[2 * Pe + q], dF = g[3 * Pe + q];
-      double fr = g[q] + cRu - g[4 * Pe + qd[k]];
-      double ff = g[Pe + q] + cFu - g[4 * Pe + qs[k]];
+      double fr = g[q] + cRu - g[4 * Pe + s_pdst[q]];
+      double ff = g[Pe + q] + cFu - g[4 * Pe + s_psrc[q]];
       if (a.cnull) {
         fr -= a.cnull[q];
         ff -= a.cnull[q];
       }
-      fR[k] = (float)fr;
-      fF[k] = (float)ff;
-      dRh[k] = (float)dR;
-      dRl[k] = (float)(dR - (double)dRh[k]);
-      dFh[k] = (float)dF;
-      dFl[k] = (float)(dF - (double)dFh[k]);
       const double lRp = cRu + dR, lFp = cFu + dF;
       double cRn = a.first ? lRp : g[x0 + 2 * Pe + q];
       double cFn = a.first ? lFp : g[x0 + 3 * Pe + q];
       if (!isfinite(cRn)) cRn = 0.0;
       if (!isfinite(cFn)) cFn = 0.0;
-      cRh[k] = (float)cRn;
-      cRl[k] = (float)(cRn - (double)cRh[k]);
-      cFh[k] = (float)cFn;
-      cFl[k] = (float)(cFn - (double)cFh[k]);
-      if (blockIdx.x == 0 && wib == 0) {
+      c[0] = (float)ff;
+      c[1] = (float)fr;
+      c[2] = (float)dF;
+      c[3] = (float)(dF - (double)c[2]);
+      c[4] = (float)dR;
+      c[5] = (float)(dR - (double)c[4]);
+      c[6] = (float)cRn;
+      c[7] = (float)(cRn - (double)c[6]);
+      c[8] = (float)cFn;
+      c[9] = (float)(cFn - (double)c[8]);
+      if (blockIdx.x == 0) {
         double* o = a.glob_out;
-        o[x0 + q] = (double)cRh[k] + (double)cRl[k];
-        o[x0 + Pe + q] = (double)cFh[k] + (double)cFl[k];
+        o[x0 + q] = (double)c[6] + (double)c[7];
+        o[x0 + Pe + q] = (double)c[8] + (double)c[9];
         o[x0 + 2 * Pe + q] = lRp;
         o[x0 + 3 * Pe + q] = lFp;
       }
     }
+#pragma unroll
+    for (int x = 0; x < 10; ++x) s_cst[x * Pp + q] = c[x];
   }
+  __syncthreads();
+  float fF[QPL], fR[QPL], dFh[QPL], dFl[QPL], dRh[QPL], dRl[QPL], cRh[QPL], cRl[QPL], cFh[QPL], cFl[QPL];
+  int qd[QPL], qs[QPL];
+#pragma unroll
+  for (int k = 0; k < QPL; ++k) {
+    const int q = min(qo + k, Pp - 1);
+    fF[k] = s_cst[q];
+    fR[k] = s_cst[Pp + q];
+    dFh[k] = s_cst[2 * Pp + q];
+    dFl[k] = s_cst[3 * Pp + q];
+    dRh[k] = s_cst[4 * Pp + q];
+    dRl[k] = s_cst[5 * Pp + q];
+    cRh[k] = s_cst[6 * Pp + q];
+    cRl[k] = s_cst[7 * Pp + q];
+    cFh[k] = s_cst[8 * Pp + q];
+    cFl[k] = s_cst[9 * Pp + q];
+    qd[k] = q < Pe ? s_pdst[q] : 0;
+    qs[k] = q < Pe ? s_psrc[q] : 0;
+  }
+  __syncthreads();  // the MU_raw rows take the constants' place
   float mxF[QPL], mxR[QPL];
   OnlineLse<float> lr[QPL], lf[QPL], lmu[PPL];
   bool any_last = false;
@@ -1213,32 +1231,33 @@ vertex_warp_kernel(const VertexUpdArgs<float> a) {
   cp_wait0();
   __syncthreads();  // the rings become the reduction area
 
-  const int nmax = 2 * Pe, nlse = 2 * Pe + Pn, slots = nmax + 2 * nlse;
-  double* red = reinterpret_cast<double*>(smem + L.ring);
-  double* r = red + (size_t)wib * slots;
+  const int nmax = 2 * Pe, nlse = 2 * Pe + Pn;
+  double* red_s = reinterpret_cast<double*>(smem + L.ring);
+  float* red_m = reinterpret_cast<float*>(red_s + (size_t)kVw * nlse);
+  double* rs = red_s + (size_t)wib * nlse;
+  float* rm = red_m + (size_t)wib * (nmax + nlse);
 #pragma unroll
   for (int k = 0; k < QPL; ++k) {
     const int q = qo + k;
     if (q < Pe) {
-      r[q] = (double)mxF[k];
-      r[Pe + q] = (double)mxR[k];
-      r[nmax + 2 * q] = lr[k].mval();
-      r[nmax + 2 * q + 1] = lr[k].sval();
-      r[nmax + 2 * (Pe + q)] = lf[k].mval();
-      r[nmax + 2 * (Pe + q) + 1] = lf[k].sval();
+      rm[q] = mxF[k];
+      rm[Pe + q] = mxR[k];
+      rm[nmax + q] = lr[k].m;
+      rs[q] = lr[k].sval();
+      rm[nmax + Pe + q] = lf[k].m;
+      rs[Pe + q] = lf[k].sval();
     }
   }
 #pragma unroll
   for (int j = 0; j < PPL; ++j) {
     const int p = lane + 32 * j;
     if (p < Pn) {
-      r[nmax + 2 * (2 * Pe + p)] = lmu[j].mval();
-      r[nmax + 2 * (2 * Pe + p) + 1] = lmu[j].sval();
+      rm[nmax + 2 * Pe + p] = lmu[j].m;
+      rs[2 * Pe + p] = lmu[j].sval();
     }
   }
   __syncthreads();
-  write_block_partials(red, kVw, nmax, nlse, a.bpart, gridDim.x, blockIdx.x,
-                       kMergeF32);
+  write_block_partials_f32(red_m, red_s, kVw, nmax, nlse, a.bpart, gridDim.x, blockIdx.x);
 }
 
 template <typename T>
