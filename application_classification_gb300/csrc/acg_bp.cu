@@ -129,26 +129,48 @@ __device__ void block_partials_out(const double* red, int nwarps, StatSpec spec,
 }
 
 // ------------------------------------------------------------- finalize
+// A double as a signed integer of the same order, NaN as -inf (fmax passes it over).
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  const long long k = b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+  constexpr long long kInf = 0x7ff0000000000000LL;
+  return (b & 0x7fffffffffffffffLL) > kInf ? ~kInf : k;  // ~kInf: the key of -inf
+}
+__device__ __forceinline__ double order_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+
+// One block per output.  A launch of a microsecond's work in a chain of kernels, so
+// bound by its own latency: the partials are read once and kept (two a thread; more
+// blocks than that are read again), and the maxima compare as integers, FP64
+// compares being 16 cycles an instruction and SM.
 __global__ void __launch_bounds__(256)
 stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spec,
                      double* __restrict__ out, const StatCapture cap) {
-  __shared__ double sm[8], ss[8];
+  __shared__ long long sm[8];
+  __shared__ double ss[8];
+  const int o = blockIdx.x, p = o - cap.first;
+  const bool capture = cap.iters_p && p >= 0 && cap.iters_p[p] == cap.t;
   dep_launch();
   dep_wait();
-  const int o = blockIdx.x;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (o < spec.nmax) {
-    double m = -CUDART_INF;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) m = fmax(m, bpart[(size_t)o * nblocks + b]);
+  auto block_max = [&](long long m) {
 #pragma unroll
-    for (int k = 16; k >= 1; k >>= 1) m = fmax(m, shfl_xor_d(m, k));
+    for (int k = 16; k >= 1; k >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, k));
     if (lane == 0) sm[w] = m;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double r = sm[0];
-      for (int k = 1; k < 8; ++k) r = fmax(r, sm[k]);
-      out[o] = r;
-    }
+    m = sm[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) m = max(m, sm[k]);
+    return order_value(m);
+  };
+  const long long none = order_key(-CUDART_INF);
+  long long mk = none;
+  if (o < spec.nmax) {
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+      mk = max(mk, order_key(bpart[(size_t)o * nblocks + b]));
+    const double m = block_max(mk);
+    if (threadIdx.x == 0) out[o] = m;
   } else {
     // two passes: the largest m of the non-empty partials, then the sum of
     // s_b exp(m_b - m) -- one independent exponential per partial; the sum
@@ -156,19 +178,31 @@ stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spe
     const int sl = spec.nmax + 2 * (o - spec.nmax);
     const double* pm = bpart + (size_t)sl * nblocks;
     const double* ps = bpart + (size_t)(sl + 1) * nblocks;
-    double m = -CUDART_INF;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-      if (lse_nonempty(pm[b], ps[b])) m = fmax(m, pm[b]);
+    constexpr int kKept = 2;
+    double vm[kKept], vs[kKept];
 #pragma unroll
-    for (int k = 16; k >= 1; k >>= 1) m = fmax(m, shfl_xor_d(m, k));
-    if (lane == 0) sm[w] = m;
-    __syncthreads();
-    m = sm[0];
-    for (int k = 1; k < 8; ++k) m = fmax(m, sm[k]);
+    for (int k = 0; k < kKept; ++k) {
+      const int b = threadIdx.x + 256 * k;
+      vm[k] = b < nblocks ? pm[b] : -CUDART_INF;
+      vs[k] = b < nblocks ? ps[b] : 0.0;
+    }
+    auto nonempty = [&](double m, double s) {  // (lse_nonempty)
+      return order_key(m) > none && (__double_as_longlong(s) << 1) != 0;
+    };
+#pragma unroll
+    for (int k = 0; k < kKept; ++k)
+      if (nonempty(vm[k], vs[k])) mk = max(mk, order_key(vm[k]));
+    for (int b = threadIdx.x + 256 * kKept; b < nblocks; b += 256)
+      if (nonempty(pm[b], ps[b])) mk = max(mk, order_key(pm[b]));
+    const double m = block_max(mk);
     double s = 0.0;
-    if (m > -CUDART_INF)
-      for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-        if (lse_nonempty(pm[b], ps[b])) s += ps[b] * merge_exp(pm[b] - m, spec.mode);
+    if (order_key(m) > none) {
+#pragma unroll
+      for (int k = 0; k < kKept; ++k)
+        if (nonempty(vm[k], vs[k])) s += vs[k] * merge_exp(vm[k] - m, spec.mode);
+      for (int b = threadIdx.x + 256 * kKept; b < nblocks; b += 256)
+        if (nonempty(pm[b], ps[b])) s += ps[b] * merge_exp(pm[b] - m, spec.mode);
+    }
 #pragma unroll
     for (int k = 16; k >= 1; k >>= 1) s += shfl_xor_d(s, k);
     if (lane == 0) ss[w] = s;
@@ -178,8 +212,7 @@ stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spe
       for (int k = 0; k < 8; ++k) t += ss[k];
       const double r = (m > -CUDART_INF && t > 0.0) ? m + log(t) : -CUDART_INF;
       out[o] = r;
-      const int p = o - cap.first;
-      if (cap.iters_p && p >= 0 && cap.iters_p[p] == cap.t) cap.S_final[p] = r;
+      if (capture) cap.S_final[p] = r;
     }
   }
 }
