@@ -1405,7 +1405,9 @@ int vertex_update_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sm
                                                       sm) != cudaSuccess)
       nb = 1;
   });
-  if (warp) return num_sms * (nb < 1 ? 1 : nb);
+  // (two per SM at most, whatever registers the compiler takes: the grid fixes the
+  // warps' ranges of vertices, and with them the statistics' order of summation)
+  if (warp) return num_sms * std::min(std::max(nb, 1), 2);
   const int V = kBT / (pp / VecT<T>::W);
   const long long tiles = (dn + V - 1) / V;
   const long long b = (long long)num_sms * vertex_update_blocks_per_sm<T>(pn, pe, pp);

@@ -333,6 +333,32 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   const int* s_psrc = s_pat;
   const int* s_pdst = s_pat + Pe;
 
+  const int gl = tid % (32 * NW), group = tid / (32 * NW);
+  const long long ng = (long long)gridDim.x * kNG;
+  const long long gg = (long long)blockIdx.x * kNG + group;
+  const int vb = (int)(gg * Dn / ng), ve = (int)((gg + 1) * Dn / ng);
+  unsigned char* ring = smem + L.ring + (size_t)group * L.group_ring;
+  const size_t rowb = (size_t)Pp * 8, crow = (size_t)Pnp * 8;
+  auto issue = [&](int v0, int buf) {
+    const int nv = min(kFxVps, ve - v0);
+    if (nv <= 0) return;
+    unsigned char* st = ring + (size_t)buf * L.stage;
+    const int n16 = (int)((size_t)nv * rowb / 16);
+    const size_t go = (size_t)v0 * rowb;
+    for (int c = gl; c < n16; c += 32 * NW) {
+      fcp16(st + G.oM * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.M) + go + c * 16);
+      fcp16(st + G.oY * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.vf) + go + c * 16);
+      fcp16(st + G.oE * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.dEmin) + go + c * 16);
+      fcp16(st + G.oB * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.B) + go + c * 16);
+    }
+    const int c16 = (int)((size_t)nv * crow / 16);
+    const size_t co = (size_t)v0 * crow;
+    for (int c = gl; c < c16; c += 32 * NW)
+      fcp16(st + G.oC * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.CV) + co + c * 16);
+  };
+  issue(vb, 0);  // (flies while the constants are formed)
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+
   // ---- the columns' constants (acg_iter.cu has the algebra), their bounds
   const double* g = a.glob_in;
   const int x0 = 4 * Pe + Pn;
@@ -394,7 +420,18 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   // (at most 50: finer than a double from 4 on, and B, dEmin may reach 2^10)
   const int Q = fixed ? min(50, 60 - ((__float_as_int(bound) >> 23) - 126)) : 47;
 
-  const int gl = tid % (32 * NW), group = tid / (32 * NW);
+  // in fixed point, once per block (the second stage of the first group's ring: not
+  // yet in use; 48 Pp bytes of at least 64 Pp); the shifts also as they are
+  // subtracted: multiples of 2^-Q, exact as doubles
+  static_assert(kFxVps >= 2, "room for the columns' constants");
+  long long* s_fix = reinterpret_cast<long long*>(smem + L.ring + L.stage);
+  for (int t = tid; t < 6 * Pp; t += kFT) {
+    const long long k = fixed ? __double2ll_rn(s_cst[t] * (double)(1ull << Q)) : 0ll;
+    s_fix[t] = k;
+    if (fixed && t >= 4 * Pp) s_cst[t] = (double)k * (1.0 / (double)(1ull << Q));
+  }
+  __syncthreads();
+
   const int qo = gl * QPL;
   uint64_t* s_tab = reinterpret_cast<uint64_t*>(smem + L.tab);
   const FxAr fx{Q, fx_scaled_factor(Q), (uint32_t)(1083 - Q) << 20, s_tab};
@@ -405,9 +442,7 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   for (int k = 0; k < QPL; ++k) {
     const int q = qo + k;
     const bool on = q < Pp;
-    auto cst = [&](int i) {  // rounded to Q fraction bits
-      return on && fixed ? __double2ll_rn(s_cst[i * Pp + q] * (double)(1ull << Q)) : 0ll;
-    };
+    auto cst = [&](int i) { return on ? s_fix[i * Pp + q] : 0ll; };  // rounded to Q fraction bits
     fFx[k] = cst(0);
     fRx[k] = cst(1);
     dFx[k] = cst(2);
@@ -420,15 +455,7 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
     fx_init(S.lf[k]);
     S.mxF[k] = S.mxR[k] = (long long)0x8000000000000000ull;
   }
-  if (fixed) {
-    // the shifts as they are subtracted: multiples of 2^-Q, exact as doubles
-    __syncthreads();
-    for (int q = tid; q < Pp; q += kFT)
-      for (int i = 4; i < 6; ++i)
-        s_cst[i * Pp + q] = (double)__double2ll_rn(s_cst[i * Pp + q] * (double)(1ull << Q)) *
-                            (1.0 / (double)(1ull << Q));
-  }
-  __syncthreads();
+  __syncthreads();  // s_fix is read: the ring may fill
   if (blockIdx.x == 0)
     for (int q = tid; q < Pe; q += kFT) {
       a.glob_out[x0 + q] = s_cst[5 * Pp + q];
@@ -442,30 +469,6 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
     if (p < Pn && __ldg(a.iters_p + p) == a.t) plast |= 1u << j;
   }
 
-  const long long ng = (long long)gridDim.x * kNG;
-  const long long gg = (long long)blockIdx.x * kNG + group;
-  const int vb = (int)(gg * Dn / ng), ve = (int)((gg + 1) * Dn / ng);
-  unsigned char* ring = smem + L.ring + (size_t)group * L.group_ring;
-  StageCtx x{&a, nullptr, reinterpret_cast<double*>(smem + L.mu) + (size_t)group * L.mu_n, s_sched,
-             s_mxd + (size_t)group * 2 * Pp, gl, group, 0, 0, L.mu_row};
-  const size_t rowb = (size_t)Pp * 8, crow = (size_t)Pnp * 8;
-  auto issue = [&](int v0, int buf) {
-    const int nv = min(kFxVps, ve - v0);
-    if (nv <= 0) return;
-    unsigned char* st = ring + (size_t)buf * L.stage;
-    const int n16 = (int)((size_t)nv * rowb / 16);
-    const size_t go = (size_t)v0 * rowb;
-    for (int c = gl; c < n16; c += 32 * NW) {
-      fcp16(st + G.oM * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.M) + go + c * 16);
-      fcp16(st + G.oY * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.vf) + go + c * 16);
-      fcp16(st + G.oE * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.dEmin) + go + c * 16);
-      fcp16(st + G.oB * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.B) + go + c * 16);
-    }
-    const int c16 = (int)((size_t)nv * crow / 16);
-    const size_t co = (size_t)v0 * crow;
-    for (int c = gl; c < c16; c += 32 * NW)
-      fcp16(st + G.oC * 8 + c * 16, reinterpret_cast<const unsigned char*>(a.CV) + co + c * 16);
-  };
   // The stage's M, Y and CV rows again, where fixed point had begun on them (Y's
   // row in memory is rewritten at the end of its stage only).
   auto restage = [&](int v0, int nv, unsigned char* st) {
@@ -480,8 +483,8 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
       *reinterpret_cast<uint4*>(st + G.oC * 8 + c * 16) =
           *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.CV) + (size_t)v0 * crow + c * 16);
   };
-  issue(vb, 0);
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  StageCtx x{&a, nullptr, reinterpret_cast<double*>(smem + L.mu) + (size_t)group * L.mu_n, s_sched,
+             s_mxd + (size_t)group * 2 * Pp, gl, group, 0, 0, L.mu_row};
   int buf = 0;
   for (int v0 = vb; v0 < ve; v0 += kFxVps, buf ^= 1) {
     issue(v0 + kFxVps, buf ^ 1);  // the next stage flies while this one computes
