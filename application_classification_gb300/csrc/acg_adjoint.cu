@@ -1381,7 +1381,9 @@ struct Adj {
 
   acg_status scatter() {
     ScatArgs<T> a{P->sw.items, P->sw.wsplit, D->pos_in_dst, D->scsr.other, W->emask, (const T*)W->gM,
-                  (T*)W->gVRe, (T*)W->pscat, Pp, Pe, P->sw.nparts, P->range_ctr};
+                  (T*)W->gVRe, (T*)W->pscat, Pp, Pe, P->sw.nparts,
+                  // (every range some warp's first: no claims)
+                  P->sw.nparts > P->src_blocks * (kT / 32) ? P->range_ctr : nullptr};
     ACG_TRY(fill(W->gVRe, vrow(), T(0)));  // sources without out-edges
     bool done = false;
 #define ADJ_SC(NP_, NQ_)                                                        \
