@@ -13,12 +13,15 @@
 //   warp: a warp walks its own range, then claims further ranges from a
 //   counter as it finishes, so the SMs stay full until the last ranges.  Every
 //   item is written by exactly one warp, whichever it is, so the result does
-//   not depend on the order of the claims.  A chunk writes a partial row;
-//   heavy_combine_kernel takes the max of a heavy vertex's partial rows.
+//   not depend on the order of the claims.  A chunk writes a partial row; the max
+//   of a heavy vertex's partial rows is taken by the warp that finishes the last
+//   one (FP32 without argmax) or by heavy_combine_kernel.
 //
-// Phase B, vertex_warp_kernel (patterns up to 64 x 64) -- one warp per
+// Phase B, vertex_warp_kernel (FP32, patterns up to 64 x 64) -- one warp per
 //   contiguous vertex range, rows staged per warp with cp.async; see its own
-//   comment.  The block-tile form below it serves larger patterns.
+//   comment.  FP32 patterns of more than 64 edge columns take acg_vertex_wide.cu's
+//   kernel, FP64 ones acg_vertex_fx.cu's; the block-tile form below is left with
+//   FP32 patterns of up to 64 edge columns and more than 64 vertices.
 //
 // Phase B, vertex_update_kernel -- everything per vertex, streamed with
 //   coalesced 16-byte accesses: FMax, RMax, MU_raw (compensated sum), the next
@@ -703,11 +706,9 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
     const T* gCV = a.CV + (size_t)v0 * Pnp;
     T* sCV = reinterpret_cast<T*>(st + L.sCV);
     for (int c = tid * W; c < nv * Pnp; c += kBT * W) cp16(sCV + c, gCV + c);
-    if constexpr (sizeof(T) == 4) {
-      const T* gCVl = a.CVlo + (size_t)v0 * Pnp;
-      T* sCVl = reinterpret_cast<T*>(st + L.sCVl);
-      for (int c = tid * W; c < nv * Pnp; c += kBT * W) cp16(sCVl + c, gCVl + c);
-    }
+    const T* gCVl = a.CVlo + (size_t)v0 * Pnp;
+    T* sCVl = reinterpret_cast<T*>(st + L.sCVl);
+    for (int c = tid * W; c < nv * Pnp; c += kBT * W) cp16(sCVl + c, gCVl + c);
     int* sOff = reinterpret_cast<int*>(st + L.sOff);
     for (int j = tid; j <= nv; j += kBT) cp4(sOff + j, a.d_off + v0 + j);
   };
@@ -760,12 +761,11 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
       const T* rowR = s_R + j * Pp;
       CSum<T> mu;
       mu.init(-sCV[j * Pnp + pc]);
-      if constexpr (sizeof(T) == 4)
-        mu.lo = -reinterpret_cast<const T*>(st + L.sCVl)[j * Pnp + pc];
+      mu.lo = -reinterpret_cast<const T*>(st + L.sCVl)[j * Pnp + pc];
       for (int t = in0; t < in1; ++t) mu.add(rowF[s_inq[t]]);
       for (int t = out0; t < out1; ++t) mu.add(rowR[s_outq[t]]);
       s_MU[j * Pn + pc] = mu.hi;
-      if constexpr (sizeof(T) == 4) s_MUlo[j * Pn + pc] = mu.lo;
+      s_MUlo[j * Pn + pc] = mu.lo;
       lmu.add2(mu.hi, mu.lo);
       if (my_last) a.mu_raw[(size_t)vv * Pn + pc] = mu.dvalue();
     }
@@ -781,16 +781,10 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
         // f = VF' - cR, r = VR' - cF; the shift is taken off the compensated
         // MU_raw first (for the entries that matter the two are close, so the
         // difference is exact) and the small message after
-        T f, r;
-        if constexpr (sizeof(T) == 4) {
-          const VT cRl = *reinterpret_cast<const VT*>(s_cRlo + qv * W);
-          const VT cFl = *reinterpret_cast<const VT*>(s_cFlo + qv * W);
-          f = ((myMU[pdst[w]] - vg<T>(cR, w)) - vg<T>(fo, w)) + (myMUlo[pdst[w]] - vg<T>(cRl, w));
-          r = ((myMU[psrc[w]] - vg<T>(cF, w)) - vg<T>(ro, w)) + (myMUlo[psrc[w]] - vg<T>(cFl, w));
-        } else {
-          f = (myMU[pdst[w]] - vg<T>(cR, w)) - vg<T>(fo, w);
-          r = (myMU[psrc[w]] - vg<T>(cF, w)) - vg<T>(ro, w);
-        }
+        const VT cRl = *reinterpret_cast<const VT*>(s_cRlo + qv * W);
+        const VT cFl = *reinterpret_cast<const VT*>(s_cFlo + qv * W);
+        const T f = ((myMU[pdst[w]] - vg<T>(cR, w)) - vg<T>(fo, w)) + (myMUlo[pdst[w]] - vg<T>(cRl, w));
+        T r = ((myMU[psrc[w]] - vg<T>(cF, w)) - vg<T>(ro, w)) + (myMUlo[psrc[w]] - vg<T>(cFl, w));
         T y;
         if (qv * W + w < Pe) {
           mxF[w] = fmax(mxF[w], f);
@@ -882,6 +876,12 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
 // Every sum keeps its terms and their order, so the results do not depend on
 // how the jobs are spread.  Vertices without in-edges have M rows of -inf (set
 // once, never written by phase A).
+// Bound by instruction issue (2.7 of 4 a cycle from 16 warps an SM) and the shared
+// memory pipe: one more load a term cost 5%.  R-MAT 22, pattern 32/64 (3.2 GB,
+// 0.47 ms at the copy bandwidth): 1.74 ms an iteration with 102.9 M instructions
+// and 10.1 M conflict cycles at R-MAT 18, 1.59 ms with 88.7 M and 5.3 M so.  The
+// tail of a stage by a branch (predicated: 1% slower).  On a small graph a launch
+// is its constants and its block partials.
 constexpr int kVps = 4;  // vertices per stage (one add4_fast per column)
 constexpr int kVw = kBT / 32;
 template <int PPL>
