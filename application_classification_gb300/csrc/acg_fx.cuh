@@ -101,7 +101,7 @@ ACG_FX_HD int32_t fx_mulhi(int32_t a, int32_t b) {
 #endif
 }
 
-// |x| below this (2^14) takes the integer path; the high word's bits
+// |x| below this (2^14) takes fx_add's integer path; the high word's bits
 constexpr uint32_t kFxLimit = 0x40d00000u;
 
 // exp(x) = 2^k f / 2^61 from x with 60 fraction bits modulo 2^64 (X) and
@@ -244,8 +244,9 @@ ACG_FX_HD double fx_expd(double x) {
 
 // A log-sum-exp state in four words.  Integer form (bit 31 of w[3] clear):
 // w[0] = K, w[1..3] the 96-bit sum of exp(x) 2^(61 - K).  Wide form (bit set),
-// entered when a value lies outside +-2^14: w[0..1] the running maximum m,
-// w[2..3] minus the sum of exp(x - m), both doubles.
+// entered where the sum is of values beyond +-2^24: w[0..1] the running maximum
+// m, w[2..3] minus the sum of exp(x - m), both doubles.  Only fx_add, fx_add_far
+// and fx_merge take a wide state; fx_add_term does not.
 struct FxLse {
   uint32_t w[4];
 };
@@ -277,25 +278,6 @@ ACG_FX_HD void fx_pair(const FxLse& a, double& m, double& s) {
 #endif
   s = (double)a.w[3] * 8.0 + (double)(((uint64_t)a.w[2] << 32) | a.w[1]) * 0x1p-61;
   s += s * d;
-}
-
-// Value x outside the integer form's range, or a state already wide.
-ACG_FX_SLOW FxLse fx_add_wide(FxLse a, double x) {
-  if (!(x > fx_double(0xfff0000000000000ull))) return a;  // NaN, -inf: nothing
-  double m, s;
-  fx_pair(a, m, s);
-  if (x > m) {
-    s = s > 0.0 ? s * exp(m - x) + 1.0 : 1.0;
-    m = x;
-  } else {
-    s += exp(x - m);
-  }
-  const uint64_t mb = fx_bits(m), sb = fx_bits(-s);
-  a.w[0] = (uint32_t)mb;
-  a.w[1] = (uint32_t)(mb >> 32);
-  a.w[2] = (uint32_t)sb;
-  a.w[3] = (uint32_t)(sb >> 32) | 0x80000000u;
-  return a;
 }
 
 // the sum shifted right by sh >= 0 bits
@@ -346,6 +328,55 @@ ACG_FX_HD void fx_add_term(FxLse& a, int k, uint64_t f) {
 #endif
 }
 
+// Value x outside fx_add's range (|x| >= 2^14), or a state already wide.  Up to
+// 2^24 the integer form holds it, n rounded from FP64 (the series' argument is
+// formed modulo 2^64 as before).  A term more than e^-100 below the sum adds
+// nothing, and a wide sum more than that below x is dropped for x: so one vertex
+// far from everything leaves the state in integer form, or returns it there with
+// the next ordinary value.
+constexpr double kFxFar = 100.0;
+ACG_FX_SLOW FxLse fx_add_far(FxLse a, double x) {
+  if (!(x > fx_double(0xfff0000000000000ull))) return a;  // NaN, -inf: nothing
+  const uint64_t b = fx_bits(x);
+  const uint32_t t = (uint32_t)(b >> 32) & 0x7fffffffu;
+  const bool fits = t < 0x41700000u;
+  double m, s;
+  fx_pair(a, m, s);
+  if (fits && fx_wide(a) && x - m > kFxFar) fx_init(a);  // (s below 2^33)
+  if (!fx_wide(a)) {
+    if (fits) {
+      int k;
+      uint64_t f;
+      if (t < kFxLimit) {
+        f = fx_exp(b, k);
+      } else {
+#ifdef __CUDA_ARCH__
+        const int n = __double2int_rn(x * 92.332482616893656877);
+#else
+        const int n = (int)std::lrint(x * 92.332482616893656877);
+#endif
+        const uint64_t X = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << ((int)(t >> 20) - 1015);
+        f = fx_exp_core((b >> 63) ? 0ull - X : X, n, k);
+      }
+      fx_add_term(a, k, f);
+      return a;
+    }
+    if (s > 0.0 && m - x > kFxFar) return a;
+  }
+  if (x > m) {
+    s = s > 0.0 ? s * exp(m - x) + 1.0 : 1.0;
+    m = x;
+  } else {
+    s += exp(x - m);
+  }
+  const uint64_t mb = fx_bits(m), sb = fx_bits(-s);
+  a.w[0] = (uint32_t)mb;
+  a.w[1] = (uint32_t)(mb >> 32);
+  a.w[2] = (uint32_t)sb;
+  a.w[3] = (uint32_t)(sb >> 32) | 0x80000000u;
+  return a;
+}
+
 ACG_FX_HD void fx_add(FxLse& a, double x) {
   const uint64_t b = fx_bits(x);
   const uint32_t hi = (uint32_t)(b >> 32);
@@ -354,7 +385,7 @@ ACG_FX_HD void fx_add(FxLse& a, double x) {
     const uint64_t f = fx_exp(b, k);
     fx_add_term(a, k, f);
   } else if (hi != 0xfff00000u) {  // (-inf adds nothing)
-    a = fx_add_wide(a, x);
+    a = fx_add_far(a, x);
   }
 }
 

@@ -115,7 +115,7 @@ struct FxAr {
   __device__ __forceinline__ void add(FxLse& l, V x) const {
     int k;
     const uint64_t f = fx_exp_scaled(x, Q, c, tab, k);
-    fx_add_term(l, k, f);  // (a stage with a wide sum runs in FP64)
+    fx_add_term(l, k, f);  // (no sum is wide here: see run_stage)
   }
 };
 struct Fp64Ar {
@@ -147,8 +147,11 @@ struct StageCtx {
 // changed, when the stage holds a value that fixed point does not cover: M or Y
 // at 2^(60 - Q) or beyond (low ones only lose to the fill, as -inf does), CV
 // outside +-2^(60 - Q), a NaN with a clear sign (fmax drops a NaN; a set sign
-// reads as a low value), or a sum that an FP64 stage took out of the integer
-// form.
+// reads as a low value), or a sum that is in the wide form.  B may lie anywhere:
+// the terms of a vertex with a finite B outside +-2^(60 - Q) are added by
+// fx_add_far once the stage's others are, so that fx_add_term never meets the wide
+// form such a term may leave behind (beyond 2^24; the next stage then runs in FP64,
+// whose ordinary terms bring the sum back).
 template <typename A, int QPL, int PPL, int NW>
 __device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const typename A::V (&fF)[QPL],
                                           const typename A::V (&fR)[QPL], const typename A::V (&dF)[QPL],
@@ -229,6 +232,7 @@ __device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const t
   }
   group_sync<NW>(x.group);
   // ---- 3. MU_raw outputs and statistics, the new Y and Z
+  bool far = false;
 #pragma unroll
   for (int jv = 0; jv < kFxVps; ++jv) {
     if (jv >= x.nv) break;
@@ -268,9 +272,8 @@ __device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const t
               const V bx = ar.in(b);
               ar.add(S.lr[k], f + bx);
               ar.add(S.lf[k], r + bx);
-            } else if (hb != 0xfff00000u) {  // (no out-edges, B = -inf: adds nothing)
-              S.lr[k] = fx_add_wide(S.lr[k], ar.out(f) + b);
-              S.lf[k] = fx_add_wide(S.lf[k], ar.out(r) + b);
+            } else {
+              far |= hb != 0xfff00000u;  // (no out-edges, B = -inf: adds nothing)
             }
           } else {
             x.mxd[qo + k] = fmax(x.mxd[qo + k], f);
@@ -301,6 +304,22 @@ __device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const t
         for (int k = 0; k < QPL; ++k) {
           a.rec_f[v * Pp + qo + k] = fo[k];
           a.rec_r[v * Pp + qo + k] = zo[k];
+        }
+      }
+    }
+  }
+  if constexpr (kFx) {
+    if (far) {  // (a.last leaves it clear; the stage's rows are as above)
+#pragma unroll 1
+      for (int jv = 0; jv < x.nv; ++jv) {
+        const V* mu = smu + jv * x.mu_row;
+#pragma unroll
+        for (int k = 0; k < QPL; ++k) {
+          const int i = jv * Pp + qo + k;
+          const double b = x.st[G.oB + i];
+          if (qo + k >= Pe || ((uint32_t)__double2hiint(b) & 0x7fffffffu) < ar.lim) continue;
+          S.lr[k] = fx_add_far(S.lr[k], ar.out((mu[qd[k]] - cR[k]) - sv[G.oM + i]) + b);
+          S.lf[k] = fx_add_far(S.lf[k], ar.out((mu[qs[k]] - cF[k]) - sv[G.oY + i]) + b);
         }
       }
     }
