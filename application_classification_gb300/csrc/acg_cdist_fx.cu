@@ -6,11 +6,13 @@
 // two 32-bit subtractions, and the sum of squares three 64-bit accumulators fed
 // by one wide multiply-add each, so five integer instructions per feature and
 // pair; the sum is exact and its root is formed by fx_root, correctly rounded.
-// The unit is 2^(a - 57) with 2^a twice to four times the largest pattern
-// feature (and the largest of the block's first rows), so a double of the size
-// of the data's keeps all its bits; smaller ones keep 2^-58 of the largest.
-// Pairs closer than 2^-6 of that range, where this could show, and rows or
-// patterns with values outside it (or not finite) are formed in FP64 as before.
+// The unit is 2^(a - 57) with 2^a twice to four times the largest feature of the
+// pattern and of a sample of the rows, so a double of the size of the data's keeps
+// all its bits; smaller ones keep 2^-58 of the largest.  The sample is the same in
+// every block: a row's costs depend on its values, not on its place, and equal rows
+// have equal costs.  Pairs closer than 2^-6 of that range, where the unit could
+// show, and rows or patterns with values outside it (or not finite) are formed in
+// FP64 as before.
 //
 // One thread per row: its features in registers, the pattern's parts in shared
 // memory (broadcast 16-byte loads of two features), two columns at a time.
@@ -29,6 +31,7 @@ namespace acg {
 namespace {
 
 constexpr int kXT = 256;
+constexpr int kSample = 128;  // rows that the scale is formed from, spread over all
 
 // FP64 form of one pair, for what fixed point does not cover.
 __device__ __noinline__ double pair_fp64(const double* __restrict__ x, const double* __restrict__ y,
@@ -61,8 +64,8 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
       if (x != 0x7ff) e = max(e, x);
     };
     for (int t = threadIdx.x; t < P * K; t += kXT) see(a.y[t]);
-    const long long r = (long long)blockIdx.x * kXT + threadIdx.x;
-    if (r < a.nrows) {
+    if (threadIdx.x < kSample) {
+      const long long r = threadIdx.x * a.nrows / kSample;
       const double* xr = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride;
       for (int k = 0; k < K; ++k) see(__ldg(xr + k));
     }
