@@ -2,17 +2,17 @@
 //
 // ||x - y|| over K features takes 2 K FP64 instructions and a root (about 44 at
 // K = 17), each 16 SM cycles per warp: the FP64 edge matrix ran at 0.2 TB/s.
-// Here a feature is fixed point of 57 bits in two parts (FxPart), a difference
-// two 32-bit subtractions, and the sum of squares three 64-bit accumulators fed
-// by one wide multiply-add each, so five integer instructions per feature and
-// pair; the sum is exact and its root is formed by fx_root, correctly rounded.
-// The unit is 2^(a - 57) with 2^a twice to four times the largest feature of the
-// pattern and of a sample of the rows, so a double of the size of the data's keeps
-// all its bits; smaller ones keep 2^-58 of the largest.  The sample is the same in
-// every block: a row's costs depend on its values, not on its place, and equal rows
-// have equal costs.  Pairs closer than 2^-6 of that range, where the unit could
-// show, and rows or patterns with values outside it (or not finite) are formed in
-// FP64 as before.
+// Here a feature is fixed point of W = 57 to 61 bits (the fewer features, the more:
+// FxWindow) in two parts, a difference two 32-bit subtractions, and the sum of
+// squares three 64-bit accumulators fed by one wide multiply-add each, so five
+// integer instructions per feature and pair; the sum of the rounded features'
+// squares is exact, and fx_root forms its root.
+// The unit is 2^(a - W) with 2^a twice to four times the largest feature of the
+// pattern and of a sample of the rows.  The sample is the same in every block: a
+// row's costs depend on its values, not on its place, and equal rows have equal
+// costs.  Pairs so close that the unit would show beside FP64's own roundings, and
+// rows or patterns with values outside the range (or not finite) are formed in
+// FP64.
 //
 // One thread per row: its features in registers, the pattern's parts in shared
 // memory (broadcast 16-byte loads of two features), two columns at a time.
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
     bool bad = false;
     for (int t = threadIdx.x; t < Pp * KM; t += kXT) {
       const int q = t / KM, k = t % KM;
-      s_y[t] = (q < P && k < K) ? fx_part(a.y[(size_t)q * K + k], ax, &bad) : FxPart{0, 0};
+      s_y[t] = (q < P && k < K) ? fx_part<KM>(a.y[(size_t)q * K + k], ax, &bad) : FxPart{0, 0};
     }
     if (bad) s_bad = 1;
   }
@@ -89,11 +89,11 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
        r += (long long)gridDim.x * kXT) {
     const double* xr = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride;
     FxPart x[KM];
-    bool big = ybad;
+    bool big = ybad || K == 1;
 #pragma unroll
     for (int k = 0; k < KM; ++k) {
       x[k] = FxPart{0, 0};
-      if (k < K) x[k] = fx_part(__ldg(xr + k), ax, &big);
+      if (k < K) x[k] = fx_part<KM>(__ldg(xr + k), ax, &big);
     }
     double* orow = a.out + (size_t)r * a.ostride;
     for (int q0 = 0; q0 < Pp; q0 += 2) {
@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
           sl += (uint64_t)((int64_t)l1 * l1);
         }
         if (q0 + j >= P) d[j] = 0.0;
-        else if (big || fx_small(sh)) d[j] = pair_fp64(xr, a.y + (size_t)(q0 + j) * K, K);
-        else d[j] = fx_root(sh, sc, sl, ax);
+        else if (big || fx_small<KM>(sh)) d[j] = pair_fp64(xr, a.y + (size_t)(q0 + j) * K, K);
+        else d[j] = fx_root<KM>(sh, sc, sl, ax);
         if (a.wide && q0 + j < P) d[j] = edge_word(d[j], a.wide);
       }
       *reinterpret_cast<double2*>(orow + q0) = make_double2(d[0], d[1]);
