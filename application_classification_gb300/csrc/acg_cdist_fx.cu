@@ -31,7 +31,7 @@ namespace acg {
 namespace {
 
 constexpr int kXT = 256;
-constexpr int kSample = 128;  // rows that the scale is formed from, spread over all
+constexpr int kSample = 64;  // rows that the scale is formed from, spread over all
 
 // FP64 form of one pair, for what fixed point does not cover.
 __device__ __noinline__ double pair_fp64(const double* __restrict__ x, const double* __restrict__ y,
@@ -63,12 +63,26 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
       const int x = (__double2hiint(v) >> 20) & 0x7ff;
       if (x != 0x7ff) e = max(e, x);
     };
-    for (int t = threadIdx.x; t < P * K; t += kXT) see(a.y[t]);
-    if (threadIdx.x < kSample) {
-      const long long r = threadIdx.x * a.nrows / kSample;
-      const double* xr = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride;
-      for (int k = 0; k < K; ++k) see(__ldg(xr + k));
+    // (kLanes threads to a sampled row, their loads in flight together)
+    constexpr int kLanes = kXT / kSample;
+    const int k0 = threadIdx.x % kLanes;
+    const long long r = threadIdx.x / kLanes * a.nrows / kSample;
+    const double* xr = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride;
+    double v[(KM + kLanes - 1) / kLanes];
+#pragma unroll
+    for (int k = 0; k < KM; k += kLanes) v[k / kLanes] = k0 + k < K ? __ldg(xr + k0 + k) : 0.0;
+    // (and the thread's own first row on its way)
+    const long long r0 = (long long)blockIdx.x * kXT + threadIdx.x;
+    if (r0 < a.nrows) {
+      const double* x0 = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r0) : r0) * a.kstride;
+#pragma unroll
+      for (int k = 0; k < KM; k += 16)
+        if (k < K) asm volatile("prefetch.global.L1 [%0];" ::"l"(x0 + k));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(x0 + K - 1));
     }
+    for (int t = threadIdx.x; t < P * K; t += kXT) see(a.y[t]);
+#pragma unroll
+    for (int k = 0; k < KM; k += kLanes) see(v[k / kLanes]);
     e = __reduce_max_sync(0xffffffffu, e);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_exp, e);
   }
