@@ -145,8 +145,7 @@ __device__ __forceinline__ double order_value(long long k) {
 // blocks than that are read again), and the maxima compare as integers, FP64
 // compares being 16 cycles an instruction and SM.
 __global__ void __launch_bounds__(256)
-stat_finalize_kernel(const double* __restrict__ bpart, int nblocks, StatSpec spec,
-                     double* __restrict__ out, const StatCapture cap) {
+stat_finalize_kernel(const double* bpart, int nblocks, StatSpec spec, double* out, const StatCapture cap) {
   __shared__ long long sm[8];
   __shared__ double ss[8];
   const int o = blockIdx.x, p = o - cap.first;
@@ -379,8 +378,7 @@ init_vertex_kernel(const InitArgs<T> a) {
   block_partials_out(s_red, kWarps, spec, a.bpart, gridDim.x, blockIdx.x);
 }
 
-__global__ void mu_output_kernel(double* __restrict__ mu, const double* __restrict__ S,
-                                 long long n, int Pn) {
+__global__ void mu_output_kernel(double* mu, const double* S, long long n, int Pn) {
   dep_launch();
   dep_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;

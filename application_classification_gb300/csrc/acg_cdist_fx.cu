@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
 // LSE(-d) as block partials.  Thread t takes column t % P of rows t / P,
 // t / P + 256 / P, ... of the block's contiguous rows.
 __global__ void __launch_bounds__(kXT)
-cdist_stats_kernel(const double* __restrict__ d, long long nrows, int P, int stride, double* __restrict__ part) {
+cdist_stats_kernel(const double* d, long long nrows, int P, int stride, double* part) {
   dep_launch();
   dep_wait();
   __shared__ FxLse s_p[kXT], s_n[kXT];
@@ -156,7 +156,7 @@ cdist_stats_kernel(const double* __restrict__ d, long long nrows, int P, int str
   double mn = CUDART_INF;
   if (rl < rs) {
     for (long long r = r0 + rl; r < r1; r += rs) {
-      const double x = __ldg(d + (size_t)r * stride + c);
+      const double x = d[(size_t)r * stride + c];
       mn = fmin(mn, x);
       fx_add(lp, x);
       fx_add(ln, -x);

@@ -34,8 +34,12 @@ namespace acg {
 // one before has completed and its writes are visible) it touches only what no
 // kernel of a match writes.  dep_launch() lets the next such kernel start early.
 // An iteration of a small graph is four to five kernels of about 8 us, so the
-// gaps between them and their prologues count (1,000 vertices: FP64 571 -> 451 us a
-// match, mixed 480 -> 406).
+// gaps between them and their prologues count (1,000 vertices: FP64 571 -> 457 us a
+// match, mixed 480 -> 413).
+// Such a kernel lives while its predecessors still write, so it reads what they
+// write by ordinary loads (or ld_cs, or cp.async), which stay behind dep_wait():
+// __ldg and const __restrict__ parameters are for memory that nobody writes in the
+// kernel's life, and the compiler may move those loads ahead of the wait.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... KA, typename... A>
@@ -52,6 +56,29 @@ cudaError_t launch_kernel(bool early, void (*kernel)(KA...), int blocks, int thr
   c.attrs = at;
   c.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, KA(args)...);
+}
+
+// Streaming loads (evicted first), not moved across dep_wait().
+__device__ __forceinline__ float ld_cs(const float* p) {
+  float x;
+  asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(x) : "l"(p));
+  return x;
+}
+__device__ __forceinline__ double ld_cs(const double* p) {
+  double x;
+  asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(x) : "l"(p));
+  return x;
+}
+__device__ __forceinline__ float4 ld_cs(const float4* p) {
+  float4 x;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "l"(p));
+  return x;
+}
+__device__ __forceinline__ double2 ld_cs(const double2* p) {
+  double2 x;
+  asm volatile("ld.global.cs.v2.f64 {%0, %1}, [%2];" : "=d"(x.x), "=d"(x.y) : "l"(p));
+  return x;
 }
 
 constexpr int kNumSMs = 152;  // GB300: 2 dies x 76 SMs

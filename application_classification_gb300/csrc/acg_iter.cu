@@ -250,8 +250,8 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
       for (int k = 0; k < NQV; ++k) {
         const int qv = qc + NPOW * k;
         if (ok && qv * W < Pp) {
-          x[u][k] = __ldg(reinterpret_cast<const VT*>(a.vr_in + (size_t)sidx[u] * Pp) + qv);
-          y[u][k] = __ldcs(reinterpret_cast<const VT*>(a.dE + (size_t)e * Pp) + qv);
+          x[u][k] = reinterpret_cast<const VT*>(a.vr_in + (size_t)sidx[u] * Pp)[qv];
+          y[u][k] = ld_cs(reinterpret_cast<const VT*>(a.dE + (size_t)e * Pp) + qv);
         } else {
           x[u][k] = vfill<T>(kLazy ? T(-0x1p127) : neg_inf<T>());
           y[u][k] = vfill<T>(T(kLazy ? 1 : 0));
@@ -446,9 +446,8 @@ __device__ __forceinline__ T max_of(T a, T b) {
 constexpr int kHeavyCols = 256;  // columns of a row at most
 template <typename T>
 __global__ void __launch_bounds__(256)
-heavy_combine_kernel(const T* __restrict__ partial, const int* __restrict__ hbase,
-                     const int* __restrict__ hcount, const int* __restrict__ hvert, int Pp,
-                     T* __restrict__ M) {
+heavy_combine_kernel(const T* partial, const int* __restrict__ hbase,
+                     const int* __restrict__ hcount, const int* __restrict__ hvert, int Pp, T* M) {
   __shared__ T part[8][kHeavyCols];
   dep_launch();
   dep_wait();

@@ -238,7 +238,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
         for (int k = 0; k < NQV; ++k) {
           const int qv = qc + NPOW * k;
           x[u][k] = (okv[u] && qv * W < Pp)
-                        ? __ldg(reinterpret_cast<const VT*>(a.dE + (size_t)ridx[u] * Pp) + qv)
+                        ? reinterpret_cast<const VT*>(a.dE + (size_t)ridx[u] * Pp)[qv]
                         : sfill<T>(pos_inf<T>());
         }
       }
@@ -340,7 +340,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
           for (int k = 0; k < NQV; ++k) {
             const int qv = qc + NPOW * k;
             if (qv * W >= Pp) continue;
-            const VT xv = __ldg(reinterpret_cast<const VT*>(row) + qv);
+            const VT xv = reinterpret_cast<const VT*>(row)[qv];
 #pragma unroll
             for (int w = 0; w < W; ++w)
               kahan_add(sm[k * W + w], sc[k * W + w], exp_fast(mn[k * W + w] - sg<T>(xv, w)));
@@ -540,7 +540,7 @@ dst_quirk_kernel(const DstQuirkArgs<T> a) {
         for (int k = 0; k < NQV; ++k) {
           const int qv = qc + NPOW * k;
           x[u][k] = (ok && qv * W < Pqc)
-                        ? __ldcs(reinterpret_cast<const VT*>(a.dE + (size_t)e * (a.dstride ? a.dstride : Pp)) + qv)
+                        ? ld_cs(reinterpret_cast<const VT*>(a.dE + (size_t)e * (a.dstride ? a.dstride : Pp)) + qv)
                         : sfill<T>(pos_inf<T>());
         }
       }
@@ -695,15 +695,15 @@ init_warp_kernel(const InitArgs<T> a) {
     for (int k = 0; k < QPL; ++k) {
       const int q = qo + k;
       const bool on = q < Pp;
-      r.b[k] = on ? __ldcs(a.B + (size_t)v * Pp + q) : T(0);
-      r.em[k] = on ? __ldcs(a.dEmin + (size_t)v * Pp + q) : T(0);
-      r.rq[k] = q < qcov ? __ldcs(a.Rq + (size_t)v * Pqc + q) : T(0);
-      r.fq[k] = q < qcov ? __ldcs(a.Fq + (size_t)v * Pqc + q) : T(0);
+      r.b[k] = on ? ld_cs(a.B + (size_t)v * Pp + q) : T(0);
+      r.em[k] = on ? ld_cs(a.dEmin + (size_t)v * Pp + q) : T(0);
+      r.rq[k] = q < qcov ? ld_cs(a.Rq + (size_t)v * Pqc + q) : T(0);
+      r.fq[k] = q < qcov ? ld_cs(a.Fq + (size_t)v * Pqc + q) : T(0);
     }
 #pragma unroll
     for (int j = 0; j < PPL; ++j) {
       const int p = lane + 32 * j;
-      r.cv[j] = p < Pn ? __ldcs(a.CV + (size_t)v * Pnp + p) : T(0);
+      r.cv[j] = p < Pn ? ld_cs(a.CV + (size_t)v * Pnp + p) : T(0);
     }
   };
 
