@@ -108,7 +108,7 @@ constexpr uint32_t kFxLimit = 0x40d00000u;
 // n = 64 x / ln 2 rounded; f in (0.99, 2.02) 2^61.
 ACG_FX_HD uint64_t fx_exp_core(uint64_t X, int n, int& k) {
   // r = x - n ln2 / 64: 92 fraction bits of ln2 / 64
-  const int64_t r = (int64_t)(X - (uint64_t)((int64_t)n * (int64_t)0x2c5c85fdf473dell)) -
+  const int64_t r = (int64_t)(X - (uint64_t)(int64_t)n * 0x2c5c85fdf473deull) -
                     (((int64_t)n * (int64_t)0x6af278edll) >> 32);
   const uint64_t T = fx_exp_entry(n & 63);
   k = n >> 6;
@@ -130,7 +130,7 @@ ACG_FX_HD uint64_t fx_exp_core(uint64_t X, int n, int& k) {
   const uint32_t Th = (uint32_t)(T >> 32), Tl = (uint32_t)T;
   const int64_t a = (int64_t)(int32_t)Th * ph;
   const int64_t b = (int64_t)((uint64_t)Th * pl) + (int64_t)Tl * ph;
-  return T + (uint64_t)(a << 4) + (uint64_t)(b >> 28);
+  return T + ((uint64_t)a << 4) + (uint64_t)(b >> 28);
 }
 
 // exp(x) for a double, |x| < 2^14.
@@ -175,7 +175,7 @@ ACG_FX_HD uint64_t fx_table_entry(int j) {
 }
 // n = 1024 x / ln 2 rounded
 ACG_FX_HD uint64_t fx_exp_tab(uint64_t X, int n, const uint64_t* tab, int& k) {
-  const int64_t r = (int64_t)(X - (uint64_t)((int64_t)n * (int64_t)0x2c5c85fdf473dll)) -
+  const int64_t r = (int64_t)(X - (uint64_t)(int64_t)n * 0x2c5c85fdf473dull) -
                     (((int64_t)n * (int64_t)0x735793c7ll) >> 31);
   const uint64_t T = tab[n & (kFxTable - 1)];
   k = n >> 10;
@@ -188,7 +188,7 @@ ACG_FX_HD uint64_t fx_exp_tab(uint64_t X, int n, const uint64_t* tab, int& k) {
   const uint32_t Th = (uint32_t)(T >> 32), Tl = (uint32_t)T;
   const int64_t a = (int64_t)(int32_t)Th * ph;
   const int64_t b = (int64_t)((uint64_t)Th * pl) + (int64_t)Tl * ph;
-  return T + (uint64_t)(a << 4) + (uint64_t)(b >> 28);
+  return T + ((uint64_t)a << 4) + (uint64_t)(b >> 28);
 }
 
 // exp(x) for x = X / 2^Q, 47 <= Q <= 54 and |x| < 2^14.
@@ -555,7 +555,7 @@ ACG_FX_HD double fx_root(uint64_t sh, int64_t sc, uint64_t sl, int a) {
   const uint32_t r0 = fx_f2u(nf * y * 65536.f);
   const int64_t e0 = (int64_t)(n - (uint64_t)r0 * r0);
   const int32_t d0 = fx_f2i((float)(int32_t)(e0 >> 14) * y * 32768.f);
-  const uint64_t r1 = ((uint64_t)r0 << 32) + (uint64_t)((int64_t)d0 << 14);
+  const uint64_t r1 = ((uint64_t)r0 << 32) + ((uint64_t)(int64_t)d0 << 14);
   const uint32_t h1 = (uint32_t)(r1 >> 32), l1 = (uint32_t)r1;
   const int32_t e1 = (int32_t)(n - (uint64_t)h1 * h1 - (((uint64_t)h1 * l1) >> 31));
   const uint64_t r = r1 + (uint64_t)(int64_t)fx_f2i((float)e1 * y * 32768.f);
