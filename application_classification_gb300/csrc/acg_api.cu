@@ -435,7 +435,7 @@ vertex_phase:
   va.lse_pos = P->gv + Pn;
   va.wide = P->edge_wide;
   va.early = early;
-  const bool wide = sizeof(T) == 4 && Pp > 64;
+  const bool wide = sizeof(T) == 4 && Pp > 64 && P->vsched;
   if constexpr (sizeof(T) == 4) va.rowpart = (float*)P->rowpart;
   if (beside && t > 1) ACG_CUDA_TRY(cudaStreamWaitEvent(s, P->ev_stats, 0));
   if constexpr (std::is_same_v<T, double>) ACG_TRY(launch_vertex_fx(va, P->vert_blocks, s));

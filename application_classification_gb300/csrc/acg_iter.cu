@@ -21,7 +21,8 @@
 //   contiguous vertex range, rows staged per warp with cp.async; see its own
 //   comment.  FP32 patterns of more than 64 edge columns take acg_vertex_wide.cu's
 //   kernel, FP64 ones acg_vertex_fx.cu's; the block-tile form below is left with
-//   FP32 patterns of up to 64 edge columns and more than 64 vertices.
+//   FP32 patterns of up to 64 edge columns and more than 64 vertices, and with wide
+//   ones around a hub (kWideTerms).
 //
 // Phase B, vertex_update_kernel -- everything per vertex, streamed with
 //   coalesced 16-byte accesses: FMax, RMax, MU_raw (compensated sum), the next
@@ -1369,7 +1370,7 @@ bool warp_form(int pn, int pp, F&& f) {
 
 template <typename T>
 acg_status launch_vertex_update(const VertexUpdArgs<T>& a, int blocks, cudaStream_t s) {
-  if (a.Pp > 64) return launch_vertex_wide(a, blocks, s);
+  if (a.Pp > 64 && a.vsched) return launch_vertex_wide(a, blocks, s);
   cudaError_t le = cudaSuccess;
   if (a.vsched == nullptr && a.Pn > 0 && a.Pn <= 64 && a.Pp <= 64)
     return set_error(ACG_ERR_INVALID_ARGUMENT, "vertex phase: no schedule for the warp form");

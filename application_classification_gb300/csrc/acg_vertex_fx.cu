@@ -44,34 +44,8 @@ namespace acg {
 namespace {
 
 constexpr int kFT = 256;     // threads per block
-constexpr int kFxVps = 2;    // vertices per stage
-constexpr int kFW = kFT / 32;
-
-__host__ __device__ inline size_t f16(size_t b) { return (b + 15) & ~size_t(15); }
-
-struct FxSmem {
-  size_t pat, sched, tab, cst, mxd, amp, flags, ring, mu, total, stage, group_ring, mu_n;
-  int mu_row;
-  __host__ __device__ FxSmem(int Pn, int Pe, int Pp, int Pnp, int nterms, int nw) {
-    const int ng = kFW / nw;  // groups
-    size_t o = 0;
-    pat = o; o += f16(sizeof(int) * (size_t)(4 * Pe + 2 * (Pn + 1)));
-    sched = o; o += f16(sizeof(uint32_t) * (size_t)nterms * 32 * nw);
-    tab = o; o += sizeof(uint64_t) * kFxTable;            // 2^(j / 1024)
-    cst = o; o += f16(sizeof(double) * (size_t)6 * Pp);   // fF fR dF dR cF cR
-    mxd = o; o += f16(sizeof(double) * (size_t)2 * Pp * ng);  // maxima of FP64 stages
-    amp = o; o += f16(sizeof(float) * (size_t)2 * Pp);    // |F|, |R| bounds
-    flags = o; o += 16;
-    stage = sizeof(double) * (size_t)VwStage(Pp, Pnp, false, kFxVps).n;
-    group_ring = 2 * stage;
-    const size_t red = sizeof(uint32_t) * (size_t)ng * (4 * Pe + 4 * (2 * Pe + Pn));  // aliases the rings
-    ring = o; o += f16(std::max(red, ng * group_ring));
-    mu_row = (Pn + 31) / 32 * 32 + 1;
-    mu_n = (size_t)kFxVps * mu_row;
-    mu = o; o += f16(sizeof(double) * ng * mu_n);
-    total = o;
-  }
-};
+constexpr int kFW = kFxWarps;
+static_assert(kFT == 32 * kFxWarps && kFxTableBytes == (int)sizeof(uint64_t) * kFxTable);
 
 __device__ __forceinline__ void fcp16(void* sdst, const void* gsrc) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
@@ -327,12 +301,13 @@ __device__ __forceinline__ bool run_stage(const A ar, const StageCtx& x, const t
   return false;
 }
 
-template <int QPL, int PPL, int NW>
+// GS: the schedule stays in global memory (acg_vschedule.h).
+template <int QPL, int PPL, int NW, bool GS>
 __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<double> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int Pe = a.Pe, Pn = a.Pn, Pp = a.Pp, Pnp = a.Pnp, Dn = a.Dn, nterms = a.vterms;
   constexpr int kNG = kFW / NW;
-  const FxSmem L(Pn, Pe, Pp, Pnp, nterms, NW);
+  const FxSmem L(Pn, Pe, Pp, Pnp, nterms, NW, GS);
   const VwStage G(Pp, Pnp, false, kFxVps);
   const int tid = threadIdx.x;
   int* s_pat = reinterpret_cast<int*>(smem + L.pat);
@@ -342,7 +317,8 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
   float* s_amp = reinterpret_cast<float*>(smem + L.amp);
   int* s_bound = reinterpret_cast<int*>(smem + L.flags);  // float bits: [0] columns, [1] MU_raw
   for (int t = tid; t < 4 * Pe + 2 * (Pn + 1); t += kFT) s_pat[t] = a.pat[t];
-  for (int t = tid; t < nterms * 32 * NW; t += kFT) s_sched[t] = a.vsched[t];
+  if constexpr (!GS)
+    for (int t = tid; t < nterms * 32 * NW; t += kFT) s_sched[t] = a.vsched[t];
   for (int t = tid; t < 2 * Pp * kNG; t += kFT) s_mxd[t] = -CUDART_INF;
   for (int t = tid; t < kFxTable; t += kFT) reinterpret_cast<uint64_t*>(smem + L.tab)[t] = fx_table_entry(t);
   if (tid < 2) s_bound[tid] = 0;
@@ -502,7 +478,7 @@ __global__ void __launch_bounds__(kFT, 2) vertex_fx_kernel(const VertexUpdArgs<d
       *reinterpret_cast<uint4*>(st + G.oC * 8 + c * 16) =
           *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(a.CV) + (size_t)v0 * crow + c * 16);
   };
-  StageCtx x{&a, nullptr, reinterpret_cast<double*>(smem + L.mu) + (size_t)group * L.mu_n, s_sched,
+  StageCtx x{&a, nullptr, reinterpret_cast<double*>(smem + L.mu) + (size_t)group * L.mu_n, GS ? a.vsched : s_sched,
              s_mxd + (size_t)group * 2 * Pp, gl, group, 0, 0, L.mu_row};
   int buf = 0;
   for (int v0 = vb; v0 < ve; v0 += kFxVps, buf ^= 1) {
@@ -605,17 +581,29 @@ int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vec
   return vertex_warp_schedule(pat, pn, pe, pp, pnp, kFxVps, out, 32 * vertex_fx_warps(pn, pp), 2, 8);
 }
 
+// f(kernel, shared memory) of the kernel for a pattern.
+template <typename F>
+static void fx_kernel(int pn, int pe, int pp, int pnp, int nterms, F&& f) {
+  fx_form(pn, pp, [&]<int QPL, int PPL, int NW>() {
+    const size_t sm = FxSmem(pn, pe, pp, pnp, nterms, NW, false).total;
+    if constexpr (NW == 4)  // (fewer warps' schedules fit, of every pattern)
+      if (sm > kBlockSmem) {
+        f(vertex_fx_kernel<QPL, PPL, NW, true>, FxSmem(pn, pe, pp, pnp, nterms, NW, true).total);
+        return;
+      }
+    f(vertex_fx_kernel<QPL, PPL, NW, false>, sm);
+  });
+}
+
 acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s) {
   if (a.vsched == nullptr)
     return set_error(ACG_ERR_INVALID_ARGUMENT, "vertex phase: no schedule of the sums");
   cudaError_t le = cudaSuccess;
-  fx_form(a.Pn, a.Pp, [&]<int QPL, int PPL, int NW>() {
-    const size_t sm = FxSmem(a.Pn, a.Pe, a.Pp, a.Pnp, a.vterms, NW).total;
+  fx_kernel(a.Pn, a.Pe, a.Pp, a.Pnp, a.vterms, [&](auto kernel, size_t sm) {
     if (sm > 48 * 1024)
-      le = cudaFuncSetAttribute(vertex_fx_kernel<QPL, PPL, NW>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      le = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (le != cudaSuccess) return;
-    le = launch_kernel(a.early, vertex_fx_kernel<QPL, PPL, NW>, blocks, kFT, sm, s, a);
+    le = launch_kernel(a.early, kernel, blocks, kFT, sm, s, a);
   });
   if (le != cudaSuccess)
     return set_error(ACG_ERR_CUDA, "vertex_fx_kernel launch: %s", cudaGetErrorString(le));
@@ -624,14 +612,10 @@ acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStre
 
 int vertex_fx_blocks(int pn, int pe, int pp, int pnp, int nterms, int num_sms, int dn) {
   int nb = 0;
-  fx_form(pn, pp, [&]<int QPL, int PPL, int NW>() {
-    const size_t sm = FxSmem(pn, pe, pp, pnp, nterms, NW).total;
+  fx_kernel(pn, pe, pp, pnp, nterms, [&](auto kernel, size_t sm) {
     if (sm > 48 * 1024)
-      cudaFuncSetAttribute(vertex_fx_kernel<QPL, PPL, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sm);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, vertex_fx_kernel<QPL, PPL, NW>, kFT, sm) !=
-        cudaSuccess)
-      nb = 1;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, kFT, sm) != cudaSuccess) nb = 1;
   });
   // (a stage per group at least: fewer partials to finalise on small graphs)
   const int per = kFxVps * kFW / vertex_fx_warps(pn, pp);

@@ -35,27 +35,14 @@ namespace acg {
 namespace {
 
 constexpr int kTileThreads = 256;  // the tile form's block, which fixes V
-constexpr int kWv = 2;             // vertices (tiles) per stage
-
-__host__ __device__ inline size_t w16(size_t b) { return (b + 15) & ~size_t(15); }
-
-struct WideSmem {
-  size_t pat, sched, cst, ring, mu, total, stage, row_ring, mu_n;
-  int mu_row;
-  __host__ __device__ WideSmem(int V, int Pn, int Pe, int Pp, int Pnp, int nterms, int nw) {
-    size_t o = 0;
-    pat = o; o += w16(sizeof(int) * (size_t)(2 * Pe));
-    sched = o; o += w16(sizeof(uint32_t) * (size_t)nterms * 32 * nw);
-    cst = o; o += w16(sizeof(float) * (size_t)10 * Pp);
-    stage = sizeof(float) * (size_t)VwStage(Pp, Pnp, true, kWv).n;
-    row_ring = 2 * stage;
-    ring = o; o += w16(V * row_ring);
-    mu_row = (Pn + 31) / 32 * 32 + 1;  // (the schedule's slots)
-    mu_n = (size_t)kWv * mu_row;
-    mu = o; o += w16(sizeof(float) * 2 * 2 * V * mu_n);  // two stages: hi, lo of each row
-    total = o;
-  }
-};
+// Terms a lane above which a pattern whose rows take two warps is left to the
+// block-tile form: a hub's sum is one lane's, in each row, while the tile form's
+// threads share out the rows.  100,000 vertices, ten iterations, tile form / this one:
+// 136 edges, longest sum 86 and 110 terms 7.13 / 7.00 and 7.42 / 7.66 ms; 170, 105 and
+// 138: 8.46 / 8.43 and 9.07 / 9.35; 254, 79 and 155: 9.07 / 8.70 and 10.91 / 11.03; a
+// star of 254: 12.95 / 14.03.  Rows of one warp gain for every hub (a star of 128
+// edges 6.40 / 5.45).
+constexpr int kWideTerms = 104;
 
 __device__ __forceinline__ void wcp16(void* sdst, const void* gsrc) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
@@ -405,7 +392,10 @@ acg_status launch_wide(const VertexUpdArgs<float>& a, int V, int blocks, cudaStr
 }  // namespace
 
 int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out) {
-  return vertex_warp_schedule(pat, pn, pe, pp, pnp, kWv, out, 32 * wide_warps(pp), 4);
+  const int nt = vertex_warp_schedule(pat, pn, pe, pp, pnp, kWv, out, 32 * wide_warps(pp), 4);
+  if (wide_warps(pp) == 1 || nt <= kWideTerms) return nt;
+  out->clear();
+  return 0;
 }
 
 size_t wide_rowpart_floats(int pp, int blocks) {

@@ -13,6 +13,7 @@
 #pragma once
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <vector>
 
@@ -152,5 +153,62 @@ inline int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp,
   }
   return nt;
 }
+
+// ---- shared memory of the kernels that share a stage between warps
+constexpr size_t kBlockSmem = 227 * 1024;  // sm_103a, dynamic
+ACG_VS_HD inline size_t vs16(size_t b) { return (b + 15) & ~size_t(15); }
+
+// vertex_fx_kernel (acg_vertex_fx.cu): groups of nw warps share a stage.
+constexpr int kFxVps = 2;           // vertices per stage
+constexpr int kFxWarps = 8;         // of a block
+constexpr int kFxTableBytes = 8192; // 2^(j / 1024)
+// A lane's terms are as many as its longest job's, 1 + twice the pattern's edges for
+// a vertex that all of them leave and enter: of such hubs the schedule of a group of
+// four warps is up to 264 KB.  Where it does not fit a block's memory beside the rest
+// it stays in global memory (in_global).
+struct FxSmem {
+  size_t pat, sched, tab, cst, mxd, amp, flags, ring, mu, total, stage, group_ring, mu_n;
+  int mu_row;
+  ACG_VS_HD FxSmem(int Pn, int Pe, int Pp, int Pnp, int nterms, int nw, bool in_global) {
+    const int ng = kFxWarps / nw;  // groups
+    size_t o = 0;
+    pat = o; o += vs16(sizeof(int) * (size_t)(4 * Pe + 2 * (Pn + 1)));
+    sched = o; o += in_global ? 0 : vs16(sizeof(uint32_t) * (size_t)nterms * 32 * nw);
+    tab = o; o += kFxTableBytes;
+    cst = o; o += vs16(sizeof(double) * (size_t)6 * Pp);   // fF fR dF dR cF cR
+    mxd = o; o += vs16(sizeof(double) * (size_t)2 * Pp * ng);  // maxima of FP64 stages
+    amp = o; o += vs16(sizeof(float) * (size_t)2 * Pp);    // |F|, |R| bounds
+    flags = o; o += 16;
+    stage = sizeof(double) * (size_t)VwStage(Pp, Pnp, false, kFxVps).n;
+    group_ring = 2 * stage;
+    const size_t red = sizeof(uint32_t) * (size_t)ng * (4 * Pe + 4 * (2 * Pe + Pn));  // aliases the rings
+    ring = o; o += vs16(red > ng * group_ring ? red : ng * group_ring);
+    mu_row = (Pn + 31) / 32 * 32 + 1;
+    mu_n = (size_t)kFxVps * mu_row;
+    mu = o; o += vs16(sizeof(double) * ng * mu_n);
+    total = o;
+  }
+};
+
+// vertex_wide_kernel (acg_vertex_wide.cu): V rows of nw warps; schedules of more
+// than kWideTerms terms a lane are not made.
+constexpr int kWv = 2;  // vertices (tiles) per stage
+struct WideSmem {
+  size_t pat, sched, cst, ring, mu, total, stage, row_ring, mu_n;
+  int mu_row;
+  ACG_VS_HD WideSmem(int V, int Pn, int Pe, int Pp, int Pnp, int nterms, int nw) {
+    size_t o = 0;
+    pat = o; o += vs16(sizeof(int) * (size_t)(2 * Pe));
+    sched = o; o += vs16(sizeof(uint32_t) * (size_t)nterms * 32 * nw);
+    cst = o; o += vs16(sizeof(float) * (size_t)10 * Pp);
+    stage = sizeof(float) * (size_t)VwStage(Pp, Pnp, true, kWv).n;
+    row_ring = 2 * stage;
+    ring = o; o += vs16(V * row_ring);
+    mu_row = (Pn + 31) / 32 * 32 + 1;  // (the schedule's slots)
+    mu_n = (size_t)kWv * mu_row;
+    mu = o; o += vs16(sizeof(float) * 2 * 2 * V * mu_n);  // two stages: hi, lo of each row
+    total = o;
+  }
+};
 
 }  // namespace acg
