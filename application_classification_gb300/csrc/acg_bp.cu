@@ -257,8 +257,10 @@ __global__ void inverse_perm_kernel(const int* __restrict__ perm, long long n, i
 // CV = dV - LSE_v(dV), MU0 = -dV - LSE_v(-dV) (main.cu:112,116-117);
 // RMax0/FMax0 from the quirk buffer maxima (main.cu:113-114,119-120,135-146);
 // then VF, VR of the first iteration (main.cu:165-176) and their statistics.
+// (the widest FP64 form: the rare calls of its log-sum-exps would take it past the 128
+// registers of two blocks per SM: 204,307 vertices, 200 columns 1.9 -> 3.1 ms)
 template <typename T, int G, int NQV>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 8 && NQV == 4 ? 2 : 0)
 init_vertex_kernel(const InitArgs<T> a) {
   constexpr int W = Vec<T>::W;
   constexpr int NQ = NQV * W;

@@ -328,46 +328,23 @@ ACG_FX_HD void fx_add_term(FxLse& a, int k, uint64_t f) {
 #endif
 }
 
-// Value x outside fx_add's range (|x| >= 2^14), or a state already wide.  Up to
-// 2^24 the integer form holds it, n rounded from FP64 (the series' argument is
-// formed modulo 2^64 as before).  A term more than e^-100 below the sum adds
-// nothing, and a wide sum more than that below x is dropped for x: so one vertex
-// far from everything leaves the state in integer form, or returns it there with
-// the next ordinary value.
+// x beyond +-2^24, or a wide state that x does not replace.  Values further apart
+// than e^100 (nearly all, at this scale) need no exponential.
 constexpr double kFxFar = 100.0;
-ACG_FX_SLOW FxLse fx_add_far(FxLse a, double x) {
+ACG_FX_SLOW FxLse fx_add_wide(FxLse a, double x) {
   if (!(x > fx_double(0xfff0000000000000ull))) return a;  // NaN, -inf: nothing
-  const uint64_t b = fx_bits(x);
-  const uint32_t t = (uint32_t)(b >> 32) & 0x7fffffffu;
-  const bool fits = t < 0x41700000u;
   double m, s;
   fx_pair(a, m, s);
-  if (fits && fx_wide(a) && x - m > kFxFar) fx_init(a);  // (s below 2^33)
-  if (!fx_wide(a)) {
-    if (fits) {
-      int k;
-      uint64_t f;
-      if (t < kFxLimit) {
-        f = fx_exp(b, k);
-      } else {
-#ifdef __CUDA_ARCH__
-        const int n = __double2int_rn(x * 92.332482616893656877);
-#else
-        const int n = (int)std::lrint(x * 92.332482616893656877);
-#endif
-        const uint64_t X = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << ((int)(t >> 20) - 1015);
-        f = fx_exp_core((b >> 63) ? 0ull - X : X, n, k);
-      }
-      fx_add_term(a, k, f);
-      return a;
-    }
-    if (s > 0.0 && m - x > kFxFar) return a;
-  }
-  if (x > m) {
-    s = s > 0.0 ? s * exp(m - x) + 1.0 : 1.0;
+  const double d = x - m;
+  if (s > 0.0 && d < -kFxFar) return a;
+  if (!(s > 0.0) || d > kFxFar) {
+    m = x;
+    s = 1.0;
+  } else if (d > 0.0) {
+    s = s * exp(-d) + 1.0;
     m = x;
   } else {
-    s += exp(x - m);
+    s += exp(d);
   }
   const uint64_t mb = fx_bits(m), sb = fx_bits(-s);
   a.w[0] = (uint32_t)mb;
@@ -375,6 +352,36 @@ ACG_FX_SLOW FxLse fx_add_far(FxLse a, double x) {
   a.w[2] = (uint32_t)sb;
   a.w[3] = (uint32_t)(sb >> 32) | 0x80000000u;
   return a;
+}
+
+// Value x outside fx_add's range (|x| >= 2^14), or a state already wide.  Up to
+// 2^24 the integer form holds it, n rounded from FP64 (the series' argument is
+// formed modulo 2^64 as before).  A term more than e^-100 below the sum adds
+// nothing, and a wide sum more than that below x is dropped for x: so one vertex
+// far from everything leaves the state in integer form, or returns it there with
+// the next ordinary value.
+ACG_FX_SLOW FxLse fx_add_far(FxLse a, double x) {
+  const uint64_t b = fx_bits(x);
+  const uint32_t t = (uint32_t)(b >> 32) & 0x7fffffffu;
+  if (t < 0x41700000u) {
+    if (fx_wide(a) && x - fx_double(((uint64_t)a.w[1] << 32) | a.w[0]) > kFxFar)
+      fx_init(a);  // (its scaled sum is below 2^33)
+    if (!fx_wide(a)) {
+#ifdef __CUDA_ARCH__
+      const int n = __double2int_rn(x * 92.332482616893656877);
+#else
+      const int n = (int)std::lrint(x * 92.332482616893656877);
+#endif
+      const uint64_t m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+      const int c = (int)(t >> 20) - 1015;
+      const uint64_t X = c >= 0 ? m << c : (c > -53 ? m >> -c : 0ull);
+      int k;
+      const uint64_t f = fx_exp_core((b >> 63) ? 0ull - X : X, n, k);
+      fx_add_term(a, k, f);
+      return a;
+    }
+  }
+  return fx_add_wide(a, x);
 }
 
 ACG_FX_HD void fx_add(FxLse& a, double x) {
