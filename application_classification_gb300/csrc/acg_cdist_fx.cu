@@ -44,10 +44,39 @@ __device__ __noinline__ double pair_fp64(const double* __restrict__ x, const dou
   return sqrt(s);
 }
 
+// One feature: |x - y|, where squaring it neither overflows nor underflows the root
+// of its square.
+__device__ __forceinline__ double pair_one(double x, double y) {
+  const double t = x - y, u = fabs(t);
+  const uint32_t e = (uint32_t)__double2hiint(u) >> 20;
+  return e > 1023 - 500 && e < 1023 + 500 ? u : sqrt(t * t);
+}
+__device__ void rows_one(const CdistRbArgs<double, double>& a) {
+  for (long long r = (long long)blockIdx.x * kXT + threadIdx.x; r < a.nrows;
+       r += (long long)gridDim.x * kXT) {
+    const double x = __ldg(a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride);
+    double* orow = a.out + (size_t)r * a.ostride;
+    for (int q0 = 0; q0 < a.Pp; q0 += 2) {
+      double d[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        d[j] = q0 + j < a.P ? pair_one(x, __ldg(a.y + q0 + j)) : 0.0;
+        if (a.wide && q0 + j < a.P) d[j] = edge_word(d[j], a.wide);
+      }
+      *reinterpret_cast<double2*>(orow + q0) = make_double2(d[0], d[1]);
+    }
+  }
+}
+
 template <int KM>
 __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double, double> a) {
   dep_launch();
   dep_wait();
+  if constexpr (KM == 2)
+    if (a.K == 1) {
+      rows_one(a);
+      return;
+    }
   extern __shared__ __align__(16) unsigned char smem[];
   FxPart* s_y = reinterpret_cast<FxPart*>(smem);  // [Pp][KM], zero past P and K
   __shared__ int s_exp, s_bad;
@@ -103,7 +132,7 @@ __global__ void __launch_bounds__(kXT) cdist_fx_kernel(const CdistRbArgs<double,
        r += (long long)gridDim.x * kXT) {
     const double* xr = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride;
     FxPart x[KM];
-    bool big = ybad || K == 1;
+    bool big = ybad;
 #pragma unroll
     for (int k = 0; k < KM; ++k) {
       x[k] = FxPart{0, 0};
