@@ -894,7 +894,7 @@ acg_status plan_create_impl(acg_data* D, PatternSpec&& spec, const acg_options& 
     P->maxdeg = md;
     std::vector<uint32_t> vs;
     P->vterms = eb == 8 ? vertex_fx_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, &vs)
-                : Pp > 64 ? vertex_wide_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, &vs)
+                : Pp > 64 ? vertex_wide_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, Dn, &vs)
                           : vertex_warp_schedule(spec.pat.data(), Pn, Pe, Pp, P->Pnp, &vs);
     if (P->vterms > 0) {
       st = dev_alloc(&P->owned, sizeof(uint32_t) * vs.size(), (void**)&P->vsched, s);

@@ -22,7 +22,7 @@
 //   comment.  FP32 patterns of more than 64 edge columns take acg_vertex_wide.cu's
 //   kernel, FP64 ones acg_vertex_fx.cu's; the block-tile form below is left with
 //   FP32 patterns of up to 64 edge columns and more than 64 vertices, and with wide
-//   ones around a hub (kWideTerms).
+//   ones around a hub or of few vertices (vertex_wide_schedule).
 //
 // Phase B, vertex_update_kernel -- everything per vertex, streamed with
 //   coalesced 16-byte accesses: FMax, RMax, MU_raw (compensated sum), the next

@@ -102,16 +102,16 @@ struct VertexUpdArgs {
 // sums in order.  Returns the terms per lane, 0 when the pattern takes the
 // tile form.
 int vertex_warp_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
-// The vertex phase of FP64 plans (acg_vertex_fx.cu), every pattern size: its
-// schedule (nonzero for every pattern), launch and grid.
 // The vertex phase of FP32 plans with more than 64 padded edge columns
-// (acg_vertex_wide.cu): its schedule and launch; blocks as vertex_update_blocks
-// gives them.
-int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
+// (acg_vertex_wide.cu): its schedule (0: the block-tile form is the faster one) and
+// launch; blocks as vertex_update_blocks gives them.
+int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, int dn, std::vector<uint32_t>* out);
 acg_status launch_vertex_wide(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s);
 size_t wide_rowpart_floats(int pp, int blocks);
 // The block partials (bpart) of a wide launch from its rows' statistics.
 acg_status launch_wide_partials(const VertexUpdArgs<float>& a, int blocks, cudaStream_t s);
+// The vertex phase of FP64 plans (acg_vertex_fx.cu), every pattern size: its
+// schedule (nonzero for every pattern), launch and grid.
 int vertex_fx_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out);
 int vertex_fx_warps(int pn, int pp);  // warps that share a stage
 acg_status launch_vertex_fx(const VertexUpdArgs<double>& a, int blocks, cudaStream_t s);

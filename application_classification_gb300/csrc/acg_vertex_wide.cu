@@ -354,7 +354,8 @@ __global__ void __launch_bounds__(kThreads, kBlocks) vertex_wide_kernel(const Ve
 __global__ void __launch_bounds__(256)
 wide_partials_kernel(const float* __restrict__ rowpart, int V, int Pe, int Pn, int Pp,
                      double* __restrict__ bpart) {
-  const int bx = blockIdx.x, gx = gridDim.x, nmax = 2 * Pe, prows = kTileThreads / Pn;
+  const int bx = blockIdx.x, gx = gridDim.x, nmax = 2 * Pe;
+  const int rows = min(kTileThreads / Pn, V);  // (threads beyond the tile's rows added nothing)
   for (int j = threadIdx.x; j < 2 * Pe + Pn; j += 256) {
     double m = -CUDART_INF, s = 0;
     if (j < 2 * Pe) {
@@ -368,7 +369,7 @@ wide_partials_kernel(const float* __restrict__ rowpart, int V, int Pe, int Pn, i
       bpart[(size_t)j * gx + bx] = f;
     } else {
       const float* rm = rowpart + (size_t)gx * V * 8 * Pp + (size_t)bx * 3 * kTileThreads + (j - 2 * Pe);
-      for (int r = 0; r < prows; ++r, rm += Pn)
+      for (int r = 0; r < rows; ++r, rm += Pn)
         lse_merge(m, s, (double)rm[0], (double)rm[kTileThreads] - (double)rm[2 * kTileThreads]);
     }
     bpart[(size_t)(nmax + 2 * j) * gx + bx] = m;
@@ -391,7 +392,20 @@ acg_status launch_wide(const VertexUpdArgs<float>& a, int V, int blocks, cudaStr
 
 }  // namespace
 
-int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, std::vector<uint32_t>* out) {
+// Few pattern vertices share many edges: their long sums are a few lanes' of each
+// row, and a large graph has the tiles over which the tile form spreads them.  Ten
+// iterations, tile form / this one: 33,000 vertices, 8 and 132, 8 and 256: 2.40 / 2.55,
+// 2.79 / 2.90 ms (20,000: 1.94 / 1.94, 2.06 / 2.20); 200,000, 16 and 132, 20 and 144:
+// 7.98 / 8.98, 8.24 / 8.53 (33,000: 2.45 / 2.45, 2.47 / 2.36); rows of one warp, 2 and
+// 100, 4 and 100: 200,000 6.08 / 7.80, 5.97 / 6.60, 33,000 2.22 / 2.13, 2.18 / 1.96.
+static bool few_vertices(int pn, int pp, int dn) {
+  if (wide_warps(pp) == 1) return pn <= 2 && dn >= 1 << 16;
+  return (pn <= 8 && dn >= 1 << 15) || (pn <= 16 && kTileThreads / (pp / 4) >= 6 && dn >= 1 << 16);
+}
+
+int vertex_wide_schedule(const int* pat, int pn, int pe, int pp, int pnp, int dn, std::vector<uint32_t>* out) {
+  out->clear();
+  if (few_vertices(pn, pp, dn)) return 0;
   const int nt = vertex_warp_schedule(pat, pn, pe, pp, pnp, kWv, out, 32 * wide_warps(pp), 4);
   if (wide_warps(pp) == 1 || nt <= kWideTerms) return nt;
   out->clear();
