@@ -398,7 +398,7 @@ __device__ __forceinline__ void edge_max_range(const EdgeMaxArgs<T>& a, int it, 
 // three blocks 60.3, two 67; the wide shapes keep what their registers allow.)
 template <typename T, int NQV>
 constexpr int edge_min_blocks() {
-      return sizeof(T) == 4 ? ACG_EDGE_MINB : NQV == 1 ? 4 : NQV == 2 ? 2 : 1;
+  return sizeof(T) == 4 ? ACG_EDGE_MINB : NQV == 1 ? 4 : NQV == 2 ? 2 : 1;
 }
 template <typename T, int NPOW, int NQV, bool ARG>
 __global__ void __launch_bounds__(kAT, (edge_min_blocks<T, NQV>()))

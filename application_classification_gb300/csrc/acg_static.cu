@@ -32,11 +32,6 @@ constexpr int kST = 256;  // threads per block (the edge phase's warp work uses 
 #ifndef ACG_SRC_KU
 #define ACG_SRC_KU 4
 #endif
-// An explicit minimum of one block per SM (the compiler then keeps more of the
-// pipelined loads in registers): static passes 14.3 -> 10.3 ms at RMAT-22.
-#ifndef ACG_SRC_MINB
-#define ACG_SRC_MINB 1
-#endif
 constexpr int kSU = ACG_SRC_KU;  // load steps issued back to back
 
 template <typename T>
@@ -78,20 +73,19 @@ __device__ __forceinline__ void kahan_add(T& s, T& c, T x) {
 template <typename T>
 __device__ __forceinline__ T exp_ref_limit() { return sizeof(T) == 4 ? T(60) : T(600); }
 
-// The FP32 one-vector-per-lane shapes stage the gathered dE rows through a
-// per-warp ring in shared memory with cp.async: a stage is one step's positions
+// The source-side pass gives a lane one 16-byte vector of the row (wider rows:
+// several launches).  FP32 plans stage the gathered dE rows through a per-warp ring in shared memory with cp.async: a stage is one step's positions
 // (S * kSU rows, 2 KB), issued kSrcAhead stages ahead of the step that reads
 // it, so the rows in flight no longer cost registers.
 constexpr int kSrcAhead = 3;
 constexpr int kSrcSlots = kSrcAhead + 2;  // a step spans at most two stages
 constexpr int kSrcStageBytes = 32 * kSU * 16;
-template <typename T, int NQV>
-__host__ __device__ constexpr bool src_staged() { return sizeof(T) == 4 && NQV == 1; }
-template <typename T, int NQV>
-__host__ __device__ constexpr size_t src_stage_smem() {
+template <typename T>
+__host__ __device__ constexpr bool src_staged() { return sizeof(T) == 4; }
+template <typename T>
+__host__ __device__ constexpr size_t src_smem() {
   // (FP64: the exponential's table)
-  return sizeof(T) == 8 ? sizeof(uint64_t) * kFxTable
-         : src_staged<T, NQV>() ? (size_t)(kST / 32) * kSrcSlots * kSrcStageBytes : 0;
+  return src_staged<T>() ? (size_t)(kST / 32) * kSrcSlots * kSrcStageBytes : sizeof(uint64_t) * kFxTable;
 }
 __device__ __forceinline__ void src_cp16(void* sdst, const void* gsrc) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
@@ -108,19 +102,13 @@ __device__ __forceinline__ void src_wait(int n) {
   }
 }
 
-#if ACG_SRC_MINB > 0
-#define ACG_SRC_BOUNDS __launch_bounds__(kST, ACG_SRC_MINB)
-#else
-#define ACG_SRC_BOUNDS __launch_bounds__(kST)
-#endif
 // One range of a warp's items, [it, it_end).
-template <typename T, int NPOW, int NQV>
+template <typename T, int NPOW>
 __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it, const int it_end,
                                                 const int slot, const int qc, const uint64_t* tab) {
   using VT = typename SV<T>::type;
   constexpr int W = SV<T>::W;
   constexpr int S = 32 / NPOW;
-  constexpr int NQ = NQV * W;
   constexpr int STEP = S * kSU;
   const int Pp = a.Pp, Pqc = a.Pqc, qcov = a.qcov;
   if (it >= it_end) return;
@@ -133,14 +121,14 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
   for (int u = 0; u < kSU; ++u) {
     const int e = base + slot + S * u;
     const bool ok = e < item.z;
-    ridx[u] = ok && !src_staged<T, NQV>() ? __ldg(a.row_of + e) : 0;
+    ridx[u] = ok && !src_staged<T>() ? __ldg(a.row_of + e) : 0;
     eidx[u] = ok ? __ldg(a.eid + e) : 0;
   }
   // staged: the warp's positions [P0, P1) in stages of STEP rows, stage j in
   // ring slot j % kSrcSlots
   const int lane = threadIdx.x & 31;
   const int P0 = item.y;
-  const int P1 = src_staged<T, NQV>() ? __ldg(a.items + it_end - 1).z : 0;
+  const int P1 = src_staged<T>() ? __ldg(a.items + it_end - 1).z : 0;
   const int nst = (P1 - P0 + STEP - 1) / STEP;
   VT* ring = nullptr;
   int issued = 0;
@@ -168,7 +156,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
     ++issued;
     load_rows(issued);
   };
-  if constexpr (src_staged<T, NQV>()) {
+  if constexpr (src_staged<T>()) {
     extern __shared__ __align__(16) unsigned char src_ring[];
     ring = reinterpret_cast<VT*>(src_ring) + (size_t)(threadIdx.x >> 5) * kSrcSlots * (kSrcStageBytes / 16);
     load_rows(0);
@@ -182,16 +170,16 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
   // FP64 instead keeps each column's sum in integer arithmetic relative to its
   // own largest term (acg_fx.cuh): no FP64 exponential and no range to leave.
   constexpr bool kFx = sizeof(T) == 8;
-  T mn[NQ], qx[NQ], sm[kFx ? 1 : NQ], sc[kFx ? 1 : NQ];
-  FxLse fl[kFx ? NQ : 1];
+  T mn[W], qx[W], sm[kFx ? 1 : W], sc[kFx ? 1 : W];
+  FxLse fl[kFx ? W : 1];
   constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
-  unsigned long long nb[kFx ? NQ : 1], qb[kFx ? NQ : 1];  // bits of min dE, min covered
-  int qlim32[kFx ? NQ : 1];                               // (edge ids are below 2^31)
+  unsigned long long nb[kFx ? W : 1], qb[kFx ? W : 1];  // bits of min dE, min covered
+  int qlim32[kFx ? W : 1];                               // (edge ids are below 2^31)
   // quirk coverage of column q: original edge id < lim - q * De (no edge for
   // the columns q >= qcov, whose quirk value is never read)
-  long long qlim[NQ];
+  long long qlim[W];
 #pragma unroll
-  for (int k = 0; k < NQ; ++k) {
+  for (int k = 0; k < W; ++k) {
     mn[k] = pos_inf<T>();
     qx[k] = neg_inf<T>();
     if constexpr (kFx) {
@@ -201,15 +189,15 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
       sm[k] = T(0);
       sc[k] = T(0);
     }
-    const int q = (qc + NPOW * (k / W)) * W + k % W;
+    const int q = qc * W + k;
     qlim[k] = q < qcov ? __ldg(a.qlim_col + q) : 0;
     if constexpr (kFx) qlim32[k] = (int)min(max(qlim[k], 0ll), 0x7fffffffll);
   }
   for (;;) {
-    VT x[kSU][NQV];
+    VT x[kSU];
     bool okv[kSU];
     int ecur[kSU];
-    if constexpr (src_staged<T, NQV>()) {
+    if constexpr (src_staged<T>()) {
       // the stages this step reads (its first and last position's) in place,
       // kSrcAhead more in flight
       const int jlo = (base - P0) / STEP, jhi = min(nst - 1, (base + STEP - 1 - P0) / STEP);
@@ -224,7 +212,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
         ecur[u] = eidx[u];
         const int rel = e - P0, j = rel / STEP;
         (void)jlo;
-        x[u][0] = (okv[u] && qc * W < Pp)
+        x[u] = (okv[u] && qc * W < Pp)
                       ? ring[(size_t)(j % kSrcSlots) * (kSrcStageBytes / 16) + (rel - j * STEP) * NPOW + qc - a.col0]
                       : sfill<T>(pos_inf<T>());
       }
@@ -234,13 +222,8 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
         const int e = base + slot + S * u;
         okv[u] = e < item.z;
         ecur[u] = eidx[u];
-#pragma unroll
-        for (int k = 0; k < NQV; ++k) {
-          const int qv = qc + NPOW * k;
-          x[u][k] = (okv[u] && qv * W < Pp)
-                        ? reinterpret_cast<const VT*>(a.dE + (size_t)ridx[u] * Pp)[qv]
-                        : sfill<T>(pos_inf<T>());
-        }
+        x[u] = (okv[u] && qc * W < Pp) ? reinterpret_cast<const VT*>(a.dE + (size_t)ridx[u] * Pp)[qc]
+                                       : sfill<T>(pos_inf<T>());
       }
     }
     const bool item_done = base + STEP >= item.z;
@@ -255,7 +238,7 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
     for (int u = 0; u < kSU; ++u) {
       const int e = nbase + slot + S * u;
       const bool ok = more && e < nend;
-      ridx[u] = ok && !src_staged<T, NQV>() ? __ldg(a.row_of + e) : 0;
+      ridx[u] = ok && !src_staged<T>() ? __ldg(a.row_of + e) : 0;
       eidx[u] = ok ? __ldg(a.eid + e) : 0;
     }
     // branch-free: a missing edge reads +inf, which changes no minimum, adds
@@ -263,37 +246,33 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
 #pragma unroll
     for (int u = 0; u < kSU; ++u)
 #pragma unroll
-      for (int k = 0; k < NQV; ++k)
-#pragma unroll
-        for (int w = 0; w < W; ++w) {
-          const T d = sg<T>(x[u][k], w);
-          const int j = k * W + w;
-          if constexpr (!kFx) mn[j] = fmin(mn[j], d);
-          if constexpr (kFx) {
-            // costs are not negative: minima (and the quirk maximum, as minus
-            // the minimum of the covered costs and zeros) in their bits' order
-            const bool cov = ecur[u] < qlim32[j];
-            const unsigned long long bd = (unsigned long long)__double_as_longlong(d);
-            const unsigned long long bc = cov ? bd : 0ull;
-            nb[j] = bd < nb[j] ? bd : nb[j];
-            qb[j] = bc < qb[j] ? bc : qb[j];
-            fx_add(fl[j], -d, tab);
-            continue;
-          } else {
-            kahan_add(sm[j], sc[j], exp_fast(-d));
-          }
+      for (int j = 0; j < W; ++j) {
+        const T d = sg<T>(x[u], j);
+        if constexpr (kFx) {
+          // costs are not negative: minima (and the quirk maximum, as minus
+          // the minimum of the covered costs and zeros) in their bits' order
+          const bool cov = ecur[u] < qlim32[j];
+          const unsigned long long bd = (unsigned long long)__double_as_longlong(d);
+          const unsigned long long bc = cov ? bd : 0ull;
+          nb[j] = bd < nb[j] ? bd : nb[j];
+          qb[j] = bc < qb[j] ? bc : qb[j];
+          fx_add(fl[j], -d, tab);
+        } else {
+          mn[j] = fmin(mn[j], d);
+          kahan_add(sm[j], sc[j], exp_fast(-d));
           qx[j] = fmax(qx[j], (long long)ecur[u] < qlim[j] ? -d : T(0));
         }
+      }
     if (item_done) {
-      T lm[NQ], lsum[NQ];  // the column's (reference, sum of exp(-dE - reference))
+      T lm[W], lsum[W];  // the column's (reference, sum of exp(-dE - reference))
       if constexpr (!kFx) {
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) lsum[k] = sm[k] - sc[k];
+        for (int k = 0; k < W; ++k) lsum[k] = sm[k] - sc[k];
       }
 #pragma unroll
       for (int o = NPOW; o < 32; o <<= 1)
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) {
+        for (int k = 0; k < W; ++k) {
           if constexpr (kFx) {
             const unsigned long long on = __shfl_xor_sync(0xffffffffu, nb[k], o);
             const unsigned long long oq = __shfl_xor_sync(0xffffffffu, qb[k], o);
@@ -309,10 +288,9 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
             lsum[k] += __shfl_xor_sync(0xffffffffu, lsum[k], o);
           }
         }
-      bool far = false;
       if constexpr (kFx) {
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) {
+        for (int k = 0; k < W; ++k) {
           double m = 0, sv = 0;
           if (slot == 0) fx_pair(fl[k], m, sv);
           lm[k] = m;
@@ -321,66 +299,59 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
           qx[k] = __longlong_as_double((long long)(qb[k] ^ 0x8000000000000000ull));
         }
       } else {
+        bool far = false;
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) {
+        for (int k = 0; k < W; ++k) {
           lm[k] = T(0);
           far |= mn[k] > exp_ref_limit<T>() && mn[k] < pos_inf<T>();
         }
-      }
-      if (!kFx && __any_sync(0xffffffffu, far)) if constexpr (!kFx) {
-        // sum exp(mn - dE) again over this item's edges, for every column
+        if (__any_sync(0xffffffffu, far)) {
+          // sum exp(mn - dE) again over this item's edges, for every column
 #pragma unroll
-        for (int k = 0; k < NQ; ++k) {
-          sm[k] = T(0);
-          sc[k] = T(0);
-        }
-        for (int e = item.y + slot; e < item.z; e += S) {
-          const T* row = a.dE + (size_t)__ldg(a.row_of + e) * Pp;
-#pragma unroll
-          for (int k = 0; k < NQV; ++k) {
-            const int qv = qc + NPOW * k;
-            if (qv * W >= Pp) continue;
-            const VT xv = reinterpret_cast<const VT*>(row)[qv];
-#pragma unroll
-            for (int w = 0; w < W; ++w)
-              kahan_add(sm[k * W + w], sc[k * W + w], exp_fast(mn[k * W + w] - sg<T>(xv, w)));
+          for (int k = 0; k < W; ++k) {
+            sm[k] = T(0);
+            sc[k] = T(0);
           }
+          for (int e = item.y + slot; e < item.z; e += S) {
+            const T* row = a.dE + (size_t)__ldg(a.row_of + e) * Pp;
+            if (qc * W >= Pp) continue;
+            const VT xv = reinterpret_cast<const VT*>(row)[qc];
+#pragma unroll
+            for (int w = 0; w < W; ++w) kahan_add(sm[w], sc[w], exp_fast(mn[w] - sg<T>(xv, w)));
+          }
+#pragma unroll
+          for (int k = 0; k < W; ++k) {
+            lsum[k] = sm[k] - sc[k];
+            lm[k] = -mn[k];
+          }
+#pragma unroll
+          for (int o = NPOW; o < 32; o <<= 1)
+#pragma unroll
+            for (int k = 0; k < W; ++k) lsum[k] += __shfl_xor_sync(0xffffffffu, lsum[k], o);
         }
-#pragma unroll
-        for (int k = 0; k < NQ; ++k) {
-          lsum[k] = sm[k] - sc[k];
-          lm[k] = -mn[k];
-        }
-#pragma unroll
-        for (int o = NPOW; o < 32; o <<= 1)
-#pragma unroll
-          for (int k = 0; k < NQ; ++k) lsum[k] += __shfl_xor_sync(0xffffffffu, lsum[k], o);
       }
       if (slot == 0) {
         const int v = item.x;
 #pragma unroll
-        for (int k = 0; k < NQV; ++k)
-#pragma unroll
-          for (int w = 0; w < W; ++w) {
-            const int q = (qc + NPOW * k) * W + w;
-            if (q >= Pp) continue;
-            const int j = k * W + w;
-            if (item.w >= 0) {
-              T* pr = a.partial + (size_t)item.w * (3 * Pp + Pqc);
-              pr[q] = mn[j];
-              pr[Pp + q] = lm[j];
-              pr[2 * Pp + q] = lsum[j];
-              if (q < Pqc) pr[3 * Pp + q] = qx[j];
-            } else {
-              a.dEmin[(size_t)v * Pp + q] = mn[j];
-              a.B[(size_t)v * Pp + q] =
-                  (lm[j] > neg_inf<T>() && lsum[j] > T(0)) ? lm[j] + dev_log(lsum[j]) : neg_inf<T>();
-              if (q < Pqc) a.Rq[(size_t)v * Pqc + q] = qx[j];
-            }
+        for (int j = 0; j < W; ++j) {
+          const int q = qc * W + j;
+          if (q >= Pp) continue;
+          if (item.w >= 0) {
+            T* pr = a.partial + (size_t)item.w * (3 * Pp + Pqc);
+            pr[q] = mn[j];
+            pr[Pp + q] = lm[j];
+            pr[2 * Pp + q] = lsum[j];
+            if (q < Pqc) pr[3 * Pp + q] = qx[j];
+          } else {
+            a.dEmin[(size_t)v * Pp + q] = mn[j];
+            a.B[(size_t)v * Pp + q] =
+                (lm[j] > neg_inf<T>() && lsum[j] > T(0)) ? lm[j] + dev_log(lsum[j]) : neg_inf<T>();
+            if (q < Pqc) a.Rq[(size_t)v * Pqc + q] = qx[j];
           }
+        }
       }
 #pragma unroll
-      for (int k = 0; k < NQ; ++k) {
+      for (int k = 0; k < W; ++k) {
         mn[k] = pos_inf<T>();
         qx[k] = neg_inf<T>();
         if constexpr (kFx) {
@@ -398,17 +369,18 @@ __device__ __forceinline__ void src_stats_range(const SrcStatsArgs<T>& a, int it
     }
     base = nbase;
   }
-  if constexpr (src_staged<T, NQV>()) {
+  if constexpr (src_staged<T>()) {
     src_wait(0);  // nothing of this range in flight when the ring is reused
     __syncwarp();
   }
 }
 
 // The warp's own range first, then claimed ones (as edge_max_kernel).
-// The staged shapes keep two blocks (16 warps) per SM: their rows in flight sit
-// in shared memory, not in registers.
-template <typename T, int NPOW, int NQV>
-__global__ void __launch_bounds__(kST, src_staged<T, NQV>() ? 2 : (ACG_SRC_MINB > 0 ? ACG_SRC_MINB : 1))
+// FP32 keeps two blocks (16 warps) per SM: its rows in flight sit in shared
+// memory, not in registers.  FP64: an explicit minimum of one, with which the compiler
+// keeps more of the pipelined loads in registers.
+template <typename T, int NPOW>
+__global__ void __launch_bounds__(kST, src_staged<T>() ? 2 : 1)
 src_stats_kernel(const SrcStatsArgs<T> a) {
   const int lane = threadIdx.x & 31;
   const int slot = lane / NPOW, qc = a.col0 + lane % NPOW;
@@ -426,7 +398,7 @@ src_stats_kernel(const SrcStatsArgs<T> a) {
   for (int r = gw; r < a.nranges;) {
     int rn = a.nranges;
     if (a.ctr && lane == 0) rn = nw + atomicAdd(a.ctr, 1);
-    src_stats_range<T, NPOW, NQV>(a, __ldg(a.wsplit + r), __ldg(a.wsplit + r + 1), slot, qc, tab);
+    src_stats_range<T, NPOW>(a, __ldg(a.wsplit + r), __ldg(a.wsplit + r + 1), slot, qc, tab);
     r = __shfl_sync(0xffffffffu, rn, 0);
   }
   if (a.ctr && lane == 0) {
@@ -844,11 +816,11 @@ bool init_warp_shape(int pn, int pp, F&& f) {
 #define ACG_SRC_SHAPES(X) X(1) X(2) X(4) X(8) X(16) X(32)
 #define ACG_SRC_LAUNCH(NP_)                                                                 \
   if (ws.npow == NP_) {                                                                     \
-    constexpr size_t sm = src_stage_smem<T, 1>();                                           \
+    constexpr size_t sm = src_smem<T>();                                           \
     if (sm > 48 * 1024)                                                                     \
-      ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_kernel<T, NP_, 1>,                        \
+      ACG_CUDA_TRY(cudaFuncSetAttribute(src_stats_kernel<T, NP_>,                        \
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)); \
-    ACG_CUDA_TRY(launch_kernel(a.early, src_stats_kernel<T, NP_, 1>, blocks, kST, sm, s, a));     \
+    ACG_CUDA_TRY(launch_kernel(a.early, src_stats_kernel<T, NP_>, blocks, kST, sm, s, a));     \
     continue;                                                                               \
   }
 
@@ -899,11 +871,11 @@ acg_status launch_dst_quirk(const DstQuirkArgs<T>& a, WarpShape ws, int blocks, 
 
 #define ACG_SRC_OCC(NP_)                                                                \
   if (ws.npow == NP_) {                                                                 \
-    constexpr size_t sm = src_stage_smem<T, 1>();                                       \
+    constexpr size_t sm = src_smem<T>();                                       \
     if (sm > 48 * 1024)                                                                 \
-      cudaFuncSetAttribute(src_stats_kernel<T, NP_, 1>,                                 \
+      cudaFuncSetAttribute(src_stats_kernel<T, NP_>,                                 \
                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);       \
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, src_stats_kernel<T, NP_, 1>, \
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, src_stats_kernel<T, NP_>, \
                                                       kST, sm) != cudaSuccess)          \
       nb = 1;                                                                           \
   }
