@@ -342,14 +342,19 @@ bool side_worthwhile(bool batch, long long De, int Pp, int elem) {
 // Whether kernels may start early (launch_kernel).  Not in plans whose statistics
 // run beside the edge phase: blocks of it waiting for their turn would keep those
 // off the SMs (R-MAT 17 batch 173 -> 189 ms).  And where the passes are short enough
-// for the gaps between them to count: R-MAT 16 mixed (134 MB of costs) 1.78 -> 1.70
-// ms, R-MAT 18 mixed (537 MB) 4.59 -> 4.51, 40/120 patterns on R-MAT 18 (2 GB)
-// 30.85 -> 30.75; but R-MAT 20 FP64 (8.6 GB) 132 -> 162 ms and R-MAT 22 mixed
-// (16.7 GB) 174 -> 180, where the blocks that wait take the place of running ones
-// for longer than a gap.
+// for the gaps between them to count, by the bytes of the costs; early / in turn, ms:
+//   mixed, 16/32: R-MAT 16 (0.13 GB) 1.56 / 1.66, R-MAT 18 (0.54 GB) 4.17 / 4.30;
+//   mixed, 32/64: R-MAT 18 (1.1 GB) 11.82 / 11.88, R-MAT 19 (2.15 GB) 22.11 / 21.91,
+//   R-MAT 20 (4.3 GB) 43.5 / 42.5; 40/120, R-MAT 18 (2.0 GB) 30.75 / 30.85;
+//   FP64, 16/32: R-MAT 18 (1.1 GB) 12.61 / 12.67; 16/48: R-MAT 16 (0.4 GB) 5.97 / 5.95;
+//   48/192: R-MAT 16 (1.6 GB) 49.2 / 49.4.
+// FP64 plans of 50 to 64 columns lose from small sizes on, their vertex blocks, of
+// half an SM's shared memory each, waiting beside the edge phase: 32/64, R-MAT 12
+// (0.03 GB) 1.80 / 1.89, R-MAT 14 (0.13 GB) 4.25 / 4.09, R-MAT 17 (1.1 GB) 21.9 / 18.8.
 template <typename T>
 bool early_launches(const acg_plan* P) {
-  return !P->side && (double)P->data->De * P->Pp * sizeof(T) < 3e9;
+  const double limit = sizeof(T) == 8 && P->Pp > 48 && P->Pp <= 64 ? 0.1e9 : 2.1e9;
+  return !P->side && (double)P->data->De * P->Pp * sizeof(T) < limit;
 }
 
 // The counter that warps claim further item ranges from; none where every range is
