@@ -16,8 +16,13 @@
 //
 // One thread per row: its features in registers, the pattern's parts in shared
 // memory (broadcast 16-byte loads of two features), two columns at a time.
-// R-MAT 20, 17 features x 64 columns: 90.7 -> 12.2 ms (8.6 GB written, 2.8 GB
+// R-MAT 20, 17 features x 64 columns: 90.7 -> 12.7 ms (8.6 GB written, 2.8 GB
 // of rows gathered: 1.7 ms at the copy bandwidth); the multiply-adds bound it.
+// Where many pairs are left to FP64, the call for them is still no slower than forming
+// the whole matrix in FP64 with the row in registers, as the FP64 pipe charges the
+// lanes that are active: 131,072 vertices, 16 edges each, 13 and 17 features, a 32/64
+// pattern, one iteration: N(0, 1) 4.2 / 13.1 ms; lognormal, sigma 1 and 2, 4.4 / 13.1
+// and 11.2 / 13.8; one feature 100 or 10,000 times the others 11.9 / 13.2 and 17.9 / 18.8.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -52,15 +57,17 @@ __device__ __forceinline__ double pair_one(double x, double y) {
   return e > 1023 - 500 && e < 1023 + 500 ? u : sqrt(t * t);
 }
 __device__ void rows_one(const CdistRbArgs<double, double>& a) {
+  const double* y = a.y;
   for (long long r = (long long)blockIdx.x * kXT + threadIdx.x; r < a.nrows;
        r += (long long)gridDim.x * kXT) {
-    const double x = __ldg(a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride);
+    const double* xr = a.x + (size_t)(a.row ? (long long)__ldg(a.row + r) : r) * a.kstride;
+    const double x = __ldg(xr);
     double* orow = a.out + (size_t)r * a.ostride;
     for (int q0 = 0; q0 < a.Pp; q0 += 2) {
       double d[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        d[j] = q0 + j < a.P ? pair_one(x, __ldg(a.y + q0 + j)) : 0.0;
+        d[j] = q0 + j < a.P ? pair_one(x, __ldg(y + q0 + j)) : 0.0;
         if (a.wide && q0 + j < a.P) d[j] = edge_word(d[j], a.wide);
       }
       *reinterpret_cast<double2*>(orow + q0) = make_double2(d[0], d[1]);
