@@ -877,8 +877,8 @@ vertex_update_kernel(const VertexUpdArgs<T> a) {
 // how the jobs are spread.  Vertices without in-edges have M rows of -inf (set
 // once, never written by phase A).
 // Bound by instruction issue (2.7 of 4 a cycle from 16 warps an SM) and the shared
-// memory pipe: one more load a term cost 5%.  R-MAT 22, pattern 32/64 (3.2 GB,
-// 0.47 ms at the copy bandwidth): 1.74 ms an iteration with 102.9 M instructions
+// memory pipe: one more load a term cost 5%.  R-MAT 22, pattern 32/64 (7.5 GB,
+// 1.11 ms at the copy bandwidth): 1.74 ms an iteration with 102.9 M instructions
 // and 10.1 M conflict cycles at R-MAT 18, 1.59 ms with 88.7 M and 5.3 M so.  The
 // tail of a stage by a branch (predicated: 1% slower).  On a small graph a launch
 // is its constants and its block partials.

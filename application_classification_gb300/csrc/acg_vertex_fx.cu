@@ -26,8 +26,8 @@
 // R-MAT 20, pattern 32/64 (1.05 M vertices, 3.5 GB, 0.52 ms at the copy
 // bandwidth): FP64 8.77 ms an iteration, with integer exponentials 5.9, in fixed
 // point 1.71, with the range checked on the words already in registers and the
-// larger exponential table 1.45.  ncu: 1,050 warp instructions per vertex, the
-// integer (ALU) pipe 63% busy, FP64 pipe 11%, DRAM 26%.
+// larger exponential table 1.42.  ncu: 900 warp instructions per vertex, the
+// integer (ALU) pipe 59% busy, FP64 pipe 9%, DRAM 25%.
 #include <cuda_runtime.h>
 
 #include <algorithm>

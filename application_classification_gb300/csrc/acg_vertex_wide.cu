@@ -16,7 +16,7 @@
 // those of the tile form: a block of V = 256 / (Pp / 4) rows walks the tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ...
 // R-MAT 18, pattern 40/120 (0.84 GB, 124 us at the copy bandwidth): 458 us an
-// iteration as block tiles, 234 so (and 100 of merges beside the edge phase);
+// iteration as block tiles, 233 so (and 48 of merges, in a batch beside the edge phase);
 // 131,072 vertices, patterns of 132 to 192 columns: 284 -> 190 us.  Two columns a
 // lane with twice the warps was slower (435 us: the copies, the schedule and the
 // barriers are per warp), and so were constants held in registers (326).
