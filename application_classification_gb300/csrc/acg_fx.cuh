@@ -429,13 +429,14 @@ ACG_FX_SLOW FxLse fx_merge_wide(FxLse a, FxLse b) {
   double m, s, m2, s2;
   fx_pair(a, m, s);
   fx_pair(b, m2, s2);
-  if (s2 == 0.0) return a;
-  if (s == 0.0) return b;
-  if (m2 > m) {
-    s = s * exp(m - m2) + s2;
+  const double d = m2 - m;
+  if (s2 == 0.0 || d < -kFxFar) return a;
+  if (s == 0.0 || d > kFxFar) return b;
+  if (d > 0.0) {
+    s = s * exp(-d) + s2;
     m = m2;
   } else {
-    s += s2 * exp(m2 - m);
+    s += s2 * exp(d);
   }
   const uint64_t mb = fx_bits(m), sb = fx_bits(-s);
   a.w[0] = (uint32_t)mb;
